@@ -150,10 +150,12 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
             const int lx0 = (l4 % XS) * NX, ly = (l4 / XS) % G::BY, lz = l4 / (XS * G::BY);
             const int x0 = bc.x * G::BX + lx0, y = bc.y * G::BY + ly, z = bc.z * G::BZ + lz;
             const long long s0 = (long long) b * G::BN + lx0 + G::BX * (ly + G::BY * lz);
-            const bool row_in = y < L.ny && (DIM == 2 || z < L.nz);
+            // brick slots past the lattice's end walk no cell rows: their window would start
+            // past the row's end, and past the cell ranges themselves in the last row
+            const bool row_in = x0 < L.nx && y < L.ny && (DIM == 2 || z < L.nz);
             // and, per node pair, only when a node's cell is within reach of the boundary
             int npass = 1;
-            if (walls && row_in && x0 < L.nx) {
+            if (walls && row_in) {
                 const long long c0 = (long long) x0 + (long long) L.nx * (y + (long long) L.ny * z);
                 if (bcell[c0] || (x0 + 1 < L.nx && bcell[c0 + 1])) npass = 2;
             }
