@@ -74,7 +74,8 @@ typedef struct swc_solver_opts {
     double  tolerance;             /* relative residual (reference default 1e-6) */
     int32_t max_iterations;        /* < 0: 2 * N_v (Eigen default) */
     int32_t warm_start;            /* swc_warm_start */
-    int32_t check_interval;        /* CG iterations between host convergence checks (0: auto) */
+    int32_t check_interval;        /* accepted, without effect: the solve tests for its end on the device
+                                      in every iteration */
     int32_t keep_virtual_velocity; /* store vbar_I for swc_get_virtual */
     int32_t compute_true_residual; /* evaluate |b - A x| / |b| after each solve */
     int32_t keep_features;         /* keep per-node neighbour counts (learned warm start) */
@@ -179,9 +180,11 @@ int swc_debug_neighbors(swc_ctx * ctx, int which, int64_t nq, const double * q, 
 int swc_set_profiling(swc_ctx * ctx, int on);
 int swc_get_phase_times(swc_ctx * ctx, double * ms, int n);
 /* Times `reps` back-to-back launches of one kernel on the live state with CUDA
- * events (0: CG SpMV, 1: CG update, 2: virtual gather, 3: pressure gradient,
- * 4: density, 5: forces, 6: CG direction update, 7: learned warm-start forward
- * pass, after a projection that used it); writes the mean ms per launch. */
+ * events (2: virtual gather, 3: pressure gradient, 4: density, 5: forces,
+ * 7: learned warm-start forward pass, after a projection that used it), or the
+ * phases of `reps` iterations of the CG solve (3D; 0: product with the wait for
+ * neighbouring bricks, 1: meeting for the dot products, 6: step of x, r and d);
+ * writes the mean ms per launch or iteration. */
 int swc_time_kernel(swc_ctx * ctx, int which, int reps, double * mean_ms);
 
 /* ---- Learned CG warm start (no counterpart in the reference) -------------

@@ -1,0 +1,592 @@
+// k_cg_solve.cu -- the CG solve of the projection as one resident kernel, and the
+// other row-stencil passes on the same warp-per-brick stencil (alpha_hat, residuals
+// of the CG start).
+//
+// CG (Eigen's Hestenes-Stiefel form on the full matrix, k_cg.cu) from the start
+// state to its end in one cooperative launch, one block per SM.  A group of W warps
+// (fewer where bricks are many) owns its bricks in both phases of an iteration:
+//   step      x += alpha d, r -= alpha q, d = r + beta d, u = V d       (streaming)
+//   product   q = A d from the halo tile of u (swc_stencil.cuh), and the four dot
+//             products d.q, r.q, q.q, r.r
+// alpha = r.r / d.q, and |r - alpha q|^2 = r.r - 2 alpha r.q + alpha^2 q.q gives beta
+// and the stopping test without a second trip: the sums hold 44 bits and more, the
+// quotient of two successive norms is seldom below a tenth, and where it is below
+// 1e-6 the norm is summed from r - alpha q itself.  r.r is summed from r in every
+// iteration, so nothing of a prediction is carried on.
+// Before a warp copies a tile it waits for the flags of the brick's neighbours; the
+// blocks meet once per iteration, for the sums, and each decides by itself whether to
+// go on, with no host check.  Dot products use exact FP32 products in float-float per
+// lane, triple floats below the block and FP64 above, in a fixed order.
+#include "swc_kernels.h"
+#include "swc_stencil.cuh"
+
+namespace swc {
+
+namespace {
+
+__device__ __forceinline__ float4 ld4(const float * a, long long s) { return *reinterpret_cast<const float4 *>(a + s); }
+__device__ __forceinline__ void st4(float * a, long long s, float4 v) { *reinterpret_cast<float4 *>(a + s) = v; }
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+__device__ __forceinline__ float4 fma4(float s, float4 a, float4 b) {
+    return make_float4(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y), fmaf(s, a.z, b.z), fmaf(s, a.w, b.w));
+}
+__device__ __forceinline__ float comp(const float4 & v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
+
+constexpr int kSums = 4;  // values of a meeting
+
+// Triple floats (three error-free terms, about 70 bits): the sums below the block.
+// GB300 adds or converts two FP64 values per SM and clock, so FP64 in the lanes of every
+// warp would queue for half a microsecond; a block converts its totals alone.
+struct F3 {
+    float h, m, l;
+};
+__device__ __forceinline__ F3 f3_add(const F3 & a, const F3 & b) {
+    float s, e, t, f, u, g;
+    F3 o;
+    two_sum(a.h, b.h, s, e);
+    two_sum(a.m, b.m, t, f);
+    two_sum(e, t, u, g);
+    o.l = __fadd_rn(__fadd_rn(a.l, b.l), __fadd_rn(f, g));
+    fast_two_sum(s, u, o.h, o.m);
+    return o;
+}
+__device__ __forceinline__ F3 f3_shfl(const F3 & a, int o) {
+    return F3{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.m, o),
+              __shfl_xor_sync(0xffffffffu, a.l, o)};
+}
+// Sums of four float-float values over the warp: lanes 8 k .. 8 k + 7 get value k's.
+__device__ __forceinline__ F3 warp_sum4(const FF (&p)[kSums]) {
+    const int lane = threadIdx.x & 31;
+    const bool up = lane & 16, odd = lane & 8;
+    F3 q[kSums];
+#pragma unroll
+    for (int k = 0; k < kSums; k++) q[k] = F3{p[k].hi, p[k].lo, 0.f};
+    // the halves of the warp, then its quarters, exchange the values that they give up
+    const F3 a = f3_add(up ? q[2] : q[0], f3_shfl(up ? q[0] : q[2], 16));
+    const F3 b = f3_add(up ? q[3] : q[1], f3_shfl(up ? q[1] : q[3], 16));
+    F3 c       = f3_add(odd ? b : a, f3_shfl(odd ? a : b, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c = f3_add(c, f3_shfl(c, o));
+    return c;
+}
+__device__ __forceinline__ double warp_sum_double(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// A meeting's words are 16 bytes, value and tag written and read as one.
+__device__ __forceinline__ void word_put(ulonglong2 * p, unsigned long long a, unsigned long long b) {
+    asm volatile("{\n.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(a), "l"(b)
+                 : "memory");
+}
+__device__ __forceinline__ ulonglong2 word_get(const ulonglong2 * p) {
+    ulonglong2 v;
+    asm volatile("{\n.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;\n}"
+                 : "=l"(v.x), "=l"(v.y)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+// A block's partial sum.
+__device__ __forceinline__ void slot_put(ulonglong2 * p, double v, unsigned tag) {
+    word_put(p, (unsigned long long) __double_as_longlong(v), tag);
+}
+__device__ __forceinline__ bool slot_get(const ulonglong2 * p, unsigned tag, double & v) {
+    const ulonglong2 w = word_get(p);
+    v                  = __longlong_as_double((long long) w.x);
+    return unsigned(w.y) == tag;
+}
+// What block 0 made of the sums: the step's factors and how to go on.
+enum : unsigned { kGoOn = 0, kFailed = 5, kMeasure = 6 };  // 1, 2, 3: CgState::done
+struct Outcome {
+    float    alpha, beta;
+    unsigned code;
+};
+__device__ __forceinline__ void outcome_put(ulonglong2 * p, const Outcome & o, unsigned tag) {
+    word_put(p, (unsigned long long) __float_as_uint(o.beta) << 32 | __float_as_uint(o.alpha),
+             (unsigned long long) tag << 32 | o.code);
+}
+__device__ __forceinline__ bool outcome_get(const ulonglong2 * p, unsigned tag, Outcome & o) {
+    const ulonglong2 w = word_get(p);
+    o.alpha            = __uint_as_float(unsigned(w.x));
+    o.beta             = __uint_as_float(unsigned(w.x >> 32));
+    o.code             = unsigned(w.y);
+    return unsigned(w.y >> 32) == tag;
+}
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned * p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(unsigned * p, unsigned v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long v;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v));
+    return v;
+}
+
+// Polls of one slot before a block gives up (about a second).
+constexpr int kMeetPolls = 1 << 20;
+
+// Block 0's view of the solve.
+struct CgScalars {
+    double pq, rr, rr_next, threshold;
+    int    it, max_iter;
+};
+template<int WARPS> struct MeetSmem {
+    F3        part[WARPS][kSums];
+    double    sum[kSums];
+    int       full[kSums];
+    Outcome   out;
+    CgScalars cg;  // block 0
+};
+constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer blocks poll one line
+
+// The factors and the stopping test from the sums d.q, r.q, q.q, r.r (after kMeasure:
+// from |r - alpha q|^2).
+__device__ __forceinline__ Outcome decide(CgScalars & c, const double (&sum)[kSums], float alpha, bool measured) {
+    Outcome o{alpha, 0.f, kGoOn};
+    if (!measured) {
+        c.pq      = sum[0];
+        c.rr      = sum[3];
+        c.rr_next = c.rr;
+        if (!(c.pq != 0.0) || c.pq != c.pq) {
+            o.code = 3;
+            return o;
+        }
+        o.alpha   = float(c.rr / c.pq);
+        c.rr_next = c.rr + double(o.alpha) * (double(o.alpha) * sum[2] - 2.0 * sum[1]);
+        if (c.rr_next < 1e-6 * c.rr) {
+            o.code = kMeasure;  // nearly all of r goes: its norm from r - alpha q itself
+            return o;
+        }
+    } else c.rr_next = sum[0];
+    c.it++;
+    if (c.rr_next != c.rr_next) o.code = 3;
+    else if (c.rr_next < c.threshold) o.code = 1;
+    else if (c.it >= c.max_iter) o.code = 2;
+    o.beta = float(c.rr_next / c.rr);
+    return o;
+}
+
+// Meeting of the blocks in use: v (value lane / 8 of the warp, as warp_sum4 gives it)
+// summed over their warps, and what block 0 decides on the sums, the same on every
+// thread.  Every block publishes its four partials under the meeting's tag; block 0
+// reads them all and publishes the outcome, one word that the others poll.  (With
+// every block polling every slot the polls themselves, 64 B x blocks^2 a round, kept
+// the slots from being written: 13 us a meeting of 152 blocks; with the sums published
+// and the FP64 quotients formed by every thread, 5 us.)  One set of slots serves: a
+// block publishes again only after it has the outcome, and block 0 only after every
+// block has published again.
+template<int WARPS>
+__device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int stride, int blocks, unsigned & tag,
+                                        MeetSmem<WARPS> & M, float alpha, bool measured) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ulonglong2 * outcome = slots + (long long) stride * kSums;
+    if ((lane & 7) == 0) M.part[warp][lane >> 3] = v;
+    __syncthreads();
+    if (warp == 0) {
+        const int k = lane >> 3, w = lane & 7;
+        F3 part = M.part[w][k];
+        for (int j = w + 8; j < WARPS; j += 8) part = f3_add(part, M.part[j][k]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) part = f3_add(part, f3_shfl(part, o));
+        if (w == 0)
+            slot_put(slots + (long long) blockIdx.x * kSums + k, (double(part.h) + double(part.m)) + double(part.l), tag);
+        if (blockIdx.x != 0 && lane == 0) {
+            const ulonglong2 * p = outcome + blockIdx.x % kCopies;
+            Outcome o;
+            bool there = outcome_get(p, tag, o);
+            for (int n = 0; n < kMeetPolls && !there; n++) there = outcome_get(p, tag, o);
+            if (!there) o.code = kFailed;
+            M.out = o;
+        }
+    }
+    if (blockIdx.x == 0) {
+        if (warp < kSums) {
+            double s  = 0;
+            bool full = true;
+            for (int j0 = lane; j0 < blocks; j0 += 32 * 5) {  // 5 x 32 = 160 slots at once
+                double e[5];
+                bool there[5];
+                for (int n = 0; n < kMeetPolls; n++) {
+#pragma unroll
+                    for (int k = 0; k < 5; k++) {
+                        const int j = j0 + 32 * k;
+                        e[k]        = 0.0;
+                        there[k]    = j >= blocks || slot_get(slots + (long long) j * kSums + warp, tag, e[k]);
+                    }
+                    if (there[0] && there[1] && there[2] && there[3] && there[4]) break;
+                }
+                full = full && there[0] && there[1] && there[2] && there[3] && there[4];
+                s += ((e[0] + e[1]) + (e[2] + e[3])) + e[4];
+            }
+            s    = warp_sum_double(s);
+            full = __all_sync(0xffffffffu, full);
+            if (lane == 0) {
+                M.sum[warp]  = s;
+                M.full[warp] = full;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const double sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
+            Outcome o               = decide(M.cg, sum, alpha, measured);
+            if (!(M.full[0] && M.full[1] && M.full[2] && M.full[3])) o.code = kFailed;
+            for (int k = 0; k < kCopies; k++) outcome_put(outcome + k, o, tag);
+            M.out = o;
+        }
+    }
+    __syncthreads();
+    tag++;
+    return M.out;
+}
+
+// A warp's wait for the flags of a brick's active neighbours (tab); false when they did
+// not come in time.
+__device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const int * tab, unsigned tag) {
+    const int lane = threadIdx.x & 31;
+    const int b    = lane < 27 ? tab[lane] : -1;
+    bool there     = b < 0 || ld_relaxed(flags + b) == tag;
+    for (int n = 0; n < kMeetPolls && !there; n++) there = ld_relaxed(flags + b) == tag;
+    fence_gpu();
+    return __all_sync(0xffffffffu, there);
+}
+
+// Groups of W warps own the bricks c + P (g + COUNT k): the solve's loop.
+template<int DIM, int W>
+__device__ __forceinline__ void solve(const Lattice & L, const int * __restrict__ blist, int nb, int P,
+                                      const unsigned char * __restrict__ bflag, const NodeArrays & N, const Stencil & S,
+                                      CgState * cg, ulonglong2 * slots, unsigned * flags, CgPhases * phases,
+                                      MeetSmem<WarpBrick<DIM>::WARPS> & M) {
+    using B  = WarpBrick<DIM>;
+    using G  = typename B::G;
+    using Gr = Group<DIM, W>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int grp = Gr::index(), gl = Gr::lane();
+    const bool idle  = grp >= Gr::COUNT;
+    float * tile     = reinterpret_cast<float *>(smem) + B::T::TILE * grp;
+    int * tab        = reinterpret_cast<int *>(smem + B::kTileBytes) + 27 * (B::TABS + 1) * grp;
+    unsigned * seg   = reinterpret_cast<unsigned *>(smem + B::kTileBytes + B::kTabBytes);
+    const int bfirst = idle ? nb : int(blockIdx.x) + P * grp, bstep = P * Gr::COUNT;
+    constexpr int Q  = G::BN / 4 / Gr::NT;  // float4 per thread of a brick
+    fill_segments<DIM>(seg);
+    for (int k = 0, bi = bfirst; k < B::TABS && bi < nb; k++, bi += bstep)
+        fill_neighbours<DIM>(L, bflag, blist[bi], gl, tab + 27 * k);
+    if (threadIdx.x == 0) M.cg = CgScalars{0.0, cg->rr, cg->rr, cg->threshold, 0, cg->max_iter};
+    __syncthreads();
+
+    Outcome o{0.f, 0.f, kGoOn};
+    bool first   = true, ok = true;
+    unsigned tag = cg->tick + 1;
+    CgPhases spent{0, 0, 0};
+    unsigned long long mark = phases ? global_ns() : 0;
+    auto lap = [&](unsigned long long & sum) {
+        if (phases) {
+            const unsigned long long now = global_ns();
+            sum += now - mark;
+            mark = now;
+        }
+    };
+    for (;;) {
+        for (int bi = bfirst; bi < nb; bi += bstep) {
+            const long long base = (long long) blist[bi] * G::BN + 4 * gl;
+#pragma unroll 2
+            for (int k = 0; k < Q; k++) {
+                const long long s = base + 4 * Gr::NT * k;
+                const float4 v    = ld4(N.V, s);
+                float4 d          = ld4(N.d, s);
+                if (!first) {
+                    const float4 q = ld4(N.q, s), x = ld4(N.x, s);
+                    float4 r = ld4(N.r, s);
+                    r        = fma4(-o.alpha, q, r);
+                    st4(N.x, s, fma4(o.alpha, d, x));
+                    st4(N.r, s, r);
+                    d = fma4(o.beta, d, r);
+                    st4(N.d, s, d);
+                }
+                st4(N.u, s, mul4(v, d));
+            }
+        }
+        if (!idle) {
+            Gr::sync();
+            if (gl == 0) {
+                fence_gpu();
+                for (int bi = bfirst; bi < nb; bi += bstep) st_relaxed(flags + blist[bi], tag);
+            }
+        }
+        lap(spent.step);
+
+        FF part[kSums] = {};
+        for (int k = 0, bi = bfirst; bi < nb; bi += bstep, k++) {
+            const int b = blist[bi];
+            int * t     = tab + 27 * min(k, B::TABS);
+            if (k >= B::TABS) {
+                Gr::sync();
+                fill_neighbours<DIM>(L, bflag, b, gl, t);
+                __syncwarp();
+            }
+            if (gl < 32 && !wait_neighbours(flags, t, tag)) ok = false;
+            Gr::sync();  // also past the last brick's reads of the tile
+            tile_copy<DIM, W>(seg, t, N.u, tile);
+            const long long base = (long long) b * G::BN;
+            float q[Gr::NOUT];
+            // with few bricks the row's own operands are loaded under the tile's copy
+            constexpr bool FEW  = W == B::WMAX;
+            constexpr int AHEAD = FEW ? Gr::NOUT / 4 : 1;
+            float4 d_[AHEAD], a_[AHEAD], r_[AHEAD];
+            unsigned f_[AHEAD];
+            auto operands = [&](int i, int at) {
+                const long long s = base + Gr::row(i / Gr::NX) + i % Gr::NX;
+                d_[at] = ld4(N.d, s), a_[at] = ld4(N.ahat, s), r_[at] = ld4(N.r, s);
+                f_[at] = *reinterpret_cast<const unsigned *>(N.flag + s);
+            };
+            if constexpr (FEW) {
+#pragma unroll
+                for (int i = 0; i < Gr::NOUT; i += 4) operands(i, i / 4);
+            }
+            tile_wait<DIM, W>();
+            group_stencil<DIM, W>(tile, S, q);
+#pragma unroll
+            for (int i = 0; i < Gr::NOUT; i += 4) {
+                const long long s = base + Gr::row(i / Gr::NX) + i % Gr::NX;
+                const int at      = FEW ? i / 4 : 0;
+                if constexpr (!FEW) operands(i, 0);
+                const unsigned fl = f_[at];
+                const float4 d = d_[at], a = a_[at], r = r_[at];
+                float p[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    p[j] = (fl >> (8 * j)) & 0xffu ? fmaf(comp(a, j), comp(d, j), q[i + j]) : comp(d, j);
+                    ff_add_prod(part[0], comp(d, j), p[j]);
+                    ff_add_prod(part[1], comp(r, j), p[j]);
+                    ff_add_prod(part[2], p[j], p[j]);
+                    ff_add_prod(part[3], comp(r, j), comp(r, j));
+                }
+                st4(N.q, s, make_float4(p[0], p[1], p[2], p[3]));
+            }
+        }
+        lap(spent.product);
+        o     = meet<B::WARPS>(warp_sum4(part), slots, gridDim.x, P, tag, M, 0.f, false);
+        first = false;
+        if (o.code == kMeasure) {
+#pragma unroll
+            for (int k = 0; k < kSums; k++) part[k] = FF{0.f, 0.f};
+            for (int bi = bfirst; bi < nb; bi += bstep) {
+                const long long base = (long long) blist[bi] * G::BN + 4 * gl;
+                for (int k = 0; k < Q; k++) {
+                    const long long s = base + 4 * Gr::NT * k;
+                    const float4 r    = fma4(-o.alpha, ld4(N.q, s), ld4(N.r, s));
+#pragma unroll
+                    for (int j = 0; j < 4; j++) ff_add_prod(part[0], comp(r, j), comp(r, j));
+                }
+            }
+            o = meet<B::WARPS>(warp_sum4(part), slots, gridDim.x, P, tag, M, o.alpha, true);
+        }
+        lap(spent.meeting);
+        if (o.code != kGoOn) break;
+    }
+    if (!__syncthreads_and(ok)) o.code = kFailed;
+    // the last step of x; a breakdown leaves x = 0
+    if (o.code != kFailed)
+        for (int bi = bfirst; bi < nb; bi += bstep) {
+            const long long base = (long long) blist[bi] * G::BN + 4 * gl;
+#pragma unroll
+            for (int k = 0; k < Q; k++) {
+                const long long s = base + 4 * Gr::NT * k;
+                st4(N.x, s, o.code == 3 ? make_float4(0.f, 0.f, 0.f, 0.f) : fma4(o.alpha, ld4(N.d, s), ld4(N.x, s)));
+            }
+        }
+    if (threadIdx.x == 0) {
+        if (blockIdx.x == 0) {
+            cg->rr      = M.cg.rr_next;
+            cg->rr_prev = M.cg.rr;
+            cg->pq      = M.cg.pq;
+            cg->iter    = M.cg.it;
+            cg->tick    = tag;
+            if (phases) *phases = spent;
+        }
+        if (o.code == kFailed) atomicExch(&cg->failed, 1);
+        else if (blockIdx.x == 0) cg->done = int(o.code);
+    }
+}
+
+// Few bricks: the larger groups take all bricks of a block at once (3D: at most four,
+// where their reads, 2,160 shared-memory wavefronts a brick against 1,250, still cost
+// less than the longer chain of the smaller groups).
+template<int DIM> __device__ __forceinline__ bool few_bricks(int nb, int blocks) {
+    return nb <= blocks * (DIM == 3 ? 4 : Group<DIM, WarpBrick<DIM>::WMAX>::COUNT);
+}
+
+}  // namespace
+
+template<int DIM>
+__global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
+    k_cg_solve(Lattice L, const int * __restrict__ blist, const int * __restrict__ bcount,
+               const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, CgState * cg, ulonglong2 * slots,
+               unsigned * flags, CgPhases * phases) {
+    using B = WarpBrick<DIM>;
+    constexpr int Q = B::G::BN / 4;
+    __shared__ MeetSmem<B::WARPS> M;
+    const int nb   = *bcount;
+    const int done = cg->done;
+    if (done) {
+        // no solve: a zero right-hand side (4) or a start that is not a number (3) leaves x = 0
+        if (done >= 3)
+            for (long long e = blockIdx.x * (long long) B::NT + threadIdx.x; e < (long long) nb * Q;
+                 e += (long long) gridDim.x * B::NT)
+                st4(N.x, (long long) blist[e / Q] * B::G::BN + 4 * (e % Q), make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
+    }
+    const int P = min(int(gridDim.x), nb);
+    if (int(blockIdx.x) >= P) return;
+    if (few_bricks<DIM>(nb, gridDim.x))
+        solve<DIM, B::WMAX>(L, blist, nb, P, bflag, N, S, cg, slots, flags, phases, M);
+    else solve<DIM, B::WMIN>(L, blist, nb, P, bflag, N, S, cg, slots, flags, phases, M);
+}
+
+// Row-stencil passes outside the iteration, the bricks strided over the warps of a
+// resident grid:
+//   kRowsAhat:  alpha_hat = max(-sum_J alpha_IJ, alpha0) from src = V
+//               (calculateCoef, VirtualParticle.cpp:149-169).
+//   kRowsResid: r = b - A x from src = V x: r (and d when non-null) written,
+//               |r|^2 and |b|^2 summed (deterministic) into sums[0..1].
+enum { kRowsAhat = 0, kRowsResid = 1 };
+template<int DIM, int OP, int W>
+__device__ __forceinline__ void rows_of_bricks(const Lattice & L, float alpha0, const int * __restrict__ blist, int nb,
+                                               const unsigned char * __restrict__ bflag, const NodeArrays & N,
+                                               const Stencil & S, const float * __restrict__ src,
+                                               const float * __restrict__ xin, float * __restrict__ r_out,
+                                               float * __restrict__ d_out, FF & rr, FF & bb) {
+    using B  = WarpBrick<DIM>;
+    using Gr = Group<DIM, W>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int grp = Gr::index();
+    if (grp >= Gr::COUNT) return;
+    float * tile   = reinterpret_cast<float *>(smem) + B::T::TILE * grp;
+    int * tab      = reinterpret_cast<int *>(smem + B::kTileBytes) + 27 * (B::TABS + 1) * grp;
+    unsigned * seg = reinterpret_cast<unsigned *>(smem + B::kTileBytes + B::kTabBytes);
+    for (int bi = int(blockIdx.x) + int(gridDim.x) * grp; bi < nb; bi += int(gridDim.x) * Gr::COUNT) {
+        const int b = blist[bi];
+        Gr::sync();  // the last brick's reads of the tile and the table
+        fill_neighbours<DIM>(L, bflag, b, Gr::lane(), tab);
+        Gr::sync();
+        tile_copy<DIM, W>(seg, tab, src, tile);
+        tile_wait<DIM, W>();
+        float q[Gr::NOUT];
+        group_stencil<DIM, W>(tile, S, q);
+#pragma unroll
+        for (int i = 0; i < Gr::NOUT; i += 4) {
+            const long long s = (long long) b * B::G::BN + Gr::row(i / Gr::NX) + i % Gr::NX;
+            const unsigned fl = *reinterpret_cast<const unsigned *>(N.flag + s);
+            float o[4];
+            if (OP == kRowsAhat) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) o[j] = (fl >> (8 * j)) & 0xffu ? fmaxf(-q[i + j], alpha0) : 1.f;
+                st4(N.ahat, s, make_float4(o[0], o[1], o[2], o[3]));
+            } else {
+                const float4 xv = ld4(xin, s), a = ld4(N.ahat, s), bv = ld4(N.D, s);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    o[j] = comp(bv, j) - ((fl >> (8 * j)) & 0xffu ? fmaf(comp(a, j), comp(xv, j), q[i + j]) : comp(xv, j));
+                    ff_add_prod(rr, o[j], o[j]);
+                    ff_add_prod(bb, comp(bv, j), comp(bv, j));
+                }
+                st4(r_out, s, make_float4(o[0], o[1], o[2], o[3]));
+                if (d_out) st4(d_out, s, make_float4(o[0], o[1], o[2], o[3]));
+            }
+        }
+    }
+}
+template<int DIM, int OP>
+__global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
+    k_rows_tiled(Lattice L, float alpha0, const int * __restrict__ blist, const int * __restrict__ bcount,
+                 const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, const float * __restrict__ src,
+                 const float * __restrict__ xin, float * __restrict__ r_out, float * __restrict__ d_out,
+                 double * __restrict__ sums, double * __restrict__ partials, unsigned int * __restrict__ ticket) {
+    using B = WarpBrick<DIM>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double red[B::WARPS + 1];
+    __shared__ int last;
+    fill_segments<DIM>(reinterpret_cast<unsigned *>(smem + B::kTileBytes + B::kTabBytes));
+    __syncthreads();
+    pdl_wait_and_release();
+    const int nb = *bcount;
+    FF rr{0.f, 0.f}, bb{0.f, 0.f};
+    if (few_bricks<DIM>(nb, gridDim.x))
+        rows_of_bricks<DIM, OP, B::WMAX>(L, alpha0, blist, nb, bflag, N, S, src, xin, r_out, d_out, rr, bb);
+    else rows_of_bricks<DIM, OP, B::WMIN>(L, alpha0, blist, nb, bflag, N, S, src, xin, r_out, d_out, rr, bb);
+    if (OP == kRowsResid) {
+        double part[2] = {block_sum_ff<B::NT>(rr, red), 0.0};
+        part[1]        = block_sum_ff<B::NT>(bb, red);
+        double tot[2];
+        if (grid_reduce<B::NT, 2>(part, partials, ticket, tot, red, &last) && threadIdx.x == 0) {
+            sums[0] = tot[0];
+            sums[1] = tot[1];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Launchers
+// ---------------------------------------------------------------------------
+template<int DIM> int cg_solve_prepare() {
+    const int bytes = int(WarpBrick<DIM>::kSmem);
+    auto set = [bytes](auto kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    };
+    return set(k_cg_solve<DIM>) && set(k_rows_tiled<DIM, kRowsAhat>) && set(k_rows_tiled<DIM, kRowsResid>) ? 0 : -1;
+}
+template<int DIM>
+void launch_ahat(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
+                 int blocks, cudaStream_t st) {
+    using W = WarpBrick<DIM>;
+    launch_pdl(k_rows_tiled<DIM, kRowsAhat>, blocks, W::NT, W::kSmem, st, L, P.alpha0, B.list, B.count, B.flag, N, S,
+               N.V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+}
+template<int DIM>
+void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
+                          const float * x, float * r, float * d, double * sums, CgState * cg, double * partials,
+                          int blocks, cudaStream_t st) {
+    using W = WarpBrick<DIM>;
+    launch_pdl(k_rows_tiled<DIM, kRowsResid>, blocks, W::NT, W::kSmem, st, L, 0.f, B.list, B.count, B.flag, N, S, N.u, x,
+               r, d, sums, partials, &cg->ticket[0]);
+}
+template<int DIM>
+int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
+                    ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases, cudaStream_t st) {
+    using W = WarpBrick<DIM>;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = blocks;
+    cfg.blockDim         = W::NT;
+    cfg.dynamicSmemBytes = W::kSmem;
+    cfg.stream           = st;
+    cudaLaunchAttribute at[1];
+    at[0].id              = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs    = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_cg_solve<DIM>, L, (const int *) B.list, (const int *) B.count,
+                              (const unsigned char *) B.flag, N, S, cg, slots, flags, phases) == cudaSuccess
+               ? 0
+               : -1;
+}
+
+#define SWC_INST(D)                                                                                                    \
+    template int cg_solve_prepare<D>();                                                                                \
+    template void launch_ahat<D>(const Lattice &, const Phys &, const BrickArrays &, const NodeArrays &,               \
+                                 const Stencil &, int, cudaStream_t);                                                  \
+    template void launch_rows_residual<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,   \
+                                          const float *, float *, float *, double *, CgState *, double *, int,         \
+                                          cudaStream_t);                                                               \
+    template int launch_cg_solve<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,         \
+                                    CgState *, ulonglong2 *, unsigned *, int, CgPhases *, cudaStream_t);
+SWC_INST(2)
+SWC_INST(3)
+#undef SWC_INST
+
+}  // namespace swc

@@ -496,17 +496,6 @@ __global__ void __launch_bounds__(kNT) k_compact_import(Lattice L, const int * _
     }
 }
 
-template<int DIM>
-__global__ void __launch_bounds__(kNT) k_zero_active(const int * __restrict__ blist, const int * __restrict__ bcount,
-                                                     float * __restrict__ a) {
-    using G      = BrickGeom<DIM>;
-    const int nb = *bcount;
-    for (int bi = blockIdx.x; bi < nb; bi += gridDim.x) {
-        const long long base = (long long) blist[bi] * G::BN;
-        for (int l = threadIdx.x; l < G::BN; l += kNT) a[base + l] = 0.f;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Pressure-gradient update (VirtualParticle::applyPressureGradient,
 // Cores/Structures/VirtualParticle.cpp:111-134):
@@ -616,9 +605,11 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
                                                            const float4 * __restrict__ bvel,
                                                            const float4 * __restrict__ bnrm,
                                                            const int * __restrict__ bcellStart,
-                                                           const unsigned char * __restrict__ bcell, int * queue) {
+                                                           const unsigned char * __restrict__ bcell,
+                                                           const CgState * __restrict__ cg, int * queue) {
     pdl_wait_and_release();
     using G = BrickGeom<DIM>;
+    if (cg->done == 3) return;  // the solve broke down: the velocities stay as they are
     // Row pitch 24 in 3D: a warp's particles span about four consecutive cell
     // rows of one z-plane, whose 8-node windows then fall in disjoint banks
     // (24 dy mod 32 = 0, 24, 16, 8).
@@ -746,10 +737,10 @@ template<int DIM>
 void launch_pressure_gradient(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N,
                               const int * plist, const int * pcount, const unsigned char * bnear, const float4 * pos,
                               float4 * vel, const int * cellStart, const float4 * bpos, const float4 * bvel,
-                              const float4 * bnrm, const int * bcellStart, const unsigned char * bcell, int grid,
-                              int * queue, cudaStream_t st) {
+                              const float4 * bnrm, const int * bcellStart, const unsigned char * bcell,
+                              const CgState * cg, int grid, int * queue, cudaStream_t st) {
     launch_pdl(k_pressure_gradient<DIM>, grid, kGradNT, 0, st, L, P, B.flag, N, plist, pcount, bnear, pos, vel, cellStart, bpos,
-                                                   bvel, bnrm, bcellStart, bcell, queue);
+                                                   bvel, bnrm, bcellStart, bcell, cg, queue);
 }
 template<int DIM> int pressure_gradient_blocks_per_sm() {
     int n = 0;
@@ -829,17 +820,6 @@ void launch_compact_import(const Lattice & L, const BrickArrays & B, const NodeA
     k_compact_import<DIM><<<grid, kNT, 0, st>>>(L, B.list, B.count, B.seg_off, N, in, out);
 }
 
-template<int DIM>
-void launch_zero_active(const Lattice & L, const BrickArrays & B, float * a, int grid, cudaStream_t st) {
-    (void) L;
-    k_zero_active<DIM><<<grid, kNT, 0, st>>>(B.list, B.count, a);
-}
-
-
-
-
-
-
 #define SWC_INST(D)                                                                                                    \
     template void launch_node_gather<D>(const Lattice &, const Phys &, const BrickArrays &, const NodeArrays &,        \
                                         const float4 *, const float4 *, const int *, const float4 *, const float4 *,   \
@@ -848,7 +828,8 @@ void launch_zero_active(const Lattice & L, const BrickArrays & B, float * a, int
     template void launch_pressure_gradient<D>(const Lattice &, const Phys &, const BrickArrays &, const NodeArrays &,  \
                                               const int *, const int *, const unsigned char *, const float4 *,         \
                                               float4 *, const int *, const float4 *, const float4 *, const float4 *,   \
-                                              const int *, const unsigned char *, int, int *, cudaStream_t);           \
+                                              const int *, const unsigned char *, const CgState *, int, int *,         \
+                                              cudaStream_t);                                                           \
     template int pressure_gradient_blocks_per_sm<D>();                                                                 \
     template int node_gather_blocks_per_sm<D>();                                                                       \
     template void launch_segments<D>(const Lattice &, const BrickArrays &, const NodeArrays &, int *, int,             \
@@ -861,8 +842,7 @@ void launch_zero_active(const Lattice & L, const BrickArrays & B, float * a, int
                                            long long *, double *, double *, double *, double *, double *, double *,    \
                                            unsigned short *, int, cudaStream_t);                                       \
     template void launch_compact_import<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const double *,   \
-                                           float *, int, cudaStream_t);                                                \
-    template void launch_zero_active<D>(const Lattice &, const BrickArrays &, float *, int, cudaStream_t);
+                                           float *, int, cudaStream_t);
 SWC_INST(2)
 SWC_INST(3)
 #undef SWC_INST

@@ -1,8 +1,7 @@
 // swc_api.cu -- host orchestration and C ABI of the GB300 dual-particle SPH
 // projection (see include/swc.h).  One context = one simulation on one GPU and
-// one CUDA stream.  The CG loop runs from device-resident scalars; batches of
-// iterations are replayed from captured CUDA graphs between host convergence
-// checks.
+// one CUDA stream.  A step is queued whole, the CG solve as one resident kernel that
+// decides its end on the device (k_cg_solve.cu); the host waits once, at its end.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -37,6 +36,7 @@ constexpr int kPhases = 8;
 
 struct HostCg {
     CgState st;
+    double  res2[2];  // |b - A x|^2, |b|^2 of the true residual
     int     nv;
     int     nbricks;
     int     mlp_err;
@@ -56,8 +56,8 @@ struct swc_ctx {
     Stencil         S{};
     StencilD        SD{};
     int             grid  = 1;  // grid of the 256-thread brick / streaming kernels
-    int             sgrid = 1;  // resident grid of the CG SpMV (static brick striding, deterministic pq)
-    int             rgrid = 1;  // grid of the other row-stencil kernels (one brick per block at a time)
+    int             cgrid = 1;  // grid of the CG solve and the warp-per-brick row passes (one block per SM)
+    int             rgrid = 1;  // grid of the block-per-brick row kernels (true residual, operator)
     int             ggrid = 1;  // resident grid of the virtual gather (brick queue)
     int             pgrid = 1;  // resident grid of the pressure gradient (brick queue)
     int *           queues = nullptr;  // brick queues: gather [0, 2), gradient [2, 4)
@@ -124,11 +124,12 @@ struct swc_ctx {
     unsigned long long * vmax_bits = nullptr;  // max |v|^2 (swc_get_time_step)
     int *       max_bits = nullptr;
     double *    res2 = nullptr;
-    cudaGraphExec_t g1 = nullptr, g8 = nullptr;
+    ulonglong2 *    slots  = nullptr;  // meeting slots of the CG solve (4 x (cgrid + 8))
+    unsigned *      uflags = nullptr;  // and its per-brick flags
+    CgPhases *      phases = nullptr;  // its phase times (swc_time_kernel)
 
     bool   initialized = false;
     double rho0 = 0, alpha0 = -1e6, kappa = 0;
-    int    last_iters = 16;
     bool   profiling = false;
     cudaEvent_t ev[kPhases + 2] = {};
     cudaEvent_t evA = nullptr, evB = nullptr;
@@ -222,10 +223,6 @@ int ensure_extrap_buffers(swc_ctx * c) {
     CK(cudaMemset(c->N.xm1, 0, sizeof(float) * slots));
     CK(cudaMemset(c->N.xm2, 0, sizeof(float) * slots));
     c->extrap_steps = 0;
-    // the CG graphs captured the old NodeArrays: recapture
-    if (c->g1) cudaGraphExecDestroy(c->g1);
-    if (c->g8) cudaGraphExecDestroy(c->g8);
-    c->g1 = c->g8 = nullptr;
     return SWC_OK;
 }
 
@@ -243,10 +240,6 @@ int ensure_learn_buffers(swc_ctx * c) {
     if (!c->N.d2p && (rc = dalloc(c, &c->N.d2p, slots))) return rc;
     CK(cudaMemset(c->N.d2p, 0, sizeof(float) * slots));
     CK(cudaMemset(c->mlp_err, 0, sizeof(int)));
-    // the CG graphs captured the old NodeArrays (feature pointers): recapture
-    if (c->g1) cudaGraphExecDestroy(c->g1);
-    if (c->g8) cudaGraphExecDestroy(c->g8);
-    c->g1 = c->g8 = nullptr;
     return SWC_OK;
 }
 
@@ -330,93 +323,50 @@ template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features =
     launch_node_gather<DIM>(c->L, c->P, c->B, N, c->pos, c->vel, c->cellStart, c->bpos, c->bvel, c->bcellStart,
                             c->bnear, c->bcell, c->ggrid, c->queues, c->stream);
     launch_segments<DIM>(c->L, c->B, c->N, c->scan_tiles, c->grid, c->stream);
-    if (with_ahat) launch_ahat<DIM>(c->L, c->P, c->B, c->N, c->S, c->sgrid, c->stream);
+    if (with_ahat) launch_ahat<DIM>(c->L, c->P, c->B, c->N, c->S, c->cgrid, c->stream);
 }
 
-int capture_graphs(swc_ctx * c) {
-    for (int k = 0; k < 2; k++) {
-        const int reps = k == 0 ? 1 : 8;
-        cudaGraph_t g  = nullptr;
-        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < reps; i++) {
-            if (c->dim == 2)
-                launch_cg_iteration<2>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->sgrid, c->grid, c->stream);
-            else launch_cg_iteration<3>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->sgrid, c->grid, c->stream);
-        }
-        CK(cudaStreamEndCapture(c->stream, &g));
-        cudaGraphExec_t ge = nullptr;
-        CK(cudaGraphInstantiate(&ge, g, 0));
-        cudaGraphDestroy(g);
-        if (k == 0) c->g1 = ge;
-        else c->g8 = ge;
+// Queues the CG solve from the warm start in N.x (with `started`, from the start state
+// that the caller queued) and the copies of its outcome to the host.
+template<int DIM> int queue_cg(swc_ctx * c, bool started) {
+    if (!started)
+        launch_cg_init<DIM>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->opts.tolerance, c->opts.max_iterations,
+                            c->B.seg_off + c->B.nseg, c->cgrid, c->grid, c->stream);
+    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, c->slots, c->uflags, c->cgrid, nullptr, c->stream)) {
+        c->err = std::string("CG solve: ") + cudaGetErrorString(cudaGetLastError());
+        return SWC_CUDA_ERROR;
+    }
+    CK(cudaMemcpyAsync(&c->hcg->st, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&c->hcg->nv, c->B.seg_off + c->B.nseg, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&c->hcg->nbricks, c->B.count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (c->opts.compute_true_residual) {
+        launch_true_residual<DIM>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->res2, c->rgrid, c->stream);
+        CK(cudaMemcpyAsync(c->hcg->res2, c->res2, sizeof(c->hcg->res2), cudaMemcpyDeviceToHost, c->stream));
     }
     return SWC_OK;
 }
 
-// CG solve from the warm start in N.x; fills stats.
-// CG start from the current N.x; the device state is mirrored into hcg.
-// CG start state on entry of run_cg: none (run_cg launches the initialisation),
-// on the device only (launched by the caller), or also copied to the host.
-enum { kInitNone = 0, kInitDevice = 1, kInitHost = 2 };
-
-template<int DIM> int run_cg(swc_ctx * c, swc_stats * st, int init_mode) {
-    if (!c->g1) {
-        CK(cudaStreamSynchronize(c->stream));
-        int rc = capture_graphs(c);
-        if (rc) return rc;
-    }
-    if (init_mode != kInitHost) {
-        // initial residual on the device; its state comes back with the first
-        // convergence check (the iteration kernels are no-ops once CG is done)
-        const int * nv = c->B.seg_off + c->B.nseg;
-        if (init_mode == kInitNone)
-            launch_cg_init<DIM>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->opts.tolerance, c->opts.max_iterations,
-                                nv, c->sgrid, c->grid, c->stream);
-        c->hcg->st.done     = 0;
-        c->hcg->st.iter     = 0;
-        c->hcg->st.max_iter = c->opts.max_iterations >= 0 ? c->opts.max_iterations : std::numeric_limits<int>::max();
-    }
-    // first batch: the last solve's count and one more (one convergence check in
-    // the common case; the iteration kernels are no-ops past convergence)
-    int first   = c->opts.check_interval > 0 ? c->opts.check_interval : std::max(4, c->last_iters + 1);
-    bool counts = init_mode == kInitHost;
-    while (!c->hcg->st.done) {
-        const int room = c->hcg->st.max_iter - c->hcg->st.iter;
-        int m          = std::min(first, std::max(room, 1));
-        for (; m >= 8; m -= 8) CK(cudaGraphLaunch(c->g8, c->stream));
-        for (; m > 0; m--) CK(cudaGraphLaunch(c->g1, c->stream));
-        CK(cudaMemcpyAsync(&c->hcg->st, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost, c->stream));
-        if (!counts) {
-            CK(cudaMemcpyAsync(&c->hcg->nv, c->B.seg_off + c->B.nseg, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaMemcpyAsync(&c->hcg->nbricks, c->B.count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            counts = true;
-        }
-        CK(cudaStreamSynchronize(c->stream));
-        first = c->opts.check_interval > 0 ? c->opts.check_interval : 8;
-    }
-    const double rr0 = c->hcg->st.rr0, bb = c->hcg->st.bb;
+// Status of the solve and its statistics, after the stream was waited for.
+int cg_outcome(swc_ctx * c, swc_stats * st) {
     const CgState & h = c->hcg->st;
     int status        = SWC_OK;
-    if (h.done == 4) launch_zero_active<DIM>(c->L, c->B, c->N.x, c->grid, c->stream);  // b = 0 -> x = 0
     if (h.done == 2) status = SWC_CG_NOT_CONVERGED;
     if (h.done == 3) status = SWC_NAN_DETECTED;
-    c->last_iters = std::max(1, h.iter);
+    if (h.failed) {
+        c->err = "CG solve: the blocks of the resident kernel did not meet in time";
+        status = SWC_CUDA_ERROR;
+    }
     if (st) {
         st->n_virtual            = c->hcg->nv;
         st->active_bricks        = c->hcg->nbricks;
         st->cg_iterations        = h.iter;
-        st->rhs_norm             = std::sqrt(bb);
-        st->rel_residual         = bb > 0 ? std::sqrt(h.rr / bb) : 0.0;
-        st->initial_rel_residual = bb > 0 ? std::sqrt(rr0 / bb) : 0.0;
+        st->rhs_norm             = std::sqrt(h.bb);
+        st->rel_residual         = h.bb > 0 ? std::sqrt(h.rr / h.bb) : 0.0;
+        st->initial_rel_residual = h.bb > 0 ? std::sqrt(h.rr0 / h.bb) : 0.0;
         st->true_rel_residual    = -1;
         st->status               = status;
-    }
-    if (c->opts.compute_true_residual && st) {
-        launch_true_residual<DIM>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->res2, c->rgrid, c->stream);
-        double r2[2];
-        CK(cudaMemcpyAsync(r2, c->res2, sizeof(r2), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        st->true_rel_residual = r2[1] > 0 ? std::sqrt(r2[0] / r2[1]) : 0.0;
+        if (c->opts.compute_true_residual)
+            st->true_rel_residual = c->hcg->res2[1] > 0 ? std::sqrt(c->hcg->res2[0] / c->hcg->res2[1]) : 0.0;
     }
     return status;
 }
@@ -439,8 +389,13 @@ bool history_on(const swc_ctx * c) {
                         (c->opts.keep_features && c->feat_buf));
 }
 
-// The shared tail of advance / project: virtual generation, projection, G_i.
-template<int DIM> int run_projection(swc_ctx * c, swc_stats * st) {
+// The shared tail of advance / project: virtual generation, projection, G_i, queued
+// whole; finish_projection takes what it decided once the stream was waited for.
+struct Projection {
+    int  used = 0, base_used = 0;  // warm start, and the one that a rejected prediction falls back to
+    bool hist_on = false, mlp_checked = false, picked = false, logging = false;
+};
+template<int DIM> int queue_projection(swc_ctx * c, Projection & pr) {
     const int mode     = c->opts.warm_start;
     // the gate skips the network (base start) while it keeps losing the residual test
     const bool gated   = mode == SWC_WARM_LEARNED && c->mlp_ready && c->opts.learned_gate > 0 &&
@@ -454,16 +409,17 @@ template<int DIM> int run_projection(swc_ctx * c, swc_stats * st) {
     mark(c, 4);
     const int * nv     = c->B.seg_off + c->B.nseg;
     const size_t slots = size_t(c->L.nbricks) * BrickGeom<DIM>::BN;
-    int used           = mode;
-    int init_mode      = kInitNone;
-    bool mlp_checked   = false, picked = false;
+    int & used         = pr.used;
+    bool & mlp_checked = pr.mlp_checked, & picked = pr.picked;
+    used               = mode;
+    pr.logging         = logging;
     // Pressure history (extrapolated and learned warm starts, logged features):
     // the base start is 3 p1 - 3 p2 + p3 with three steps of history, 2 p1 - p2
     // with two, p1 (node-mapped) with fewer; the history spans consecutive
     // advance calls.
-    const bool hist_on  = history_on(c);
+    const bool hist_on  = pr.hist_on = history_on(c);
     const int history   = (hist_on && c->extrap_shifted) ? std::min(c->extrap_steps, 2) : 0;
-    const int base_used = history >= 1 ? SWC_WARM_EXTRAPOLATE : SWC_WARM_NODE;
+    const int base_used = pr.base_used = history >= 1 ? SWC_WARM_EXTRAPOLATE : SWC_WARM_NODE;
     if (mode == SWC_WARM_EXTRAPOLATE || mode == SWC_WARM_LEARNED) used = base_used;
     if (learned || logging) {
         // base start (and history shift): the fallback, the network's base and the target reference
@@ -479,7 +435,7 @@ template<int DIM> int run_projection(swc_ctx * c, swc_stats * st) {
         const double * bb = &c->cg->bb;
         if (pick) {
             launch_cg_residual<DIM>(c->L, c->B, c->N, c->S, c->N.x, c->N.q, nullptr, c->cg->sums + 2, c->cg, c->partials,
-                                    c->sgrid, c->grid, c->stream);
+                                    c->cgrid, c->grid, c->stream);
             bb = c->cg->sums + 3;
         }
         if (!pick || logging) launch_rhs_norm<DIM>(c->B, c->N, c->cg, c->partials, c->grid, c->stream);
@@ -491,18 +447,17 @@ template<int DIM> int run_projection(swc_ctx * c, swc_stats * st) {
             launch_mlp_forward_nodes(c->mlp_params, c->mlp_norm, c->N, c->B, DIM == 3 ? 9 : 8, (long long) slots, bb,
                                      inv_a0, inv_r0, inv_nr, c->mlp_err, c->stream);
             CK(cudaMemcpyAsync(&c->hcg->mlp_err, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            mlp_checked = true;  // the error flag is read with CG's first check
+            mlp_checked = true;  // the error flag is read at the step's end
             if (no_fallback) {
                 used = SWC_WARM_LEARNED;  // CG initialises from the prediction
             } else {
                 // residual test on the device: the prediction's residual against the
                 // base start's (computed above), the smaller kept
                 launch_cg_residual<DIM>(c->L, c->B, c->N, c->S, c->N.x, c->N.r, c->N.d, c->cg->sums, c->cg,
-                                        c->partials, c->sgrid, c->grid, c->stream);
+                                        c->partials, c->cgrid, c->grid, c->stream);
                 launch_cg_pick<DIM>(c->B, c->N, c->xprev, c->N.q, c->mlp_err, false, c->cg, c->opts.tolerance,
                                     c->opts.max_iterations, nv, c->grid, c->stream);
-                init_mode = kInitDevice;
-                picked    = true;
+                picked = true;
             }
         } else if (mode == SWC_WARM_NODE) {
             // node-mapped previous pressure, kept in xm1 by the history shift
@@ -520,9 +475,32 @@ template<int DIM> int run_projection(swc_ctx * c, swc_stats * st) {
                                c->pcomp, c->nv_prev, nullptr, c->grid, c->stream);
     }
     mark(c, 5);
-    int rc = run_cg<DIM>(c, st, init_mode);
-    if (picked) {
-        used = c->hcg->st.start == 0 ? SWC_WARM_LEARNED : base_used;
+    int rc;
+    if ((rc = queue_cg<DIM>(c, picked))) return rc;
+    if (logging)
+        launch_mlp_targets(c->L.ncells, nv, c->slot_of, c->N.x, c->xprev, c->N.xm1, c->N.d2p, c->N.ahat, c->cg,
+                           c->tgt_buf, c->stream);
+    mark(c, 6);
+    // leaves the velocities unprojected when the solve broke down (cg->done = 3)
+    launch_pressure_gradient<DIM>(c->L, c->P, c->B, c->N, c->plist, c->pcount, c->bnear, c->pos, c->vel,
+                                  c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->cg, c->pgrid,
+                                  c->queues + 2, c->stream);
+    mark(c, 7);
+    // p in reference order (the next step's prefix warm start) and N_v for it;
+    // other modes skip it (a switch to the prefix mode exports the last solution)
+    if (mode == SWC_WARM_PREFIX) {
+        if ((rc = export_prefix<DIM>(c))) return rc;
+    } else c->pcomp_stale = true;
+    mark(c, 8);
+    return SWC_OK;
+}
+
+int finish_projection(swc_ctx * c, swc_stats * st, const Projection & pr) {
+    const int status = cg_outcome(c, st);
+    if (status == SWC_CUDA_ERROR) return status;
+    int used = pr.used;
+    if (pr.picked) {
+        used = c->hcg->st.start == 0 ? SWC_WARM_LEARNED : pr.base_used;
         if (c->opts.learned_gate > 0) {
             c->gate_rejects = used == SWC_WARM_LEARNED ? 0 : c->gate_rejects + 1;
             if (used == SWC_WARM_LEARNED) c->gate_windows = 0;
@@ -535,45 +513,25 @@ template<int DIM> int run_projection(swc_ctx * c, swc_stats * st) {
             }
         }
     }
-    if (mlp_checked && c->hcg->mlp_err) {
-        c->err = picked ? "learned warm start: the tensor-core pass timed out; CG ran from the base start"
-                        : "learned warm start: the tensor-core pass timed out; CG ran from its output";
-        used   = base_used;
+    if (pr.mlp_checked && c->hcg->mlp_err) {
+        c->err = pr.picked ? "learned warm start: the tensor-core pass timed out; CG ran from the base start"
+                           : "learned warm start: the tensor-core pass timed out; CG ran from its output";
+        used   = pr.base_used;
     }
-    c->extrap_steps   = (hist_on && c->extrap_shifted && (rc == SWC_OK || rc == SWC_CG_NOT_CONVERGED)) ? c->extrap_steps + 1 : 0;
+    const bool solved = status == SWC_OK || status == SWC_CG_NOT_CONVERGED;
+    c->extrap_steps   = pr.hist_on && c->extrap_shifted && solved ? c->extrap_steps + 1 : 0;
     c->extrap_shifted = false;
+    if (pr.logging && solved) c->features_valid = true;
     if (st) st->warm_start_used = used;
-    if (logging && (rc == SWC_OK || rc == SWC_CG_NOT_CONVERGED)) {
-        launch_mlp_targets(c->L.ncells, nv, c->slot_of, c->N.x, c->xprev, c->N.xm1, c->N.d2p, c->N.ahat, c->cg,
-                           c->tgt_buf, c->stream);
-        c->features_valid = true;
-    }
-    if (rc != SWC_OK && rc != SWC_CG_NOT_CONVERGED && rc != SWC_NAN_DETECTED) return rc;
-    const int cg_status = rc;
-    if (cg_status == SWC_NAN_DETECTED) {
-        // report, leave the velocities unprojected and drop the poisoned warm start
-        launch_zero_active<DIM>(c->L, c->B, c->N.x, c->grid, c->stream);
+    if (status == SWC_NAN_DETECTED) {
+        // drop the poisoned warm start
         CK(cudaMemsetAsync(c->nv_prev, 0, sizeof(int), c->stream));
         c->pcomp_stale = false;
-        for (int k = 6; k <= 8; k++) mark(c, k);
-        return cg_status;
+    } else if (st) {
+        st->n_particles = c->n;
+        st->n_boundary  = c->nb;
     }
-    mark(c, 6);
-    launch_pressure_gradient<DIM>(c->L, c->P, c->B, c->N, c->plist, c->pcount, c->bnear, c->pos, c->vel,
-                                  c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->pgrid, c->queues + 2,
-                                  c->stream);
-    mark(c, 7);
-    // p in reference order (the next step's prefix warm start) and N_v for it;
-    // other modes skip it (a switch to the prefix mode exports the last solution)
-    if (mode == SWC_WARM_PREFIX) {
-        if ((rc = export_prefix<DIM>(c))) return rc;
-    } else c->pcomp_stale = true;
-    mark(c, 8);
-    if (st) {
-        st->n_particles     = c->n;
-        st->n_boundary      = c->nb;
-    }
-    return cg_status;
+    return status;
 }
 
 // Activity flags of the previous step (and, for the extrapolated warm start on
@@ -617,11 +575,12 @@ template<int DIM> int do_advance(swc_ctx * c, double dt, swc_stats * st, bool mo
         launch_forces<DIM>(c->pos, c->vel, c->vel2, c->n, c->L, c->P, c->cellStart, float(dt), c->pleft, c->stream);
         std::swap(c->vel, c->vel2);
     }
-    int rc = run_projection<DIM>(c, st);
-    if (rc != SWC_OK && rc != SWC_CG_NOT_CONVERGED && rc != SWC_NAN_DETECTED) return rc;
-    const int status = rc;
+    Projection pr;
+    if (int rc = queue_projection<DIM>(c, pr)) return rc;
     CK(cudaEventRecord(c->evB, c->stream));
     CK(cudaEventSynchronize(c->evB));
+    const int status = finish_projection(c, st, pr);
+    if (status == SWC_CUDA_ERROR) return status;
     float ms = 0;
     cudaEventElapsedTime(&ms, c->evA, c->evB);
     if (st) st->device_ms = ms;
@@ -773,14 +732,18 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
     c->rgrid = std::max(1, std::min(L.nbricks, c->num_sms * 10));
     {
         const bool d3 = s->dim == 3;
-        const int so  = d3 ? cg_spmv_blocks_per_sm<3>() : cg_spmv_blocks_per_sm<2>();
         const int go  = d3 ? node_gather_blocks_per_sm<3>() : node_gather_blocks_per_sm<2>();
         const int po  = d3 ? pressure_gradient_blocks_per_sm<3>() : pressure_gradient_blocks_per_sm<2>();
-        c->sgrid      = std::max(1, std::min(L.nbricks, c->num_sms * so));
+        c->cgrid      = std::max(1, std::min(L.nbricks, c->num_sms));
         c->ggrid      = std::max(1, std::min(L.nbricks, c->num_sms * go));
         c->pgrid      = std::max(1, std::min(L.nbricks, c->num_sms * po));
     }
-    const size_t npart = 3 * size_t(std::max({c->grid, c->sgrid, c->rgrid})) + 8;
+    if (s->dim == 3 ? cg_solve_prepare<3>() : cg_solve_prepare<2>()) {
+        cudaGetLastError();
+        delete c;
+        return SWC_CUDA_ERROR;
+    }
+    const size_t npart = 3 * size_t(std::max({c->grid, c->cgrid, c->rgrid})) + 8;
     setup_phys(c);
     int rc = SWC_OK;
     const size_t slots = size_t(L.nbricks) * bx * by * bz;
@@ -808,6 +771,7 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
     if ((rc = dalloc(c, &c->pcomp, size_t(L.ncells))) || (rc = dalloc(c, &c->nv_prev, 1)) ||
         (rc = dalloc(c, &c->scan_tiles, scan_tile_count(std::max<long long>(c->B.nseg, L.ncells) + 1) + 2)) ||
         (rc = dalloc(c, &c->cg, 1)) || (rc = dalloc(c, &c->partials, npart)) || (rc = dalloc(c, &c->queues, 4)) ||
+        (rc = dalloc(c, &c->slots, 4 * size_t(c->cgrid + 8))) || (rc = dalloc(c, &c->uflags, size_t(L.nbricks))) || (rc = dalloc(c, &c->phases, 1)) ||
         (rc = dalloc(c, &c->diag_bits, 1)) || (rc = dalloc(c, &c->max_bits, 1)) || (rc = dalloc(c, &c->res2, 2)) ||
         (rc = dalloc(c, &c->cellStart, L.ncells + 1)) || (rc = dalloc(c, &c->bcellStart, L.ncells + 1)) ||
         (rc = dalloc(c, &c->bcell, L.ncells)) || (rc = dalloc(c, &c->bcell_tmp, L.ncells)))
@@ -816,6 +780,8 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
     cudaMemsetAsync(c->cg, 0, sizeof(CgState), c->stream);
     cudaMemsetAsync(c->partials, 0, sizeof(double) * npart, c->stream);
     cudaMemsetAsync(c->queues, 0, sizeof(int) * 4, c->stream);
+    cudaMemsetAsync(c->slots, 0, sizeof(ulonglong2) * 4 * size_t(c->cgrid + 8), c->stream);
+    cudaMemsetAsync(c->uflags, 0, sizeof(unsigned) * size_t(L.nbricks), c->stream);
     cudaMemsetAsync(c->B.flag, 0, L.nbricks, c->stream);
     cudaMemsetAsync(c->B.flag_prev, 0, L.nbricks, c->stream);
     cudaMemsetAsync(c->N.flag, 0, slots, c->stream);
@@ -835,8 +801,6 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
 void swc_destroy(swc_ctx * c) {
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    if (c->g1) cudaGraphExecDestroy(c->g1);
-    if (c->g8) cudaGraphExecDestroy(c->g8);
     dfree(c->pos);
     dfree(c->vel);
     dfree(c->vel2);
@@ -900,6 +864,9 @@ void swc_destroy(swc_ctx * c) {
     dfree(c->cg);
     dfree(c->partials);
     dfree(c->queues);
+    dfree(c->slots);
+    dfree(c->uflags);
+    dfree(c->phases);
     dfree(c->diag_bits);
     dfree(c->vmax_bits);
     dfree(c->max_bits);
@@ -916,9 +883,6 @@ void swc_destroy(swc_ctx * c) {
 int swc_set_stream(swc_ctx * c, void * stream) {
     if (!valid_ctx(c)) return SWC_BAD_ARG;
     CK(cudaStreamSynchronize(c->stream));
-    if (c->g1) cudaGraphExecDestroy(c->g1);
-    if (c->g8) cudaGraphExecDestroy(c->g8);
-    c->g1 = c->g8 = nullptr;
     if (c->own_stream) cudaStreamDestroy(c->stream);
     if (stream) {
         c->stream     = static_cast<cudaStream_t>(stream);
@@ -944,12 +908,7 @@ int swc_set_solver_opts(swc_ctx * c, const swc_solver_opts * o) {
     c->gate_rejects = c->gate_skip = c->gate_windows = 0;
     const size_t slots = size_t(c->L.nbricks) * (c->dim == 3 ? 512 : 256);
     int rc;
-    if (need_vbar || need_feat) {
-        CK(cudaStreamSynchronize(c->stream));
-        if (c->g1) cudaGraphExecDestroy(c->g1);
-        if (c->g8) cudaGraphExecDestroy(c->g8);
-        c->g1 = c->g8 = nullptr;
-    }
+    if (need_vbar || need_feat) CK(cudaStreamSynchronize(c->stream));
     if (need_vbar && (rc = dalloc(c, &c->N.vbar, slots))) return rc;
     if (need_feat && (rc = ensure_learn_buffers(c))) return rc;
     if (o->warm_start == SWC_WARM_EXTRAPOLATE && !c->N.xm1) {
@@ -1352,20 +1311,17 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
     if (!valid_ctx(c) || !mean_ms || reps <= 0 || !c->initialized || which < 0 || which > 7) return SWC_BAD_ARG;
     if (which == 7 && !c->mlp_ready) return SWC_BAD_ARG;  // needs a network (swc_set_mlp)
     CK(cudaStreamSynchronize(c->stream));
-    // keep the solver state: run the CG kernels against a scratch copy of the scalars
+    const bool solve = which == 0 || which == 1 || which == 6;
+    if (solve && c->dim != 3) {
+        *mean_ms = 0;  // as for every kernel that is timed in 3D only
+        return SWC_OK;
+    }
+    // keep the solver state: the CG scalars, and the vectors the timed kernel writes
     CgState saved{};
     CK(cudaMemcpy(&saved, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost));
-    CgState run = saved;
-    run.done      = 0;
-    run.iter      = 2;  // beta path of the SpMV
-    run.threshold = 0;  // never converge while timing
-    run.max_iter  = 0x7fffffff;
-    if (!(run.rr_prev > 0)) run.rr_prev = 1, run.rr = 1;
-    if (!(run.pq != 0)) run.pq = 1;
-    CK(cudaMemcpy(c->cg, &run, sizeof(CgState), cudaMemcpyHostToDevice));
     float * x_save = nullptr;
     const size_t slots = size_t(c->L.nbricks) * (c->dim == 3 ? 512 : 256);
-    if (which == 1 || which == 7) {
+    if (solve || which == 7) {
         CK(cudaMalloc(&x_save, sizeof(float) * slots * 2));
         cudaMemcpy(x_save, c->N.x, sizeof(float) * slots, cudaMemcpyDeviceToDevice);
         cudaMemcpy(x_save + slots, c->N.r, sizeof(float) * slots, cudaMemcpyDeviceToDevice);
@@ -1384,17 +1340,14 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         }
         if (c->dim == 3) {
             switch (which) {
-            case 0: launch_cg_spmv<3>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->sgrid, c->stream); break;
-            case 1: launch_cg_update<3>(c->B, c->N, c->cg, c->partials, c->grid, c->stream); break;
-            case 6: launch_cg_direction<3>(c->B, c->N, c->cg, c->grid, c->stream); break;
             case 2:
                 launch_node_gather<3>(c->L, c->P, c->B, c->N, c->pos, c->vel, c->cellStart, c->bpos, c->bvel,
                                       c->bcellStart, c->bnear, c->bcell, c->ggrid, c->queues, c->stream);
                 break;
             case 3:
                 launch_pressure_gradient<3>(c->L, c->P, c->B, c->N, c->plist, c->pcount, c->bnear, c->pos, c->vel,
-                                            c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->pgrid,
-                                            c->queues + 2, c->stream);
+                                            c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->cg,
+                                            c->pgrid, c->queues + 2, c->stream);
                 break;
             case 4: launch_density<3>(c->pos, c->vel, c->rho, c->n, c->L, c->P, c->cellStart, c->pleft, c->stream); break;
             case 5: launch_forces<3>(c->pos, c->vel, c->vel2, c->n, c->L, c->P, c->cellStart, 0.f, c->pleft, c->stream); break;
@@ -1410,14 +1363,33 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
             }
         }
     };
-    launch();  // warm
-    CK(cudaEventRecord(c->evA, c->stream));
-    for (int k = 0; k < reps; k++) launch();
-    CK(cudaEventRecord(c->evB, c->stream));
-    CK(cudaEventSynchronize(c->evB));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, c->evA, c->evB);
-    *mean_ms = ms / reps;
+    if (solve) {
+        // `reps` iterations of the resident solve from the last right-hand side and a zero
+        // start, the phases' own times
+        CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
+        CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
+        for (int k = 0; k < 2; k++) {  // warm, then timed
+            launch_cg_init<3>(c->L, c->B, c->N, c->S, c->cg, c->partials, 0.0, reps, c->B.seg_off + c->B.nseg, c->cgrid, c->grid, c->stream);
+            launch_cg_solve<3>(c->L, c->B, c->N, c->S, c->cg, c->slots, c->uflags, c->cgrid, c->phases,
+                               c->stream);
+            CK(cudaStreamSynchronize(c->stream));
+        }
+        CgPhases ph{};
+        CgState run{};
+        CK(cudaMemcpy(&ph, c->phases, sizeof(ph), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(&run, c->cg, sizeof(run), cudaMemcpyDeviceToHost));
+        saved.tick = run.tick;  // the meetings' tags are not used twice
+        *mean_ms = 1e-6 * double(which == 0 ? ph.product : which == 1 ? ph.meeting : ph.step) / std::max(run.iter, 1);
+    } else {
+        launch();  // warm
+        CK(cudaEventRecord(c->evA, c->stream));
+        for (int k = 0; k < reps; k++) launch();
+        CK(cudaEventRecord(c->evB, c->stream));
+        CK(cudaEventSynchronize(c->evB));
+        float ms = 0;
+        cudaEventElapsedTime(&ms, c->evA, c->evB);
+        *mean_ms = ms / reps;
+    }
     CK(cudaMemcpy(c->cg, &saved, sizeof(CgState), cudaMemcpyHostToDevice));
     if (x_save) {
         cudaMemcpy(c->N.x, x_save, sizeof(float) * slots, cudaMemcpyDeviceToDevice);

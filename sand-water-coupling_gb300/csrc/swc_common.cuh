@@ -511,12 +511,20 @@ struct CgState {
     double threshold;  // max(tol^2 |b|^2, DBL_MIN)
     double rr0;        // initial |r_0|^2
     int    iter;       // completed iterations (SpMV count in the loop)
-    int    done;       // 0 running, 1 converged, 2 max iterations, 3 breakdown / NaN
+    int    done;       // 0 running, 1 converged, 2 max iterations, 3 breakdown / NaN, 4 b = 0
     int    max_iter;
     int    start;      // start kept by k_cg_start: 0 prediction, 1 base
     double sums[4];    // residual sums of the CG start: |r|^2, |b|^2 (prediction / only start), |r|^2, |b|^2 (base)
     unsigned int ticket[4];
-    int    is_last[4];
+    unsigned int tick;  // meetings of the solves so far: the tags of the next solve's follow
+    int    failed;      // a block of the solve waited in vain
+};
+
+// Times of the solve's phases, summed over the iterations (ns, as the first warp of
+// block 0 saw them; written when asked for): the step of x, r, d and u, the product with
+// the wait for the neighbours' u, the meeting for the sums.
+struct CgPhases {
+    unsigned long long step, product, meeting;
 };
 
 }  // namespace swc

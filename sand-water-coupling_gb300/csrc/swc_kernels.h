@@ -130,20 +130,19 @@ template<int DIM>
 void launch_pressure_gradient(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N,
                               const int * plist, const int * pcount, const unsigned char * bnear, const float4 * pos,
                               float4 * vel, const int * cellStart, const float4 * bpos, const float4 * bvel,
-                              const float4 * bnrm, const int * bcellStart, const unsigned char * bcell, int grid,
-                              int * queue, cudaStream_t st);
+                              const float4 * bnrm, const int * bcellStart, const unsigned char * bcell,
+                              const CgState * cg, int grid, int * queue, cudaStream_t st);
 // Resident blocks per SM of the persistent brick kernels (their grids are
 // SMs x this; gather and gradient take bricks from a zero-initialised queue of
 // two ints).
 template<int DIM> int node_gather_blocks_per_sm();
 template<int DIM> int pressure_gradient_blocks_per_sm();
-template<int DIM> int cg_spmv_blocks_per_sm();
 template<int DIM>
 void launch_segments(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int * tiles, int grid,
                      cudaStream_t st);
 template<int DIM>
 void launch_ahat(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
-                 int sgrid, cudaStream_t st);
+                 int blocks, cudaStream_t st);
 template<int DIM>
 void launch_diag_max_f64(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const StencilD & S,
                          unsigned long long * out_bits, int grid, cudaStream_t st);
@@ -157,17 +156,29 @@ template<int DIM>
 void launch_compact_export(const Lattice & L, const BrickArrays & B, const NodeArrays & N, float * pcomp,
                            long long * node_id, double * rho, double * vol, double * vbar, double * div,
                            double * ahat, double * p, unsigned short * nreal_out, int grid, cudaStream_t st);
-// CG
+// CG.  The solve is one resident kernel (k_cg_solve.cu) on `blocks` blocks, one per
+// SM; `slots` (4 x (blocks + 8)) and `flags` (one per brick), zeroed once at allocation, are its
+// meeting slots and the bricks' flags.
+// A failed launch returns nonzero; a wait that times out sets cg->failed.
+// cg_solve_prepare sets the kernels' shared-memory attribute on the current device.
+template<int DIM> int cg_solve_prepare();
+template<int DIM>
+int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
+                    ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases, cudaStream_t st);
+template<int DIM>
+void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
+                          const float * x, float * r, float * d, double * sums, CgState * cg, double * partials,
+                          int blocks, cudaStream_t st);
 template<int DIM>
 void launch_cg_init(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    double * partials, double tol, int max_iterations, const int * nv, int sgrid, int ugrid,
+                    double * partials, double tol, int max_iterations, const int * nv, int rblocks, int ugrid,
                     cudaStream_t st);
 // Residual r = b - A x of one candidate CG start (r, and d when non-null;
 // |r|^2, |b|^2 into sums[0..1]).
 template<int DIM>
 void launch_cg_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                         const float * x, float * r, float * d, double * sums, CgState * cg, double * partials,
-                        int sgrid, int ugrid, cudaStream_t st);
+                        int rblocks, int ugrid, cudaStream_t st);
 // CG start from the better of the prediction (N.x, residual sums in cg->sums[0..1])
 // and the base start xb (cg->sums[2..3], residual rb), decided on the device
 // (cg->start: 0 prediction, 1 base); keep_prediction skips the comparison.
@@ -176,21 +187,8 @@ void launch_cg_pick(const BrickArrays & B, const NodeArrays & N, const float * x
                     const int * mlp_err, bool keep_prediction, CgState * cg, double tol, int max_iterations,
                     const int * nv, int ugrid, cudaStream_t st);
 template<int DIM>
-void launch_cg_iteration(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
-                         CgState * cg, double * partials, int sgrid, int ugrid, cudaStream_t st);
-template<int DIM>
-void launch_cg_direction(const BrickArrays & B, const NodeArrays & N, const CgState * cg, int ugrid, cudaStream_t st);
-template<int DIM>
-void launch_cg_spmv(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    double * partials, int sgrid, cudaStream_t st);
-template<int DIM>
-void launch_cg_update(const BrickArrays & B, const NodeArrays & N, CgState * cg, double * partials, int ugrid,
-                      cudaStream_t st);
-template<int DIM>
 void launch_apply_operator(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                            const float * in, float * out, int sgrid, cudaStream_t st);
-template<int DIM>
-void launch_zero_active(const Lattice & L, const BrickArrays & B, float * a, int grid, cudaStream_t st);
 template<int DIM>
 void launch_compact_import(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const double * in,
                            float * out, int grid, cudaStream_t st);

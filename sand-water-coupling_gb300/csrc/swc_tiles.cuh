@@ -140,20 +140,19 @@ __device__ __forceinline__ void load_tile4(const Lattice & L, const unsigned cha
     }
 }
 
-// Row stencil over a halo tile with row pitch PX, TY rows per z-plane, y/z
-// halos HY/HZ and an x halo of 4 (rows start 16-byte aligned): the BX outputs
-// of brick row (ly, lz),
-//   out[i] = sum_{0 < |k|^2 < 16} c(|k|^2) tile[node (i, ly, lz) + k].
+// Row stencil over a halo tile with row pitch PX and TY rows per z-plane (rows start
+// 16-byte aligned): the NX outputs next to `centre` + 4 (the tile's float four before
+// the first output),
+//   out[i] = sum_{0 < |k|^2 < 16} c(|k|^2) tile[node i + k].
 // The 45 (dy, dz) rows within reach (7 in 2D) fall into classes of equal
 // m = dy^2 + dz^2 (9 in 3D: 0 1 2 4 5 8 9 10 13; 4 in 2D), and all rows of a
 // class share the x-coefficients c(dx^2 + m).  The rows of a class are summed
 // first (T_m) and the 1D x-convolution is applied once per class, so in 3D a
 // row of 8 outputs costs 45 row loads, 450 adds and 416 FMAs instead of 2000
 // FMAs.
-template<int DIM, int PX, int TY, int M>
-__device__ __forceinline__ void stencil_class(const float * centre, const Stencil & S,
-                                              float (&out)[BrickGeom<DIM>::BX]) {
-    constexpr int BX = BrickGeom<DIM>::BX, TX = BX + 8;
+template<int DIM, int PX, int TY, int NX, int M>
+__device__ __forceinline__ void stencil_class(const float * centre, const Stencil & S, float (&out)[NX]) {
+    constexpr int TX = NX + 8;
     constexpr int ZR = DIM == 3 ? 3 : 0;
     constexpr int R  = M <= 6 ? 3 : (M <= 11 ? 2 : 1);  // x reach: dx^2 + M <= 15
     float T[TX];
@@ -170,7 +169,7 @@ __device__ __forceinline__ void stencil_class(const float * centre, const Stenci
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     const int k = 4 * s + j;
-                    if (k < 4 - R || k > BX + 3 + R) continue;
+                    if (k < 4 - R || k > NX + 3 + R) continue;
                     const float v = j == 0 ? t.x : (j == 1 ? t.y : (j == 2 ? t.z : t.w));
                     T[k]          = have ? T[k] + v : v;
                 }
@@ -182,69 +181,47 @@ __device__ __forceinline__ void stencil_class(const float * centre, const Stenci
         if (dx == 0 && M == 0) continue;
         const float c = S.c[dx * dx + M];
 #pragma unroll
-        for (int i = 0; i < BX; i++) out[i] = fmaf(c, T[i + 4 + dx], out[i]);
+        for (int i = 0; i < NX; i++) out[i] = fmaf(c, T[i + 4 + dx], out[i]);
     }
 }
 
-template<int DIM, int PX, int TY, int HY, int HZ>
-__device__ __forceinline__ void stencil_row_t(const float * tile, int ly, int lz, const Stencil & S,
-                                              float (&out)[BrickGeom<DIM>::BX]) {
-    constexpr int BX     = BrickGeom<DIM>::BX;
-    const float * centre = tile + PX * ((ly + HY) + TY * (DIM == 3 ? lz + HZ : 0));
+template<int DIM, int PX, int TY, int NX>
+__device__ __forceinline__ void stencil_row_t(const float * centre, const Stencil & S, float (&out)[NX]) {
 #pragma unroll
-    for (int i = 0; i < BX; i++) out[i] = 0.f;
-    stencil_class<DIM, PX, TY, 0>(centre, S, out);
-    stencil_class<DIM, PX, TY, 1>(centre, S, out);
-    if constexpr (DIM == 3) stencil_class<DIM, PX, TY, 2>(centre, S, out);
-    stencil_class<DIM, PX, TY, 4>(centre, S, out);
+    for (int i = 0; i < NX; i++) out[i] = 0.f;
+    stencil_class<DIM, PX, TY, NX, 0>(centre, S, out);
+    stencil_class<DIM, PX, TY, NX, 1>(centre, S, out);
+    if constexpr (DIM == 3) stencil_class<DIM, PX, TY, NX, 2>(centre, S, out);
+    stencil_class<DIM, PX, TY, NX, 4>(centre, S, out);
     if constexpr (DIM == 3) {
-        stencil_class<DIM, PX, TY, 5>(centre, S, out);
-        stencil_class<DIM, PX, TY, 8>(centre, S, out);
+        stencil_class<DIM, PX, TY, NX, 5>(centre, S, out);
+        stencil_class<DIM, PX, TY, NX, 8>(centre, S, out);
     }
-    stencil_class<DIM, PX, TY, 9>(centre, S, out);
+    stencil_class<DIM, PX, TY, NX, 9>(centre, S, out);
     if constexpr (DIM == 3) {
-        stencil_class<DIM, PX, TY, 10>(centre, S, out);
-        stencil_class<DIM, PX, TY, 13>(centre, S, out);
+        stencil_class<DIM, PX, TY, NX, 10>(centre, S, out);
+        stencil_class<DIM, PX, TY, NX, 13>(centre, S, out);
     }
 }
 
-// Row stencil over a brick-geometry tile (halo 4 on every side).
+// Row stencil over a brick-geometry tile (halo 4 on every side): the outputs of brick
+// row (ly, lz).
 template<int DIM>
 __device__ __forceinline__ void stencil_row(const float * tile, int ly, int lz, const Stencil & S,
                                             float (&out)[BrickGeom<DIM>::BX]) {
     using G = BrickGeom<DIM>;
-    stencil_row_t<DIM, G::PX, G::TY, G::HALO, G::HALO>(tile, ly, lz, S, out);
+    stencil_row_t<DIM, G::PX, G::TY, G::BX>(
+        tile + G::PX * ((ly + G::HALO) + G::TY * (DIM == 3 ? lz + G::HALO : 0)), S, out);
 }
 
 // Halo tile of the CG SpMV: x halo 4 (16-byte aligned rows), y/z halo 3 (the
 // stencil reach), pitch chosen so the 8 rows read by a quarter-warp's LDS.128
-// hit distinct banks.
+// hit distinct banks.  16-byte copies, zero-filled when !valid.
 __device__ __forceinline__ void cp_async16(float * smem_dst, const float * gsrc, bool valid) {
     const unsigned sa = unsigned(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gsrc), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-
-// cp.async 16-byte copies (zero-filled when !valid) and their groups.
-// Neighbour-brick table of brick b: tab[(k+1)*9 + (j+1)*3 + (i+1)] = id of brick
-// (bx+i, by+j, bz+k) when it exists and is active, else -1.
-template<int DIM>
-__device__ __forceinline__ void neighbour_table(const Lattice & L, const unsigned char * __restrict__ bflag, int b,
-                                                int * tab) {
-    const int t = threadIdx.x;
-    if (t < 27) {
-        const int3 bc = brick_coords(L, b);
-        const int i = t % 3 - 1, j = (t / 3) % 3 - 1, k = t / 9 - 1;
-        const int x = bc.x + i, y = bc.y + j, z = bc.z + k;
-        int id = -1;
-        if (x >= 0 && x < L.bnx && y >= 0 && y < L.bny && z >= 0 && z < L.bnz && (DIM == 3 || k == 0)) {
-            const int nb = x + L.bnx * (y + L.bny * z);
-            if (bflag[nb]) id = nb;
-        }
-        tab[t] = id;
-    }
-}
 
 template<int DIM> struct SpmvTile {
     using G = BrickGeom<DIM>;
