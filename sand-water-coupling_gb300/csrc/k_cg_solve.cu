@@ -455,7 +455,9 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
 //               (calculateCoef, VirtualParticle.cpp:149-169).
 //   kRowsResid: r = b - A x from src = V x: r (and d when non-null) written,
 //               |r|^2 and |b|^2 summed (deterministic) into sums[0..1].
-enum { kRowsAhat = 0, kRowsResid = 1 };
+//   kRowsDiag:  the diagonal -sum_J alpha_IJ itself (0 on inactive nodes) into N.ahat and
+//               its maximum, as the bits of a non-negative float, into *top.
+enum { kRowsAhat = 0, kRowsResid = 1, kRowsDiag = 2 };
 template<int DIM, int OP, int W>
 __device__ __forceinline__ void rows_of_bricks(const Lattice & L, float alpha0, const int * __restrict__ blist, int nb,
                                                const unsigned char * __restrict__ bflag, const NodeArrays & N,
@@ -488,6 +490,13 @@ __device__ __forceinline__ void rows_of_bricks(const Lattice & L, float alpha0, 
 #pragma unroll
                 for (int j = 0; j < 4; j++) o[j] = (fl >> (8 * j)) & 0xffu ? fmaxf(-q[i + j], alpha0) : 1.f;
                 st4(N.ahat, s, make_float4(o[0], o[1], o[2], o[3]));
+            } else if (OP == kRowsDiag) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    o[j]  = (fl >> (8 * j)) & 0xffu ? fmaxf(-q[i + j], 0.f) : 0.f;
+                    rr.hi = fmaxf(rr.hi, o[j]);
+                }
+                st4(N.ahat, s, make_float4(o[0], o[1], o[2], o[3]));
             } else {
                 const float4 xv = ld4(xin, s), a = ld4(N.ahat, s), bv = ld4(N.D, s);
 #pragma unroll
@@ -507,7 +516,8 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     k_rows_tiled(Lattice L, float alpha0, const int * __restrict__ blist, const int * __restrict__ bcount,
                  const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, const float * __restrict__ src,
                  const float * __restrict__ xin, float * __restrict__ r_out, float * __restrict__ d_out,
-                 double * __restrict__ sums, double * __restrict__ partials, unsigned int * __restrict__ ticket) {
+                 double * __restrict__ sums, double * __restrict__ partials, unsigned int * __restrict__ ticket,
+                 unsigned int * __restrict__ top) {
     using B = WarpBrick<DIM>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double red[B::WARPS + 1];
@@ -520,6 +530,10 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     if (few_bricks<DIM>(nb, gridDim.x))
         rows_of_bricks<DIM, OP, B::WMAX>(L, alpha0, blist, nb, bflag, N, S, src, xin, r_out, d_out, rr, bb);
     else rows_of_bricks<DIM, OP, B::WMIN>(L, alpha0, blist, nb, bflag, N, S, src, xin, r_out, d_out, rr, bb);
+    if (OP == kRowsDiag) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(rr.hi));
+        if ((threadIdx.x & 31) == 0) atomicMax(top, m);
+    }
     if (OP == kRowsResid) {
         double part[2] = {block_sum_ff<B::NT>(rr, red), 0.0};
         part[1]        = block_sum_ff<B::NT>(bb, red);
@@ -531,6 +545,44 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     }
 }
 
+// alpha0 calibration (VirtualParticle::setAlpha, VirtualParticle.cpp:64-73): the maximum
+// over active nodes of -sum_J alpha_IJ in FP64, among the nodes whose FP32 diagonal
+// (kRowsDiag) is within 1e-4 of the largest one.  The FP32 value is a sum of at most 250
+// terms of one sign, so it is within 250 x 2^-24 = 1.5e-5 of the FP64 value and the node
+// of the FP64 maximum is one of them.  (All nodes in FP64: 250 multiply-adds a node on a
+// pipe of two per SM and clock, 2.26 ms at 2.25M nodes; this pass with the FP32 one
+// takes 0.06.)
+template<int DIM>
+__global__ void __launch_bounds__(256)
+    k_diag_max_f64(Lattice L, const int * __restrict__ blist, const int * __restrict__ bcount,
+                   const unsigned char * __restrict__ bflag, NodeArrays N, StencilD S,
+                   const unsigned int * __restrict__ top, unsigned long long * __restrict__ out_bits) {
+    pdl_wait_and_release();
+    using G           = BrickGeom<DIM>;
+    constexpr int ZR  = DIM == 3 ? 3 : 0;
+    const float bound = __uint_as_float(*top) * (1.f - 1e-4f);
+    const long long n = (long long) *bcount * G::BN;
+    for (long long e = blockIdx.x * 256LL + threadIdx.x; e < n; e += (long long) gridDim.x * 256) {
+        const int b = blist[e / G::BN], l = int(e % G::BN);
+        const long long s = (long long) b * G::BN + l;
+        if (!N.flag[s] || N.ahat[s] < bound) continue;
+        const int3 bc = brick_coords(L, b);
+        const int x = bc.x * G::BX + l % G::BX, y = bc.y * G::BY + (l / G::BX) % G::BY,
+                  z = DIM == 3 ? bc.z * G::BZ + l / (G::BX * G::BY) : 0;
+        double acc = 0;
+        for (int dz = -ZR; dz <= ZR; dz++)
+            for (int dy = -3; dy <= 3; dy++)
+                for (int dx = -3; dx <= 3; dx++) {
+                    const int r2 = dx * dx + dy * dy + dz * dz, X = x + dx, Y = y + dy, Z = z + dz;
+                    if (r2 == 0 || r2 >= 16 || X < 0 || X >= L.nx || Y < 0 || Y >= L.ny || Z < 0 || Z >= L.nz) continue;
+                    if (!bflag[brick_of(L, X, Y, Z, G::BX, G::BY, G::BZ)]) continue;
+                    acc += S.c[r2] * double(N.V[node_slot<DIM>(L, X, Y, Z)]);
+                }
+        // positive doubles order like their bit patterns; the diagonal is >= 0
+        if (-acc >= 0) atomicMax(out_bits, (unsigned long long) __double_as_longlong(-acc));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
@@ -539,14 +591,28 @@ template<int DIM> int cg_solve_prepare() {
     auto set = [bytes](auto kernel) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
-    return set(k_cg_solve<DIM>) && set(k_rows_tiled<DIM, kRowsAhat>) && set(k_rows_tiled<DIM, kRowsResid>) ? 0 : -1;
+    return set(k_cg_solve<DIM>) && set(k_rows_tiled<DIM, kRowsAhat>) && set(k_rows_tiled<DIM, kRowsResid>) &&
+                   set(k_rows_tiled<DIM, kRowsDiag>)
+               ? 0
+               : -1;
 }
 template<int DIM>
 void launch_ahat(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                  int blocks, cudaStream_t st) {
     using W = WarpBrick<DIM>;
     launch_pdl(k_rows_tiled<DIM, kRowsAhat>, blocks, W::NT, W::kSmem, st, L, P.alpha0, B.list, B.count, B.flag, N, S,
-               N.V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+               N.V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+}
+template<int DIM>
+void launch_diag_max_f64(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
+                         const StencilD & SD, unsigned int * top, unsigned long long * out_bits, int blocks, int grid,
+                         cudaStream_t st) {
+    using W = WarpBrick<DIM>;
+    cudaMemsetAsync(top, 0, sizeof(unsigned int), st);
+    cudaMemsetAsync(out_bits, 0, sizeof(unsigned long long), st);
+    launch_pdl(k_rows_tiled<DIM, kRowsDiag>, blocks, W::NT, W::kSmem, st, L, 0.f, B.list, B.count, B.flag, N, S, N.V,
+               nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, top);
+    launch_pdl(k_diag_max_f64<DIM>, grid, 256, 0, st, L, B.list, B.count, B.flag, N, SD, top, out_bits);
 }
 template<int DIM>
 void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
@@ -554,7 +620,7 @@ void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeAr
                           int blocks, cudaStream_t st) {
     using W = WarpBrick<DIM>;
     launch_pdl(k_rows_tiled<DIM, kRowsResid>, blocks, W::NT, W::kSmem, st, L, 0.f, B.list, B.count, B.flag, N, S, N.u, x,
-               r, d, sums, partials, &cg->ticket[0]);
+               r, d, sums, partials, &cg->ticket[0], nullptr);
 }
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
@@ -583,6 +649,9 @@ int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays &
     template void launch_rows_residual<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,   \
                                           const float *, float *, float *, double *, CgState *, double *, int,         \
                                           cudaStream_t);                                                               \
+    template void launch_diag_max_f64<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,    \
+                                         const StencilD &, unsigned int *, unsigned long long *, int, int,             \
+                                         cudaStream_t);                                                                \
     template int launch_cg_solve<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,         \
                                     CgState *, ulonglong2 *, unsigned *, int, CgPhases *, cudaStream_t);
 SWC_INST(2)

@@ -313,32 +313,6 @@ __global__ void __launch_bounds__(kNT) k_segment_count(Lattice L, const int * __
     }
 }
 
-// alpha0 calibration (VirtualParticle::setAlpha, VirtualParticle.cpp:64-73):
-// max over active nodes of -sum_J alpha_IJ, accumulated in FP64.
-template<int DIM>
-__global__ void __launch_bounds__(kNT) k_diag_max_f64(Lattice L, const int * __restrict__ blist,
-                                                      const int * __restrict__ bcount,
-                                                      const unsigned char * __restrict__ bflag, NodeArrays N,
-                                                      StencilD S, unsigned long long * __restrict__ out_bits) {
-    using G = BrickGeom<DIM>;
-    __shared__ float tile[G::TILE];
-    const int nb = *bcount;
-    double m     = -1e300;
-    for (int bi = blockIdx.x; bi < nb; bi += gridDim.x) {
-        const int b   = blist[bi];
-        const int3 bc = brick_coords(L, b);
-        __syncthreads();
-        load_tile<DIM>(L, bflag, bc, tile, [&](long long s) { return N.V[s]; });
-        __syncthreads();
-        for (int l = threadIdx.x; l < G::BN; l += kNT) {
-            const long long s = (long long) b * G::BN + l;
-            if (N.flag[s]) m = fmax(m, -stencil_apply_d<DIM>(tile, tile_center<DIM>(l), S));
-        }
-    }
-    // positive doubles order like their bit patterns; the diagonal is >= 0
-    if (m >= 0) atomicMax(out_bits, (unsigned long long) __double_as_longlong(m));
-}
-
 // ---------------------------------------------------------------------------
 // Warm start of the CG solution vector x (in place; x keeps the previous
 // step's pressure in the same lattice slots).
@@ -786,13 +760,6 @@ void launch_segments(const Lattice & L, const BrickArrays & B, const NodeArrays 
 
 
 template<int DIM>
-void launch_diag_max_f64(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const StencilD & S,
-                         unsigned long long * out_bits, int grid, cudaStream_t st) {
-    cudaMemsetAsync(out_bits, 0, sizeof(unsigned long long), st);
-    k_diag_max_f64<DIM><<<grid, kNT, 0, st>>>(L, B.list, B.count, B.flag, N, S, out_bits);
-}
-
-template<int DIM>
 void launch_warm_start(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int mode, const float * pcomp,
                        const int * nv_prev, const float * given, int grid, cudaStream_t st, int history) {
     if (mode == kWarmExtrap) {
@@ -834,8 +801,6 @@ void launch_compact_import(const Lattice & L, const BrickArrays & B, const NodeA
     template int node_gather_blocks_per_sm<D>();                                                                       \
     template void launch_segments<D>(const Lattice &, const BrickArrays &, const NodeArrays &, int *, int,             \
                                      cudaStream_t);                                                                    \
-    template void launch_diag_max_f64<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const StencilD &,   \
-                                         unsigned long long *, int, cudaStream_t);                                     \
     template void launch_warm_start<D>(const Lattice &, const BrickArrays &, const NodeArrays &, int, const float *,   \
                                        const int *, const float *, int, cudaStream_t, int);                            \
     template void launch_compact_export<D>(const Lattice &, const BrickArrays &, const NodeArrays &, float *,          \

@@ -632,7 +632,8 @@ template<int DIM> int do_initialize(swc_ctx * c) {
     setup_phys(c);
     // alpha0 = max diagonal with the clamp off, in FP64 (VirtualParticle::setAlpha)
     run_generate<DIM>(c, false);
-    launch_diag_max_f64<DIM>(c->L, c->B, c->N, c->SD, c->diag_bits, c->grid, c->stream);
+    launch_diag_max_f64<DIM>(c->L, c->B, c->N, c->S, c->SD, reinterpret_cast<unsigned *>(c->max_bits), c->diag_bits,
+                             c->cgrid, c->grid, c->stream);
     unsigned long long dbits = 0;
     CK(cudaMemcpyAsync(&dbits, c->diag_bits, sizeof(dbits), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));

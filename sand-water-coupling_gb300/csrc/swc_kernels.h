@@ -143,9 +143,11 @@ void launch_segments(const Lattice & L, const BrickArrays & B, const NodeArrays 
 template<int DIM>
 void launch_ahat(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                  int blocks, cudaStream_t st);
+// max of the unclamped diagonal in FP64 (its bits into *out_bits); overwrites N.ahat
 template<int DIM>
-void launch_diag_max_f64(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const StencilD & S,
-                         unsigned long long * out_bits, int grid, cudaStream_t st);
+void launch_diag_max_f64(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
+                         const StencilD & SD, unsigned int * top, unsigned long long * out_bits, int blocks, int grid,
+                         cudaStream_t st);
 // warm-start modes
 enum { kWarmPrefix = 0, kWarmNode = 1, kWarmZero = 2, kWarmGiven = 3, kWarmExtrap = 4 };
 // history (kWarmExtrap): steps of valid pressure history before this one (0, 1 or 2)

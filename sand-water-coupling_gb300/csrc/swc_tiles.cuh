@@ -50,64 +50,6 @@ __device__ __forceinline__ long long compact_index(const Lattice & L, const int 
 // ---------------------------------------------------------------------------
 // Halo tile loading and the radial stencil.
 // ---------------------------------------------------------------------------
-template<int DIM, class Get>
-__device__ __forceinline__ void load_tile(const Lattice & L, const unsigned char * __restrict__ bflag, int3 bc,
-                                          float * tile, Get get) {
-    using G       = BrickGeom<DIM>;
-    constexpr int NT = G::TX * G::TY * G::TZ;
-    for (int t = threadIdx.x; t < NT; t += kNT) {
-        const int tx = t % G::TX, ty = (t / G::TX) % G::TY, tz = t / (G::TX * G::TY);
-        const int x = bc.x * G::BX + tx - G::HALO, y = bc.y * G::BY + ty - G::HALO;
-        const int z = DIM == 3 ? bc.z * G::BZ + tz - G::HALO : 0;
-        float v = 0.f;
-        if (x >= 0 && x < L.nx && y >= 0 && y < L.ny && (DIM == 2 || (z >= 0 && z < L.nz))) {
-            const int nbx = x / G::BX, nby = y / G::BY, nbz = DIM == 3 ? z / G::BZ : 0;
-            const int nbk = nbx + L.bnx * (nby + L.bny * nbz);
-            if (bflag[nbk])
-                v = get((long long) nbk * G::BN + (x - nbx * G::BX) + G::BX * ((y - nby * G::BY) + G::BY * (z - nbz * G::BZ)));
-        }
-        tile[tx + G::PX * (ty + G::TY * tz)] = v;
-    }
-}
-
-template<int DIM> __device__ __forceinline__ int tile_center(int l) {
-    using G      = BrickGeom<DIM>;
-    const int lx = l % G::BX, ly = (l / G::BX) % G::BY, lz = l / (G::BX * G::BY);
-    return (lx + G::HALO) + G::PX * ((ly + G::HALO) + G::TY * (DIM == 3 ? lz + G::HALO : 0));
-}
-
-// sum over offsets 0 < |k|^2 < 16 of c(|k|^2) * tile[center + k]
-template<int DIM> __device__ __forceinline__ float stencil_apply(const float * tile, int c, const Stencil & S) {
-    using G   = BrickGeom<DIM>;
-    float acc = 0.f;
-    constexpr int ZR = DIM == 3 ? 3 : 0;
-#pragma unroll
-    for (int dz = -ZR; dz <= ZR; dz++)
-#pragma unroll
-        for (int dy = -3; dy <= 3; dy++)
-#pragma unroll
-            for (int dx = -3; dx <= 3; dx++) {
-                const int r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 > 0 && r2 < 16) acc = fmaf(S.c[r2], tile[c + dx + G::PX * (dy + G::TY * dz)], acc);
-            }
-    return acc;
-}
-template<int DIM> __device__ __forceinline__ double stencil_apply_d(const float * tile, int c, const StencilD & S) {
-    using G    = BrickGeom<DIM>;
-    double acc = 0.0;
-    constexpr int ZR = DIM == 3 ? 3 : 0;
-#pragma unroll
-    for (int dz = -ZR; dz <= ZR; dz++)
-#pragma unroll
-        for (int dy = -3; dy <= 3; dy++)
-#pragma unroll
-            for (int dx = -3; dx <= 3; dx++) {
-                const int r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 > 0 && r2 < 16) acc += S.c[r2] * double(tile[c + dx + G::PX * (dy + G::TY * dz)]);
-            }
-    return acc;
-}
-
 // Threads of the row-stencil kernels: one thread per x-row of a brick.
 template<int DIM> struct RowGeom {
     static constexpr int NT = BrickGeom<DIM>::BY * BrickGeom<DIM>::BZ;  // 64 (3D) or 16 (2D)
