@@ -170,23 +170,27 @@ __global__ void k_permute(const int * __restrict__ perm, long long n, const floa
 }
 
 // Sum of w (W_h = 2 c0h w) over the neighbours within h of two particles a, b,
-// visited once for both (packed FP32x2 arithmetic).
+// visited once for both (packed FP32x2 arithmetic).  Candidates outside h add an exact
+// zero, so there is no test: some lane of the warp nearly always has a hit.  Bound by
+// instruction issue (69%) and the FP32 pipe (55%), which takes a packed operation in two
+// cycles, about 109 candidates a warp for 67 hits of its pairs: 182 us at 2.1M
+// particles (4,900 warp instructions per 64 particles), 209 with tests, masks and
+// per-point row reaches (6,250).
 template<int DIM>
 __device__ __forceinline__ float2 density_sum2(const Lattice & L, const Phys & P, const int * __restrict__ cellStart,
                                                const float4 * __restrict__ pos, float4 qa, float4 qb) {
-    const float2 qx = make_float2(qa.x, qb.x), qy = make_float2(qa.y, qb.y), qz = make_float2(qa.z, qb.z);
     float2 s = f2(0.f);
     for_each_in_radius2<DIM>(L, cellStart, make_float3(qa.x, qa.y, qa.z), make_float3(qb.x, qb.y, qb.z), P.h, P.h2,
                              [&](int j) {
                                  const float4 p  = pos[j];
-                                 const float2 dx = add2(qx, f2(-p.x)), dy = add2(qy, f2(-p.y));
-                                 float2 r2       = fma2(dy, dy, mul2(dx, dx));
+                                 const float2 dx = make_float2(qa.x - p.x, qb.x - p.x);
+                                 const float2 dy = make_float2(qa.y - p.y, qb.y - p.y);
+                                 float2 r2       = fma2(dy, dy, fma2(dx, dx, f2(1e-30f)));
                                  if (DIM == 3) {
-                                     const float2 dz = add2(qz, f2(-p.z));
+                                     const float2 dz = make_float2(qa.z - p.z, qb.z - p.z);
                                      r2              = fma2(dz, dz, r2);
                                  }
-                                 const bool m0 = r2.x < P.h2, m1 = r2.y < P.h2;
-                                 if (m0 || m1) s = add2(s, spline2(r2, m0, m1, P.inv_h).w);
+                                 s = add2(s, spline_w2(r2, P.inv_h));
                              });
     return s;
 }
@@ -263,31 +267,30 @@ __global__ void k_set_volume(float4 * __restrict__ pos, const float * __restrict
 // Cores/Structures/ParticlesBasedVectorField.cpp:56-69):
 // l += g s (m/rho_j) / m (x_j - x_i) with s = (v_j - v_i).(x_j - x_i) / r^2 and
 // gradientKernel(x_j - x_i) = -W'(r) (x_j - x_i) / r = c1h g (x_j - x_i)
-// (c1h applied by the caller); the particle itself (r = 0) adds nothing.
+// (c1h applied by the caller); the particle itself (r = 0) adds nothing, nor does a
+// candidate beyond h of one of the two (g saturates at 0).  253 us at 2.1M particles,
+// 283 with masks and per-point row reaches; issue 60%, waiting on the candidates' loads.
 template<int DIM>
 __device__ __forceinline__ void viscous_sum2(const Lattice & L, const Phys & P, const int * __restrict__ cellStart,
                                              const float4 * __restrict__ pos, const float4 * __restrict__ vel,
                                              float4 qa, float4 va, float4 qb, float4 vb, float2 & lx, float2 & ly,
                                              float2 & lz) {
-    const float2 qx = make_float2(qa.x, qb.x), qy = make_float2(qa.y, qb.y), qz = make_float2(qa.z, qb.z);
-    const float2 vx = make_float2(va.x, vb.x), vy = make_float2(va.y, vb.y), vz = make_float2(va.z, vb.z);
     for_each_in_radius2<DIM>(
         L, cellStart, make_float3(qa.x, qa.y, qa.z), make_float3(qb.x, qb.y, qb.z), P.h, P.h2, [&](int j) {
             const float4 p = pos[j];
             // x_j - x_i and v_j - v_i
-            const float2 dx = fma2(qx, f2(-1.f), f2(p.x)), dy = fma2(qy, f2(-1.f), f2(p.y));
-            const float2 dz = DIM == 3 ? fma2(qz, f2(-1.f), f2(p.z)) : f2(0.f);
-            float2 r2       = fma2(dy, dy, mul2(dx, dx));
+            const float2 dx = make_float2(p.x - qa.x, p.x - qb.x), dy = make_float2(p.y - qa.y, p.y - qb.y);
+            const float2 dz = DIM == 3 ? make_float2(p.z - qa.z, p.z - qb.z) : f2(0.f);
+            float2 r2       = fma2(dy, dy, fma2(dx, dx, f2(1e-30f)));
             if (DIM == 3) r2 = fma2(dz, dz, r2);
-            const bool m0 = r2.x < P.h2 && r2.x > 0.f, m1 = r2.y < P.h2 && r2.y > 0.f;
-            if (!(m0 || m1)) return;
+            if (!(r2.x < P.h2 || r2.y < P.h2)) return;  // both outside, or not a number
             const float4 vj = vel[j];
-            float2 dot = fma2(fma2(vy, f2(-1.f), f2(vj.y)), dy, mul2(fma2(vx, f2(-1.f), f2(vj.x)), dx));
-            if (DIM == 3) dot = fma2(fma2(vz, f2(-1.f), f2(vj.z)), dz, dot);
-            const Spline2 k = spline2(r2, m0, m1, P.inv_h);
-            const float2 gs = mul2(mul2(k.g, mul2(dot, mul2(k.ri, k.ri))), f2(vj.w * P.inv_mass));
-            lx              = fma2(gs, dx, lx);
-            ly              = fma2(gs, dy, ly);
+            float2 dot = fma2(make_float2(vj.y - va.y, vj.y - vb.y), dy, mul2(make_float2(vj.x - va.x, vj.x - vb.x), dx));
+            if (DIM == 3) dot = fma2(make_float2(vj.z - va.z, vj.z - vb.z), dz, dot);
+            const SplineG2 k = spline_g2(r2, P.inv_h);
+            const float2 gs  = mul2(mul2(k.g, mul2(dot, mul2(k.ri, k.ri))), f2(vj.w * P.inv_mass));
+            lx               = fma2(gs, dx, lx);
+            ly               = fma2(gs, dy, ly);
             if (DIM == 3) lz = fma2(gs, dz, lz);
         });
 }

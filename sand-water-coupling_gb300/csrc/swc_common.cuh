@@ -206,6 +206,28 @@ __device__ __forceinline__ Spline2 spline2(float2 r2, bool m0, bool m1, float in
     return o;
 }
 
+// The same w and g (with ri = 1/r) without masks: a and b saturate, so beyond h both are
+// an exact 0 (saturating also takes a NaN to 0).  r2 >= 1e-30.
+__device__ __forceinline__ float2 spline_w2(float2 r2, float inv_h) {
+    const float2 ri = make_float2(rsqrt_n(r2.x), rsqrt_n(r2.y));
+    const float2 r  = mul2(r2, ri);
+    const float2 a  = make_float2(__saturatef(fmaf(r.x, -inv_h, 1.f)), __saturatef(fmaf(r.y, -inv_h, 1.f)));
+    const float2 b  = make_float2(__saturatef(a.x - 0.5f), __saturatef(a.y - 0.5f));
+    return fma2(mul2(mul2(b, b), b), f2(-4.f), mul2(mul2(a, a), a));
+}
+struct SplineG2 {
+    float2 g, ri;
+};
+__device__ __forceinline__ SplineG2 spline_g2(float2 r2, float inv_h) {
+    SplineG2 o;
+    o.ri           = make_float2(rsqrt_n(r2.x), rsqrt_n(r2.y));
+    const float2 r = mul2(r2, o.ri);
+    const float2 a = make_float2(__saturatef(fmaf(r.x, -inv_h, 1.f)), __saturatef(fmaf(r.y, -inv_h, 1.f)));
+    const float2 b = make_float2(__saturatef(a.x - 0.5f), __saturatef(a.y - 0.5f));
+    o.g            = mul2(fma2(mul2(b, b), f2(-4.f), mul2(a, a)), o.ri);
+    return o;
+}
+
 __device__ __forceinline__ double kW_d(double r, double inv_h, double c0) {
     const double x = r * inv_h;
     if (x < .5) return c0 * (6 * x * x * (x - 1) + 1);
@@ -337,83 +359,58 @@ __device__ __forceinline__ float slab_dist(float q, int c, int n, float o, float
     return q < lo ? lo - q : (q > hi ? q - hi : 0.f);
 }
 
-// Neighbour iteration over cells for a query point and radius R (particle
-// queries): rows pruned by their slab distance, x-range per row from the
-// remaining radius; f(j) for every particle j of the visited cells.
+// Neighbour iteration over cells for two query points a and b at once (neighbours in
+// the sorted order, normally in one cell row) and radius R: the rows and x-ranges
+// within R of the box that holds both, so f(j) sees every particle within R of either
+// (and a few more, on which the caller's sums vanish or its distance tests fail).
+// One distance and one reach per row for both points; border rows, which also hold
+// particles clamped in from outside the lattice, count as distance 0.  The x reach comes
+// from the hardware rsqrt with a relative margin of 1e-5 (its error is below 3e-7).
+// (Distances and reaches of either point in every row cost 70 instructions a row, a
+// quarter of the density pass.)
 template<int DIM, class F>
-__device__ __forceinline__ void for_each_in_radius(const Lattice & L, const int * __restrict__ cellStart,
-                                                   float qx, float qy, float qz, float R, float R2, F && f) {
-    const int cy0 = clampi(__float2int_rd((qy - R - L.oy) * L.inv_dx), 0, L.ny - 1);
-    const int cy1 = clampi(__float2int_rd((qy + R - L.oy) * L.inv_dx), 0, L.ny - 1);
+__device__ __forceinline__ void for_each_in_radius2(const Lattice & L, const int * __restrict__ cellStart, float3 a,
+                                                    float3 b, float R, float R2, F && f) {
+    const float xlo = fminf(a.x, b.x), xhi = fmaxf(a.x, b.x), ylo = fminf(a.y, b.y), yhi = fmaxf(a.y, b.y);
+    const float zlo = fminf(a.z, b.z), zhi = fmaxf(a.z, b.z);
+    const int cy0 = clampi(__float2int_rd((ylo - R - L.oy) * L.inv_dx), 0, L.ny - 1);
+    const int cy1 = clampi(__float2int_rd((yhi + R - L.oy) * L.inv_dx), 0, L.ny - 1);
     int cz0 = 0, cz1 = 0;
     if (DIM == 3) {
-        cz0 = clampi(__float2int_rd((qz - R - L.oz) * L.inv_dx), 0, L.nz - 1);
-        cz1 = clampi(__float2int_rd((qz + R - L.oz) * L.inv_dx), 0, L.nz - 1);
+        cz0 = clampi(__float2int_rd((zlo - R - L.oz) * L.inv_dx), 0, L.nz - 1);
+        cz1 = clampi(__float2int_rd((zhi + R - L.oz) * L.inv_dx), 0, L.nz - 1);
     }
+#pragma unroll 1
     for (int cz = cz0; cz <= cz1; cz++) {
-        const float dz  = DIM == 3 ? slab_dist(qz, cz, L.nz, L.oz, L.dx) : 0.f;
-        const float rz2 = R2 - dz * dz;
-        if (rz2 <= 0.f) continue;
+        float rz2 = R2;
+        if (DIM == 3) {
+            const float lo = fmaf(float(cz), L.dx, L.oz);
+            const float dz = cz == 0 || cz == L.nz - 1 ? 0.f : fmaxf(fmaxf(lo - zhi, zlo - (lo + L.dx)), 0.f);
+            rz2            = fmaf(-dz, dz, R2);
+            if (rz2 <= 0.f) continue;
+        }
+#pragma unroll 1
         for (int cy = cy0; cy <= cy1; cy++) {
-            const float dy  = slab_dist(qy, cy, L.ny, L.oy, L.dx);
-            const float rem = rz2 - dy * dy;
+            const float lo  = fmaf(float(cy), L.dx, L.oy);
+            const float dy  = cy == 0 || cy == L.ny - 1 ? 0.f : fmaxf(fmaxf(lo - yhi, ylo - (lo + L.dx)), 0.f);
+            const float rem = fmaf(-dy, dy, rz2);
             if (rem <= 0.f) continue;
-            const float rx = sqrtf(rem) * 1.000001f + 1e-7f * L.dx;
-            const int cx0  = clampi(__float2int_rd((qx - rx - L.ox) * L.inv_dx), 0, L.nx - 1);
-            const int cx1  = clampi(__float2int_rd((qx + rx - L.ox) * L.inv_dx), 0, L.nx - 1);
-            const long long row = (long long) L.nx * (cy + (long long) L.ny * cz);
-            const int b = cellStart[row + cx0], e = cellStart[row + cx1 + 1];
-            for (int j = b; j < e; j++) f(j);
+            const float rx = fmaf(rem * rsqrt_n(fmaxf(rem, 1e-30f)), 1.00001f, 1e-6f * L.dx);
+            const int cx0  = clampi(__float2int_rd((xlo - rx - L.ox) * L.inv_dx), 0, L.nx - 1);
+            const int cx1  = clampi(__float2int_rd((xhi + rx - L.ox) * L.inv_dx), 0, L.nx - 1);
+            const int * row = cellStart + (cy + L.ny * cz) * L.nx;  // ncells < 2^31
+            const int jb = row[cx0], je = row[cx1 + 1];
+            for (int j = jb; j < je; j++) f(j);
         }
     }
 }
 
-// The same visit for two query points a and b at once (neighbours in the
-// sorted order, normally in one cell row): rows within R of either point and,
-// per row, the union of the two x-ranges, so f(j) sees every particle that
-// either single-point visit would (and a few more, which the caller's exact
-// distance tests reject).  The x reach comes from the hardware rsqrt with a
-// relative margin of 1e-5 (its error is below 3e-7).
+// The same visit for one query point.
 template<int DIM, class F>
-__device__ __forceinline__ void for_each_in_radius2(const Lattice & L, const int * __restrict__ cellStart, float3 a,
-                                                    float3 b, float R, float R2, F && f) {
-    const int cy0 = clampi(__float2int_rd((fminf(a.y, b.y) - R - L.oy) * L.inv_dx), 0, L.ny - 1);
-    const int cy1 = clampi(__float2int_rd((fmaxf(a.y, b.y) + R - L.oy) * L.inv_dx), 0, L.ny - 1);
-    int cz0 = 0, cz1 = 0;
-    if (DIM == 3) {
-        cz0 = clampi(__float2int_rd((fminf(a.z, b.z) - R - L.oz) * L.inv_dx), 0, L.nz - 1);
-        cz1 = clampi(__float2int_rd((fmaxf(a.z, b.z) + R - L.oz) * L.inv_dx), 0, L.nz - 1);
-    }
-    for (int cz = cz0; cz <= cz1; cz++) {
-        float rza = R2, rzb = R2;
-        if (DIM == 3) {
-            const float da = slab_dist(a.z, cz, L.nz, L.oz, L.dx), db = slab_dist(b.z, cz, L.nz, L.oz, L.dx);
-            rza -= da * da;
-            rzb -= db * db;
-        }
-        if (rza <= 0.f && rzb <= 0.f) continue;
-        for (int cy = cy0; cy <= cy1; cy++) {
-            const float ya = slab_dist(a.y, cy, L.ny, L.oy, L.dx), yb = slab_dist(b.y, cy, L.ny, L.oy, L.dx);
-            const float ra = rza - ya * ya, rb = rzb - yb * yb;
-            if (ra <= 0.f && rb <= 0.f) continue;
-            float lo = 3.0e38f, hi = -3.0e38f;
-            if (ra > 0.f) {
-                const float rx = ra * rsqrt_n(fmaxf(ra, 1e-30f)) * 1.00001f + 1e-6f * L.dx;
-                lo = a.x - rx;
-                hi = a.x + rx;
-            }
-            if (rb > 0.f) {
-                const float rx = rb * rsqrt_n(fmaxf(rb, 1e-30f)) * 1.00001f + 1e-6f * L.dx;
-                lo = fminf(lo, b.x - rx);
-                hi = fmaxf(hi, b.x + rx);
-            }
-            const int cx0 = clampi(__float2int_rd((lo - L.ox) * L.inv_dx), 0, L.nx - 1);
-            const int cx1 = clampi(__float2int_rd((hi - L.ox) * L.inv_dx), 0, L.nx - 1);
-            const long long row = (long long) L.nx * (cy + (long long) L.ny * cz);
-            const int jb = cellStart[row + cx0], je = cellStart[row + cx1 + 1];
-            for (int j = jb; j < je; j++) f(j);
-        }
-    }
+__device__ __forceinline__ void for_each_in_radius(const Lattice & L, const int * __restrict__ cellStart,
+                                                   float qx, float qy, float qz, float R, float R2, F && f) {
+    const float3 q = make_float3(qx, qy, qz);
+    for_each_in_radius2<DIM>(L, cellStart, q, q, R, R2, f);
 }
 
 // Row-parallel form of for_each_in_radius for one query point: the caller's
