@@ -495,38 +495,57 @@ __device__ __forceinline__ float grad_scale(float r2, float c1H) {
 }
 
 // Two nodes of a row at x offsets dx (packed FP32x2 arithmetic): returns
-// w = u (a^2 - 4 b^2) / r with a = 1 - r/4, b = max(a - 1/2, 0) and r clamped
-// to 4, i.e. the grad_scale factor above without c1H (r < 2: 1/2 - 3r/16;
-// 2 <= r < 4: 1/r - 1/2 + r/16; 0 beyond), and adds w dx to sx.
-// e = dyz2 + 1e-30 keeps r2 > 0 (a node at the particle adds 0).
-__device__ __forceinline__ float2 grad_w2(float2 dx, float e, float2 u, float2 & sx) {
-    float2 r2       = __ffma2_rn(dx, dx, make_float2(e, e));
-    r2              = make_float2(fminf(r2.x, 16.f), fminf(r2.y, 16.f));
+// w = u (a^2 - 4 b^2) / r with a = 1 - r/4 and b = 1/2 - r/4, both saturated at 0, i.e.
+// the grad_scale factor above without c1H (r < 2: 1/2 - 3r/16; 2 <= r < 4: 1/r - 1/2 +
+// r/16; 0 beyond), and adds w dx to sx.  e = dyz2 + 1e-30 keeps r2 > 0 (a node at the
+// particle adds 0).  INNER: the nodes may lie within r = 2; for others b = 0.
+template<bool INNER> __device__ __forceinline__ float2 grad_w2(float2 dx, float2 e, float2 u, float2 & sx) {
+    const float2 r2 = __ffma2_rn(dx, dx, e);
     const float2 ri = make_float2(rsqrt_n(r2.x), rsqrt_n(r2.y));
     const float2 r  = __fmul2_rn(r2, ri);
-    const float2 a  = __ffma2_rn(r, make_float2(-0.25f, -0.25f), make_float2(1.f, 1.f));
-    float2 b        = __fadd2_rn(a, make_float2(-0.5f, -0.5f));
-    b               = make_float2(fmaxf(b.x, 0.f), fmaxf(b.y, 0.f));
+    const float2 a  = make_float2(__saturatef(fmaf(r.x, -0.25f, 1.f)), __saturatef(fmaf(r.y, -0.25f, 1.f)));
     float2 g        = __fmul2_rn(a, a);
-    g               = __ffma2_rn(__fmul2_rn(b, b), make_float2(-4.f, -4.f), g);
-    const float2 w  = __fmul2_rn(__fmul2_rn(g, ri), u);
-    sx              = __ffma2_rn(w, dx, sx);
+    if (INNER) {
+        const float2 b = make_float2(__saturatef(a.x - 0.5f), __saturatef(a.y - 0.5f));
+        g              = __ffma2_rn(__fmul2_rn(b, b), make_float2(-4.f, -4.f), g);
+    }
+    const float2 w = __fmul2_rn(g, __fmul2_rn(ri, u));
+    sx             = __ffma2_rn(w, dx, sx);
     return w;
 }
 
-// One row of the 8-node x-window (node k at dx = fx - k, fx in [3, 4); dxp
-// holds the pairs (2,3) (4,5) (1,6) (0,7)): sx += sum w dx, returns the pair
-// sums of w.  Nodes 0 and 7 have |dx| >= 3 and lie outside H when dyz2 >= 7;
-// nodes 1 and 6 have |dx| >= 2 and lie outside when dyz2 >= 12.
-__device__ __forceinline__ float2 gradient_row(const float * trow, const float2 (&dxp)[4], float dyz2, float2 & sx) {
-    const float e = dyz2 + 1e-30f;
-    float2 sg     = grad_w2(dxp[0], e, make_float2(trow[2], trow[3]), sx);
-    sg            = __fadd2_rn(sg, grad_w2(dxp[1], e, make_float2(trow[4], trow[5]), sx));
-    if (dyz2 < 12.f) {
-        sg = __fadd2_rn(sg, grad_w2(dxp[2], e, make_float2(trow[1], trow[6]), sx));
-        if (dyz2 < 7.f) sg = __fadd2_rn(sg, grad_w2(dxp[3], e, make_float2(trow[0], trow[7]), sx));
+// One z-plane of the 8-node window: rows oy = 0..7 at dy = fy - oy, nodes k = 0..7 of a
+// row at dx = fx - k, fx and fy in [3, 4); dxp holds the pairs (2,3) (4,5) (1,6) (0,7).
+// A row is at least A = 3 2 1 0 0 1 2 3 away in y, the plane at least B in z, and the
+// pairs of nodes at least 0, 0, 2 and 3 in x, so what no particle can reach, and the
+// inner branch of the spline where no node can need it, are left out at compile time:
+// 204 pairs a particle, 32 with the inner branch, where the tests of every particle
+// itself ran 184 of a warp's particles in five divergent branches a row: 5,600 warp
+// instructions a warp of particles against 4,130, 433 us a launch against 364 at 2.1M
+// particles.  Left: the rsqrt unit 41% and the FP32 pipe 47% busy, the rest the wait for
+// the brick's tile and for the particles that run the wall sum.
+template<int PX, int B>
+__device__ __forceinline__ void gradient_plane(const float * rows, const float2 (&dxp)[4], float fy, float dz,
+                                               float2 & sx, float & gy, float & gz) {
+    const float dz2 = dz * dz;
+    float sum = 0.f;
+#pragma unroll
+    for (int oy = 0; oy < 8; oy++) {
+        const int A = oy < 4 ? 3 - oy : oy - 4, m = A * A + B * B;
+        if (m >= 16) continue;
+        const float dy     = fy - float(oy);
+        const float2 e     = f2(fmaf(dy, dy, dz2) + 1e-30f);
+        const float * trow = rows + PX * oy;
+        const float2 u23 = make_float2(trow[2], trow[3]), u45 = make_float2(trow[4], trow[5]);
+        float2 sg = m < 4 ? grad_w2<true>(dxp[0], e, u23, sx) : grad_w2<false>(dxp[0], e, u23, sx);
+        sg        = __fadd2_rn(sg, m < 4 ? grad_w2<true>(dxp[1], e, u45, sx) : grad_w2<false>(dxp[1], e, u45, sx));
+        if (m + 4 < 16) sg = __fadd2_rn(sg, grad_w2<false>(dxp[2], e, make_float2(trow[1], trow[6]), sx));
+        if (m + 9 < 16) sg = __fadd2_rn(sg, grad_w2<false>(dxp[3], e, make_float2(trow[0], trow[7]), sx));
+        const float s = sg.x + sg.y;
+        gy            = fmaf(dy, s, gy);
+        sum += s;
     }
-    return sg;
+    gz = fmaf(dz, sum, gz);
 }
 
 // Global-memory path for particles outside the staged tile (clamped in from
@@ -665,25 +684,29 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
                 const float2 dxp[4] = {make_float2(fx - 2.f, fx - 3.f), make_float2(fx - 4.f, fx - 5.f),
                                        make_float2(fx - 1.f, fx - 6.f), make_float2(fx, fx - 7.f)};
                 float2 sx = make_float2(0.f, 0.f);
-                float fy = 0.f, fz = 0.f;
-                for (int oz = 0; oz < (DIM == 3 ? 8 : 1); oz++) {
-                    const int kz    = DIM == 3 ? cz - 3 + oz : 0;
-                    const float dz  = DIM == 3 ? uz - float(kz) : 0.f;
-                    const float dz2 = dz * dz;
-#pragma unroll 2
-                    for (int oy = 0; oy < 8; oy++) {
-                        const int ky     = cy - 3 + oy;
-                        const float dy   = uy - float(ky);
-                        const float dyz2 = fmaf(dy, dy, dz2);
-                        if (dyz2 >= 16.f) continue;
-                        const float * trow = tile + PX * (ky + G::TY * kz) + (cx - 3);
-                        const float2 sg = gradient_row(trow, dxp, dyz2, sx);
-                        const float s   = sg.x + sg.y;
-                        fy = fmaf(dy, s, fy);
-                        fz = fmaf(dz, s, fz);
+                float gy = 0.f, gz = 0.f;
+                const float fy    = uy - float(cy - 3);
+                const float * win = tile + PX * (cy - 3) + (cx - 3);
+                if constexpr (DIM == 3) {
+                    // planes 0..3 (at least 3, 2, 1, 0 away), then 7..4
+                    constexpr int PZ = PX * G::TY;
+                    const float fz   = uz - float(cz - 3);
+                    win += PZ * (cz - 3);
+                    float dz = fz, dstep = -1.f;
+                    int step = PZ;
+#pragma unroll 1
+                    for (int h = 0; h < 2; h++) {
+                        gradient_plane<PX, 3>(win, dxp, fy, dz, sx, gy, gz);
+                        gradient_plane<PX, 2>(win + step, dxp, fy, dz + dstep, sx, gy, gz);
+                        gradient_plane<PX, 1>(win + 2 * step, dxp, fy, dz + 2.f * dstep, sx, gy, gz);
+                        gradient_plane<PX, 0>(win + 3 * step, dxp, fy, dz + 3.f * dstep, sx, gy, gz);
+                        win += 7 * PZ;
+                        step  = -PZ;
+                        dz    = fz - 7.f;
+                        dstep = 1.f;
                     }
-                }
-                f = make_float3(P.c1H * (sx.x + sx.y), P.c1H * fy, P.c1H * fz);
+                } else gradient_plane<PX, 0>(win, dxp, fy, 0.f, sx, gy, gz);
+                f = make_float3(P.c1H * (sx.x + sx.y), P.c1H * gy, P.c1H * gz);
             } else {
                 f = gradient_virtual_global<DIM>(L, P, bflag, N, q);
             }
