@@ -63,25 +63,24 @@ struct NodeSums2 {
 // With q = r / h, a = max(1 - q, 0) and b = max(a - 1/2, 0) the cubic spline is
 //   W_h = c0h (2 a^3 - 8 b^3) = 2 c0h w,   w = a^3 - 4 b^3,
 //   -W'_h(r) / r = (6 c0h / h) (a^2 - 4 b^2) / r = c1h g,
-// (q < 1/2: 2 - 3q over h; 1/2 <= q < 1: (1 - q)^2 / r; 0 beyond), and a node
-// only takes particles with r^2 < h^2 (a is zeroed otherwise).  rho_I uses W_H
+// (q < 1/2: 2 - 3q over h; 1/2 <= q < 1: (1 - q)^2 / r; 0 beyond), both saturated
+// at 0, so a particle beyond h adds an exact 0; r2 >= 1e-30.  rho_I uses W_H
 // truncated at h: for H >= 2h (FAST_H) only its inner branch
 // wH = 1 + 6 x^2 (x - 1), x = r / H, is reached; otherwise wH = 2 aH^3 - 8 bH^3.
 // FEAT adds the real-neighbour count (a feature of the learned warm start).
 template<bool REAL, bool FAST_H, bool FEAT>
 __device__ __forceinline__ void pair_add(NodeSums2 & s, const Phys & P, float2 dxx, float dy, float dz, float2 r2,
                                          bool m0, bool m1, float4 p, float4 u) {
-    const float2 ri = make_float2(rsqrt_n(fmaxf(r2.x, 1e-30f)), rsqrt_n(fmaxf(r2.y, 1e-30f)));
-    const float2 q  = mul2(mul2(r2, ri), f2(P.inv_h));
-    float2 a        = max02(fma2(q, f2(-1.f), f2(1.f)));
-    a               = make_float2(m0 ? a.x : 0.f, m1 ? a.y : 0.f);
-    const float2 b  = max02(add2(a, f2(-0.5f)));
+    const float2 ri = make_float2(rsqrt_n(r2.x), rsqrt_n(r2.y));
+    const float2 r  = mul2(r2, ri);
+    const float2 a  = make_float2(__saturatef(fmaf(r.x, -P.inv_h, 1.f)), __saturatef(fmaf(r.y, -P.inv_h, 1.f)));
+    const float2 b  = make_float2(__saturatef(a.x - 0.5f), __saturatef(a.y - 0.5f));
     const float2 a2 = mul2(a, a), b2 = mul2(b, b);
     const float2 w  = fma2(mul2(b2, b), f2(-4.f), mul2(a2, a));
     const float2 g  = mul2(fma2(b2, f2(-4.f), a2), ri);
     if (REAL) {
         float2 wH;
-        const float2 x = mul2(q, f2(P.h * P.inv_H));
+        const float2 x = mul2(r, f2(P.inv_H));
         if (FAST_H) {
             wH = fma2(mul2(mul2(x, x), add2(x, f2(-1.f))), f2(6.f), f2(1.f));
             wH = make_float2(m0 ? wH.x : 0.f, m1 ? wH.y : 0.f);
@@ -123,7 +122,9 @@ __device__ __forceinline__ void pair_add(NodeSums2 & s, const Phys & P, float2 d
 // cell row are loaded once for all of them and tested by exact distance, so
 // every node still sums exactly its neighbours within h, in cell-row order.
 // Five 128-thread blocks per SM (96 registers, no spills): 10% faster than the
-// unconstrained 109-register build at four blocks.
+// unconstrained 109-register build at four blocks; six (80 registers) take 5 times as
+// long.  456 -> 430 us at 2.25M nodes with the spline's terms saturated instead of
+// masked (123.6M warp instructions at 969k nodes, 135M before).
 // ---------------------------------------------------------------------------
 template<int DIM, bool FAST_H, bool FEAT>
 __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const int * __restrict__ blist,
@@ -185,17 +186,17 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
                     // cell rows (cy, cz) in order; the next row's range and the next
                     // candidate's position / velocity are loaded one step ahead
                     int cy = cy0, cz = cz0;
-                    long long row = (long long) L.nx * (cy + (long long) L.ny * cz);
-                    int jb = cs[row + cxa], je = cs[row + cxb + 1];
+                    const int row0 = L.nx * (cy + L.ny * cz);  // ncells < 2^31
+                    int jb = cs[row0 + cxa], je = cs[row0 + cxb + 1];
                     for (;;) {
                         int ny = cy + 1, nz = cz;
                         if (ny > cy1) ny = cy0, nz++;
                         const bool more = nz <= cz1;
                         int nb_ = 0, ne_ = 0;
                         if (more) {
-                            const long long nrow = (long long) L.nx * (ny + (long long) L.ny * nz);
-                            nb_ = cs[nrow + cxa];
-                            ne_ = cs[nrow + cxb + 1];
+                            const int row = L.nx * (ny + L.ny * nz);
+                            nb_ = cs[row + cxa];
+                            ne_ = cs[row + cxb + 1];
                         }
                         float4 pn = make_float4(0.f, 0.f, 0.f, 0.f), un = pn;
                         if (jb < je) pn = X[jb], un = U[jb];
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
                             if (j + 1 < je) pn = X[j + 1], un = U[j + 1];
                             const float2 dyz = add2(add2(yzn, make_float2(-p.y, -p.z)), yzl);
                             const float dy = dyz.x, dz = DIM == 3 ? dyz.y : 0.f;
-                            const float ryz = fmaf(dz, dz, dy * dy);
+                            const float ryz = fmaf(dz, dz, fmaf(dy, dy, 1e-30f));  // > 0 for the rsqrt
                             if (ryz >= P.h2 + P.tie2) continue;
                             const float2 dxx = add2(add2(xn, f2(-p.x)), xl);
                             const float2 r2  = fma2(dxx, dxx, f2(ryz));
