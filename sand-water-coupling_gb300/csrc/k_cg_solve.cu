@@ -34,9 +34,11 @@ __device__ __forceinline__ float comp(const float4 & v, int j) { return j == 0 ?
 
 constexpr int kSums = 4;  // values of a meeting
 
-// Triple floats (three error-free terms, about 70 bits): the sums below the block.
-// GB300 adds or converts two FP64 values per SM and clock, so FP64 in the lanes of every
-// warp would queue for half a microsecond; a block converts its totals alone.
+// Triple floats (three error-free terms, about 70 bits) hold the sums above the lane and
+// the scalars of the iteration.  GB300 adds or converts two FP64 values per SM and
+// clock, with a latency of 65 clocks and far more for a quotient: with FP64 here a meeting
+// took 7,100 clocks in a block alone.  The sums are scaled by the power of two that
+// brings |b|^2 to about 1, so they stay in the range of the FP32 products.
 struct F3 {
     float h, m, l;
 };
@@ -54,13 +56,13 @@ __device__ __forceinline__ F3 f3_shfl(const F3 & a, int o) {
     return F3{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.m, o),
               __shfl_xor_sync(0xffffffffu, a.l, o)};
 }
-// Sums of four float-float values over the warp: lanes 8 k .. 8 k + 7 get value k's.
-__device__ __forceinline__ F3 warp_sum4(const FF (&p)[kSums]) {
+// Sums of four float-float values, scaled, over the warp: lanes 8 k .. 8 k + 7 get value k's.
+__device__ __forceinline__ F3 warp_sum4(const FF (&p)[kSums], float scale) {
     const int lane = threadIdx.x & 31;
     const bool up = lane & 16, odd = lane & 8;
     F3 q[kSums];
 #pragma unroll
-    for (int k = 0; k < kSums; k++) q[k] = F3{p[k].hi, p[k].lo, 0.f};
+    for (int k = 0; k < kSums; k++) q[k] = F3{p[k].hi * scale, p[k].lo * scale, 0.f};
     // the halves of the warp, then its quarters, exchange the values that they give up
     const F3 a = f3_add(up ? q[2] : q[0], f3_shfl(up ? q[0] : q[2], 16));
     const F3 b = f3_add(up ? q[3] : q[1], f3_shfl(up ? q[1] : q[3], 16));
@@ -69,10 +71,31 @@ __device__ __forceinline__ F3 warp_sum4(const FF (&p)[kSums]) {
     for (int o = 4; o > 0; o >>= 1) c = f3_add(c, f3_shfl(c, o));
     return c;
 }
-__device__ __forceinline__ double warp_sum_double(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// a * k (k a float)
+__device__ __forceinline__ F3 f3_scale(const F3 & a, float k) {
+    const float p = __fmul_rn(a.h, k), e = __fmaf_rn(a.h, k, -p), q = __fmul_rn(a.m, k);
+    const float f = __fmaf_rn(a.m, k, -q);
+    float s, t;
+    F3 o;
+    two_sum(e, q, s, t);
+    o.l = __fmaf_rn(a.l, k, __fadd_rn(f, t));
+    fast_two_sum(p, s, o.h, o.m);
+    return o;
+}
+// float(a / b): the FP32 quotient and one correction from the exact remainder (about 44
+// bits before the last rounding)
+__device__ __forceinline__ float f3_quotient(const F3 & a, const F3 & b) {
+    const float q = __fdiv_rn(a.h, b.h);
+    const F3 r    = f3_add(a, f3_scale(b, -q));
+    return __fadd_rn(q, __fdiv_rn(__fadd_rn(r.h, r.m), b.h));
+}
+__device__ __forceinline__ double f3_double(const F3 & a) { return (double(a.h) + double(a.m)) + double(a.l); }
+__device__ __forceinline__ F3 f3_of(double v) {
+    F3 o;
+    o.h = float(v);
+    o.m = float(v - double(o.h));
+    o.l = float((v - double(o.h)) - double(o.m));
+    return o;
 }
 
 // A meeting's words are 16 bytes, value and tag written and read as one.
@@ -88,14 +111,15 @@ __device__ __forceinline__ ulonglong2 word_get(const ulonglong2 * p) {
                  : "memory");
     return v;
 }
-// A block's partial sum.
-__device__ __forceinline__ void slot_put(ulonglong2 * p, double v, unsigned tag) {
-    word_put(p, (unsigned long long) __double_as_longlong(v), tag);
+// A block's partial sum and its tag.
+__device__ __forceinline__ void slot_put(ulonglong2 * p, const F3 & v, unsigned tag) {
+    word_put(p, (unsigned long long) __float_as_uint(v.m) << 32 | __float_as_uint(v.h),
+             (unsigned long long) tag << 32 | __float_as_uint(v.l));
 }
-__device__ __forceinline__ bool slot_get(const ulonglong2 * p, unsigned tag, double & v) {
+__device__ __forceinline__ bool slot_get(const ulonglong2 * p, unsigned tag, F3 & v) {
     const ulonglong2 w = word_get(p);
-    v                  = __longlong_as_double((long long) w.x);
-    return unsigned(w.y) == tag;
+    v = F3{__uint_as_float(unsigned(w.x)), __uint_as_float(unsigned(w.x >> 32)), __uint_as_float(unsigned(w.y))};
+    return unsigned(w.y >> 32) == tag;
 }
 // What block 0 made of the sums: the step's factors and how to go on.
 enum : unsigned { kGoOn = 0, kFailed = 5, kMeasure = 6 };  // 1, 2, 3: CgState::done
@@ -132,14 +156,15 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Polls of one slot before a block gives up (about a second).
 constexpr int kMeetPolls = 1 << 20;
 
-// Block 0's view of the solve.
+// Block 0's view of the solve (scaled; the threshold as two floats).
 struct CgScalars {
-    double pq, rr, rr_next, threshold;
-    int    it, max_iter;
+    F3    pq, rr, rr_next;
+    float threshold_h, threshold_l;
+    int   it, max_iter;
 };
 template<int WARPS> struct MeetSmem {
     F3        part[WARPS][kSums];
-    double    sum[kSums];
+    F3        sum[kSums];
     int       full[kSums];
     Outcome   out;
     CgScalars cg;  // block 0
@@ -148,55 +173,55 @@ constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer bloc
 
 // The factors and the stopping test from the sums d.q, r.q, q.q, r.r (after kMeasure:
 // from |r - alpha q|^2).
-__device__ __forceinline__ Outcome decide(CgScalars & c, const double (&sum)[kSums], float alpha, bool measured) {
+__device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums], float alpha, bool measured) {
     Outcome o{alpha, 0.f, kGoOn};
     if (!measured) {
         c.pq      = sum[0];
         c.rr      = sum[3];
         c.rr_next = c.rr;
-        if (!(c.pq != 0.0) || c.pq != c.pq) {
+        if (!(c.pq.h != 0.f) || c.pq.h != c.pq.h) {
             o.code = 3;
             return o;
         }
-        o.alpha   = float(c.rr / c.pq);
-        c.rr_next = c.rr + double(o.alpha) * (double(o.alpha) * sum[2] - 2.0 * sum[1]);
-        if (c.rr_next < 1e-6 * c.rr) {
+        o.alpha   = f3_quotient(c.rr, c.pq);
+        const F3 t = f3_add(f3_scale(sum[2], o.alpha), f3_scale(sum[1], -2.f));
+        c.rr_next  = f3_add(c.rr, f3_scale(t, o.alpha));
+        if (c.rr_next.h < 1e-6f * c.rr.h) {
             o.code = kMeasure;  // nearly all of r goes: its norm from r - alpha q itself
             return o;
         }
     } else c.rr_next = sum[0];
     c.it++;
-    if (c.rr_next != c.rr_next) o.code = 3;
-    else if (c.rr_next < c.threshold) o.code = 1;
+    const F3 & n = c.rr_next;
+    if (n.h != n.h) o.code = 3;
+    else if (n.h < c.threshold_h || (n.h == c.threshold_h && n.m < c.threshold_l)) o.code = 1;
     else if (c.it >= c.max_iter) o.code = 2;
-    o.beta = float(c.rr_next / c.rr);
+    o.beta = f3_quotient(n, c.rr);
     return o;
 }
 
 // Meeting of the blocks in use: v (value lane / 8 of the warp, as warp_sum4 gives it)
-// summed over their warps, and what block 0 decides on the sums, the same on every
-// thread.  Every block publishes its four partials under the meeting's tag; block 0
-// reads them all and publishes the outcome, one word that the others poll.  (With
-// every block polling every slot the polls themselves, 64 B x blocks^2 a round, kept
-// the slots from being written: 13 us a meeting of 152 blocks; with the sums published
-// and the FP64 quotients formed by every thread, 5 us.)  One set of slots serves: a
-// block publishes again only after it has the outcome, and block 0 only after every
-// block has published again.
+// summed over their first `active` warps, and what block 0 decides on the sums, the
+// same on every thread.  Every block publishes its four partials under the meeting's
+// tag; block 0 reads them all and publishes the outcome, one word that the others poll.  (With every block polling every slot the polls themselves, 64 B x
+// blocks^2 a round, kept the slots from being written: 13 us a meeting of 152 blocks;
+// with the sums published and FP64 quotients formed by every thread, 5 us.)  One set of
+// slots serves: a block publishes again only after it has the outcome, and block 0
+// only after every block has published again.
 template<int WARPS>
-__device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int stride, int blocks, unsigned & tag,
-                                        MeetSmem<WARPS> & M, float alpha, bool measured) {
+__device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int stride, int blocks, int active,
+                                        unsigned & tag, MeetSmem<WARPS> & M, float alpha, bool measured) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ulonglong2 * outcome = slots + (long long) stride * kSums;
     if ((lane & 7) == 0) M.part[warp][lane >> 3] = v;
     __syncthreads();
     if (warp == 0) {
         const int k = lane >> 3, w = lane & 7;
-        F3 part = M.part[w][k];
-        for (int j = w + 8; j < WARPS; j += 8) part = f3_add(part, M.part[j][k]);
+        F3 part{0.f, 0.f, 0.f};
+        for (int j = w; j < active; j += 8) part = f3_add(part, M.part[j][k]);
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) part = f3_add(part, f3_shfl(part, o));
-        if (w == 0)
-            slot_put(slots + (long long) blockIdx.x * kSums + k, (double(part.h) + double(part.m)) + double(part.l), tag);
+        if (w == 0) slot_put(slots + (long long) blockIdx.x * kSums + k, part, tag);
         if (blockIdx.x != 0 && lane == 0) {
             const ulonglong2 * p = outcome + blockIdx.x % kCopies;
             Outcome o;
@@ -207,25 +232,29 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
         }
     }
     if (blockIdx.x == 0) {
+        // a warp per value, five slots a lane at once
         if (warp < kSums) {
-            double s  = 0;
+            F3 s{0.f, 0.f, 0.f};
             bool full = true;
-            for (int j0 = lane; j0 < blocks; j0 += 32 * 5) {  // 5 x 32 = 160 slots at once
-                double e[5];
-                bool there[5];
-                for (int n = 0; n < kMeetPolls; n++) {
+            for (int j0 = lane; j0 < blocks; j0 += 32 * 5) {
+                F3 e[5];
+                bool there = false;
+                for (int n = 0; n < kMeetPolls && !there; n++) {
+                    there = true;
 #pragma unroll
-                    for (int k = 0; k < 5; k++) {
-                        const int j = j0 + 32 * k;
-                        e[k]        = 0.0;
-                        there[k]    = j >= blocks || slot_get(slots + (long long) j * kSums + warp, tag, e[k]);
+                    for (int q = 0; q < 5; q++) {
+                        const int j = j0 + 32 * q;
+                        e[q]        = F3{0.f, 0.f, 0.f};
+                        if (j < blocks) there = slot_get(slots + (long long) j * kSums + warp, tag, e[q]) && there;
                     }
-                    if (there[0] && there[1] && there[2] && there[3] && there[4]) break;
                 }
-                full = full && there[0] && there[1] && there[2] && there[3] && there[4];
-                s += ((e[0] + e[1]) + (e[2] + e[3])) + e[4];
+                full = full && there;
+                if (blocks > 32) e[0] = f3_add(f3_add(f3_add(e[0], e[1]), f3_add(e[2], e[3])), e[4]);
+                s = f3_add(s, e[0]);
             }
-            s    = warp_sum_double(s);
+            __syncwarp();
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) s = f3_add(s, f3_shfl(s, d));
             full = __all_sync(0xffffffffu, full);
             if (lane == 0) {
                 M.sum[warp]  = s;
@@ -233,12 +262,14 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
             }
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const double sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
-            Outcome o               = decide(M.cg, sum, alpha, measured);
+        if (warp == 0) {
+            const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
+            CgScalars c         = M.cg;
+            Outcome o           = decide(c, sum, alpha, measured);
             if (!(M.full[0] && M.full[1] && M.full[2] && M.full[3])) o.code = kFailed;
-            for (int k = 0; k < kCopies; k++) outcome_put(outcome + k, o, tag);
-            M.out = o;
+            if (lane < kCopies) outcome_put(outcome + lane, o, tag);
+            __syncwarp();
+            if (lane == 0) M.cg = c, M.out = o;
         }
     }
     __syncthreads();
@@ -277,8 +308,14 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     fill_segments<DIM>(seg);
     for (int k = 0, bi = bfirst; k < B::TABS && bi < nb; k++, bi += bstep)
         fill_neighbours<DIM>(L, bflag, blist[bi], gl, tab + 27 * k);
-    if (threadIdx.x == 0) M.cg = CgScalars{0.0, cg->rr, cg->rr, cg->threshold, 0, cg->max_iter};
+    // the sums' power of two
+    const float scale = exp2f(float(-max(-120, min(120, ilogb(cg->bb)))));
+    if (threadIdx.x == 0) {
+        const F3 rr = f3_of(cg->rr * double(scale)), t = f3_of(cg->threshold * double(scale));
+        M.cg        = CgScalars{F3{0.f, 0.f, 0.f}, rr, rr, t.h, t.m, 0, cg->max_iter};
+    }
     __syncthreads();
+    const int active = W * min(Gr::COUNT, (nb - int(blockIdx.x) + P - 1) / P);  // warps with bricks
 
     Outcome o{0.f, 0.f, kGoOn};
     bool first   = true, ok = true;
@@ -371,7 +408,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
             }
         }
         lap(spent.product);
-        o     = meet<B::WARPS>(warp_sum4(part), slots, gridDim.x, P, tag, M, 0.f, false);
+        o     = meet<B::WARPS>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, 0.f, false);
         first = false;
         if (o.code == kMeasure) {
 #pragma unroll
@@ -385,7 +422,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                     for (int j = 0; j < 4; j++) ff_add_prod(part[0], comp(r, j), comp(r, j));
                 }
             }
-            o = meet<B::WARPS>(warp_sum4(part), slots, gridDim.x, P, tag, M, o.alpha, true);
+            o = meet<B::WARPS>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, o.alpha, true);
         }
         lap(spent.meeting);
         if (o.code != kGoOn) break;
@@ -403,9 +440,9 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
         }
     if (threadIdx.x == 0) {
         if (blockIdx.x == 0) {
-            cg->rr      = M.cg.rr_next;
-            cg->rr_prev = M.cg.rr;
-            cg->pq      = M.cg.pq;
+            cg->rr      = f3_double(M.cg.rr_next) / double(scale);
+            cg->rr_prev = f3_double(M.cg.rr) / double(scale);
+            cg->pq      = f3_double(M.cg.pq) / double(scale);
             cg->iter    = M.cg.it;
             cg->tick    = tag;
             if (phases) *phases = spent;

@@ -1313,10 +1313,6 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
     if (which == 7 && !c->mlp_ready) return SWC_BAD_ARG;  // needs a network (swc_set_mlp)
     CK(cudaStreamSynchronize(c->stream));
     const bool solve = which == 0 || which == 1 || which == 6;
-    if (solve && c->dim != 3) {
-        *mean_ms = 0;  // as for every kernel that is timed in 3D only
-        return SWC_OK;
-    }
     // keep the solver state: the CG scalars, and the vectors the timed kernel writes
     CgState saved{};
     CK(cudaMemcpy(&saved, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost));
@@ -1370,9 +1366,13 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
         CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
         for (int k = 0; k < 2; k++) {  // warm, then timed
-            launch_cg_init<3>(c->L, c->B, c->N, c->S, c->cg, c->partials, 0.0, reps, c->B.seg_off + c->B.nseg, c->cgrid, c->grid, c->stream);
-            launch_cg_solve<3>(c->L, c->B, c->N, c->S, c->cg, c->slots, c->uflags, c->cgrid, c->phases,
-                               c->stream);
+            auto go = [&](auto init, auto run) {
+                init(c->L, c->B, c->N, c->S, c->cg, c->partials, 0.0, reps, c->B.seg_off + c->B.nseg, c->cgrid, c->grid,
+                     c->stream);
+                run(c->L, c->B, c->N, c->S, c->cg, c->slots, c->uflags, c->cgrid, c->phases, c->stream);
+            };
+            if (c->dim == 3) go(launch_cg_init<3>, launch_cg_solve<3>);
+            else go(launch_cg_init<2>, launch_cg_solve<2>);
             CK(cudaStreamSynchronize(c->stream));
         }
         CgPhases ph{};
