@@ -176,11 +176,11 @@ __global__ void k_permute(const int * __restrict__ perm, long long n, const floa
 // cycles, about 109 candidates a warp for 67 hits of its pairs: 182 us at 2.1M
 // particles (4,900 warp instructions per 64 particles), 209 with tests, masks and
 // per-point row reaches (6,250).
-template<int DIM>
+template<int DIM, int S>
 __device__ __forceinline__ float2 density_sum2(const Lattice & L, const Phys & P, const int * __restrict__ cellStart,
-                                               const float4 * __restrict__ pos, float4 qa, float4 qb) {
+                                               const float4 * __restrict__ pos, float4 qa, float4 qb, int part) {
     float2 s = f2(0.f);
-    for_each_in_radius2<DIM>(L, cellStart, make_float3(qa.x, qa.y, qa.z), make_float3(qb.x, qb.y, qb.z), P.h, P.h2,
+    for_each_in_radius2<DIM, S>(L, cellStart, make_float3(qa.x, qa.y, qa.z), make_float3(qb.x, qb.y, qb.z), P.h, P.h2,
                              [&](int j) {
                                  const float4 p  = pos[j];
                                  const float2 dx = make_float2(qa.x - p.x, qb.x - p.x);
@@ -191,31 +191,49 @@ __device__ __forceinline__ float2 density_sum2(const Lattice & L, const Phys & P
                                      r2              = fma2(dz, dz, r2);
                                  }
                                  s = add2(s, spline_w2(r2, P.inv_h));
-                             });
+                             }, part);
     return s;
+}
+
+// Sum over the S lanes of a group (fixed tree; every lane gets it).
+template<int S> __device__ __forceinline__ float2 group_sum(float2 v) {
+#pragma unroll
+    for (int o = S / 2; o > 0; o >>= 1)
+        v = add2(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+    return v;
 }
 
 // rho_i = m sum_j W_h(x_i - x_j)  (SmoothedParticles::computeDensities,
 // Cores/Structures/SmoothedParticles.cpp:25-31); writes vel.w = m / rho_i and rho_i.
-// One thread per pair of consecutive sorted particles.  A pair that is not in
-// one cell row is appended to left (left[0] = count, ids from left[2]) and
-// visited particle by particle by k_density_left, so no warp runs both paths.
-template<int DIM>
+// One group of S lanes per pair of consecutive sorted particles, the cell rows of the
+// pair's window spread over the lanes (S = 1 where the pairs alone fill the SMs, see
+// pair_lanes).  A pair that is not in one cell row is appended to left (left[0] =
+// count, ids from left[2]) and visited particle by particle by k_density_left, so no
+// warp runs both paths.
+template<int DIM, int S>
 __global__ void __launch_bounds__(256) k_density(const float4 * __restrict__ pos, float4 * __restrict__ vel,
                                                  float * __restrict__ rho_out, long long n, Lattice L, Phys P,
                                                  const int * __restrict__ cellStart, float mass, int * __restrict__ left) {
     pdl_wait_and_release();
     const long long npair = (n + 1) / 2;
     const float c         = 2.f * P.c0h * mass;
-    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < npair;
-         t += (long long) gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, part = lane % S;
+    for (long long t0 = (blockIdx.x * (long long) blockDim.x + (threadIdx.x - lane)) / S; t0 < npair;
+         t0 += (long long) gridDim.x * blockDim.x / S) {
+        const long long t  = t0 + lane / S;
         const long long ia = 2 * t, ib = ia + 1 < n ? ia + 1 : ia;
-        const float4 qa = pos[ia], qb = pos[ib];
-        if (!near_pair<DIM>(L, qa, qb)) {
-            left[2 + atomicAdd(left, 1)] = int(t);
-            continue;
+        bool on  = t < npair;
+        float2 s = f2(0.f);
+        if (on) {
+            const float4 qa = pos[ia], qb = pos[ib];
+            if (near_pair<DIM>(L, qa, qb)) s = density_sum2<DIM, S>(L, P, cellStart, pos, qa, qb, part);
+            else {
+                if (part == 0) left[2 + atomicAdd(left, 1)] = int(t);
+                on = false;
+            }
         }
-        const float2 s  = density_sum2<DIM>(L, P, cellStart, pos, qa, qb);
+        s = group_sum<S>(s);
+        if (!on || part != 0) continue;
         const float ra = c * s.x, rb = c * s.y;
         if (rho_out) rho_out[ia] = ra;
         vel[ia].w = mass / ra;
@@ -270,12 +288,12 @@ __global__ void k_set_volume(float4 * __restrict__ pos, const float * __restrict
 // (c1h applied by the caller); the particle itself (r = 0) adds nothing, nor does a
 // candidate beyond h of one of the two (g saturates at 0).  253 us at 2.1M particles,
 // 283 with masks and per-point row reaches; issue 60%, waiting on the candidates' loads.
-template<int DIM>
+template<int DIM, int S>
 __device__ __forceinline__ void viscous_sum2(const Lattice & L, const Phys & P, const int * __restrict__ cellStart,
                                              const float4 * __restrict__ pos, const float4 * __restrict__ vel,
-                                             float4 qa, float4 va, float4 qb, float4 vb, float2 & lx, float2 & ly,
-                                             float2 & lz) {
-    for_each_in_radius2<DIM>(
+                                             float4 qa, float4 va, float4 qb, float4 vb, int part, float2 & lx,
+                                             float2 & ly, float2 & lz) {
+    for_each_in_radius2<DIM, S>(
         L, cellStart, make_float3(qa.x, qa.y, qa.z), make_float3(qb.x, qb.y, qb.z), P.h, P.h2, [&](int j) {
             const float4 p = pos[j];
             // x_j - x_i and v_j - v_i
@@ -292,7 +310,7 @@ __device__ __forceinline__ void viscous_sum2(const Lattice & L, const Phys & P, 
             lx               = fma2(gs, dx, lx);
             ly               = fma2(gs, dy, ly);
             if (DIM == 3) lz = fma2(gs, dz, lz);
-        });
+        }, part);
 }
 
 // Gravity (applyExternalForces, SmthParticleHydrodLiquid.cpp:84-88) followed by
@@ -311,7 +329,7 @@ __device__ __forceinline__ float4 forces_out(float4 v, float gx, float gy, float
     return v;
 }
 
-template<int DIM>
+template<int DIM, int S>
 __global__ void __launch_bounds__(256) k_forces(const float4 * __restrict__ pos, const float4 * __restrict__ vel,
                                                 float4 * __restrict__ vel_out, long long n, Lattice L, Phys P,
                                                 const int * __restrict__ cellStart, float dt, int * __restrict__ left) {
@@ -320,18 +338,28 @@ __global__ void __launch_bounds__(256) k_forces(const float4 * __restrict__ pos,
     const float gx = P.gravity_on ? P.gx * dt : 0.f, gy = P.gravity_on ? P.gy * dt : 0.f;
     const float gz = P.gravity_on && DIM == 3 ? P.gz * dt : 0.f;
     const long long npair = (n + 1) / 2;
-    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < npair;
-         t += (long long) gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, part = lane % S;
+    for (long long t0 = (blockIdx.x * (long long) blockDim.x + (threadIdx.x - lane)) / S; t0 < npair;
+         t0 += (long long) gridDim.x * blockDim.x / S) {
+        const long long t  = t0 + lane / S;
         const long long ia = 2 * t, ib = ia + 1 < n ? ia + 1 : ia;
-        const float4 qa = pos[ia], qb = pos[ib], va = vel[ia], vb = vel[ib];
+        bool on   = t < npair;
         float2 lx = f2(0.f), ly = f2(0.f), lz = f2(0.f);
-        if (P.viscosity != 0.f) {
-            if (!near_pair<DIM>(L, qa, qb)) {
-                left[2 + atomicAdd(left, 1)] = int(t);
-                continue;
+        float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
+        if (on) {
+            const float4 qa = pos[ia], qb = pos[ib];
+            va = vel[ia], vb = vel[ib];
+            if (P.viscosity != 0.f) {
+                if (near_pair<DIM>(L, qa, qb))
+                    viscous_sum2<DIM, S>(L, P, cellStart, pos, vel, qa, va, qb, vb, part, lx, ly, lz);
+                else {
+                    if (part == 0) left[2 + atomicAdd(left, 1)] = int(t);
+                    on = false;
+                }
             }
-            viscous_sum2<DIM>(L, P, cellStart, pos, vel, qa, va, qb, vb, lx, ly, lz);
         }
+        lx = group_sum<S>(lx), ly = group_sum<S>(ly), lz = group_sum<S>(lz);
+        if (!on || part != 0) continue;
         vel_out[ia] = forces_out(va, gx, gy, gz, visc, lx.x, ly.x, lz.x, DIM == 3);
         if (ib != ia) vel_out[ib] = forces_out(vb, gx, gy, gz, visc, lx.y, ly.y, lz.y, DIM == 3);
     }
@@ -772,12 +800,27 @@ void launch_bin(const Lattice & L, long long n, float4 *& pos, float4 *& vel, fl
     std::swap(id, S.id2);
 }
 
+// Lanes per particle pair of the density and viscosity passes: as many as keep the
+// threads within 2^17 (about 27 warps per SM, where the passes stop gaining from
+// more), at most one per row of the window's five in 2D.  Measured, density / viscosity
+// with 1, 2, 4, 8 lanes: 32 22 15 12 / 41 28 20 15 us at 15,625 particles, 34 33 30 33 /
+// 42 40 46 52 at 167k, 57 60 63 81 / 68 77 97 130 at 524k.
+template<int DIM> static inline int pair_lanes(long long n) {
+    int S = DIM == 3 ? 8 : 4;
+    while (S > 1 && (n + 1) / 2 * S > (1 << 17)) S /= 2;
+    return S;
+}
+
 template<int DIM>
 void launch_density(const float4 * pos, float4 * vel, float * rho, long long n, const Lattice & L, const Phys & P,
                     const int * cellStart, int * left, cudaStream_t st) {
     if (n <= 0) return;
-    launch_pdl(k_density<DIM>, grid_for((n + 1) / 2, 256, 1 << 20), 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass,
-                                                                         left);
+    const int S   = pair_lanes<DIM>(n);
+    const auto go = [&](auto kernel) {
+        launch_pdl(kernel, grid_for((n + 1) / 2 * S, 256, 1 << 20), 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass,
+                   left);
+    };
+    DIM == 3 && S == 8 ? go(k_density<DIM, 8>) : S == 4 ? go(k_density<DIM, 4>) : S == 2 ? go(k_density<DIM, 2>) : go(k_density<DIM, 1>);
     launch_pdl(k_density_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass, left);
 }
 void launch_set_volume(float4 * pos, const float * rho, long long n, float mass, cudaStream_t st) {
@@ -787,8 +830,12 @@ template<int DIM>
 void launch_forces(const float4 * pos, const float4 * vel, float4 * vel_out, long long n, const Lattice & L,
                    const Phys & P, const int * cellStart, float dt, int * left, cudaStream_t st) {
     if (n <= 0) return;
-    launch_pdl(k_forces<DIM>, grid_for((n + 1) / 2, 256, 1 << 20), 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt,
-                                                                       left);
+    const int S   = pair_lanes<DIM>(n);
+    const auto go = [&](auto kernel) {
+        launch_pdl(kernel, grid_for((n + 1) / 2 * S, 256, 1 << 20), 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt,
+                   left);
+    };
+    DIM == 3 && S == 8 ? go(k_forces<DIM, 8>) : S == 4 ? go(k_forces<DIM, 4>) : S == 2 ? go(k_forces<DIM, 2>) : go(k_forces<DIM, 1>);
     launch_pdl(k_forces_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt, left);
 }
 template<int DIM>

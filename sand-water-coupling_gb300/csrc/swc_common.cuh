@@ -367,10 +367,11 @@ __device__ __forceinline__ float slab_dist(float q, int c, int n, float o, float
 // particles clamped in from outside the lattice, count as distance 0.  The x reach comes
 // from the hardware rsqrt with a relative margin of 1e-5 (its error is below 3e-7).
 // (Distances and reaches of either point in every row cost 70 instructions a row, a
-// quarter of the density pass.)
-template<int DIM, class F>
+// quarter of the density pass.)  With S > 1 the rows are shared by S lanes, lane
+// `part` taking rows part, part + S, ... of the window.
+template<int DIM, int S = 1, class F>
 __device__ __forceinline__ void for_each_in_radius2(const Lattice & L, const int * __restrict__ cellStart, float3 a,
-                                                    float3 b, float R, float R2, F && f) {
+                                                    float3 b, float R, float R2, F && f, int part = 0) {
     const float xlo = fminf(a.x, b.x), xhi = fmaxf(a.x, b.x), ylo = fminf(a.y, b.y), yhi = fmaxf(a.y, b.y);
     const float zlo = fminf(a.z, b.z), zhi = fmaxf(a.z, b.z);
     const int cy0 = clampi(__float2int_rd((ylo - R - L.oy) * L.inv_dx), 0, L.ny - 1);
@@ -380,27 +381,39 @@ __device__ __forceinline__ void for_each_in_radius2(const Lattice & L, const int
         cz0 = clampi(__float2int_rd((zlo - R - L.oz) * L.inv_dx), 0, L.nz - 1);
         cz1 = clampi(__float2int_rd((zhi + R - L.oz) * L.inv_dx), 0, L.nz - 1);
     }
+    auto z_reach = [&](int cz) {
+        const float lo = fmaf(float(cz), L.dx, L.oz);
+        const float dz = cz == 0 || cz == L.nz - 1 ? 0.f : fmaxf(fmaxf(lo - zhi, zlo - (lo + L.dx)), 0.f);
+        return DIM == 3 ? fmaf(-dz, dz, R2) : R2;
+    };
+    auto row = [&](int cy, int cz, float rz2) {
+        const float lo  = fmaf(float(cy), L.dx, L.oy);
+        const float dy  = cy == 0 || cy == L.ny - 1 ? 0.f : fmaxf(fmaxf(lo - yhi, ylo - (lo + L.dx)), 0.f);
+        const float rem = fmaf(-dy, dy, rz2);
+        if (rem <= 0.f) return;
+        const float rx = fmaf(rem * rsqrt_n(fmaxf(rem, 1e-30f)), 1.00001f, 1e-6f * L.dx);
+        const int cx0  = clampi(__float2int_rd((xlo - rx - L.ox) * L.inv_dx), 0, L.nx - 1);
+        const int cx1  = clampi(__float2int_rd((xhi + rx - L.ox) * L.inv_dx), 0, L.nx - 1);
+        const int * cells = cellStart + (cy + L.ny * cz) * L.nx;  // ncells < 2^31
+        const int jb = cells[cx0], je = cells[cx1 + 1];
+        for (int j = jb; j < je; j++) f(j);
+    };
+    if constexpr (S == 1) {
 #pragma unroll 1
-    for (int cz = cz0; cz <= cz1; cz++) {
-        float rz2 = R2;
-        if (DIM == 3) {
-            const float lo = fmaf(float(cz), L.dx, L.oz);
-            const float dz = cz == 0 || cz == L.nz - 1 ? 0.f : fmaxf(fmaxf(lo - zhi, zlo - (lo + L.dx)), 0.f);
-            rz2            = fmaf(-dz, dz, R2);
+        for (int cz = cz0; cz <= cz1; cz++) {
+            const float rz2 = z_reach(cz);
             if (rz2 <= 0.f) continue;
-        }
 #pragma unroll 1
-        for (int cy = cy0; cy <= cy1; cy++) {
-            const float lo  = fmaf(float(cy), L.dx, L.oy);
-            const float dy  = cy == 0 || cy == L.ny - 1 ? 0.f : fmaxf(fmaxf(lo - yhi, ylo - (lo + L.dx)), 0.f);
-            const float rem = fmaf(-dy, dy, rz2);
-            if (rem <= 0.f) continue;
-            const float rx = fmaf(rem * rsqrt_n(fmaxf(rem, 1e-30f)), 1.00001f, 1e-6f * L.dx);
-            const int cx0  = clampi(__float2int_rd((xlo - rx - L.ox) * L.inv_dx), 0, L.nx - 1);
-            const int cx1  = clampi(__float2int_rd((xhi + rx - L.ox) * L.inv_dx), 0, L.nx - 1);
-            const int * row = cellStart + (cy + L.ny * cz) * L.nx;  // ncells < 2^31
-            const int jb = row[cx0], je = row[cx1 + 1];
-            for (int j = jb; j < je; j++) f(j);
+            for (int cy = cy0; cy <= cy1; cy++) row(cy, cz, rz2);
+        }
+    } else {
+        int cy = cy0 + part, cz = cz0;
+#pragma unroll 1
+        for (;;) {
+            while (cy > cy1) cy -= cy1 - cy0 + 1, cz++;
+            if (cz > cz1) break;
+            row(cy, cz, z_reach(cz));
+            cy += S;
         }
     }
 }
