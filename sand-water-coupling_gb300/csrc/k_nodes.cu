@@ -4,6 +4,8 @@
 // alpha_hat, warm starts and the matrix-free CG (stencil SpMV fused with the
 // search-direction update, and the x/r update), all with deterministic
 // FP64 reductions.
+#include <type_traits>
+
 #include "swc_kernels.h"
 #include "swc_tiles.cuh"
 
@@ -120,13 +122,25 @@ __device__ __forceinline__ void pair_add(NodeSums2 & s, const Phys & P, float2 d
 // (boundary: m_b, rho_b, V_b) except weight, rho_I and V_I (real only).
 // Each thread handles NX consecutive nodes along x: the candidate particles of a
 // cell row are loaded once for all of them and tested by exact distance, so
-// every node still sums exactly its neighbours within h, in cell-row order.
+// every node still sums exactly its neighbours within h, in cell-row order.  With
+// S > 1 the cell rows are shared by S lanes and their sums added in a fixed tree.  A
+// queue item is what 128 threads take at once: half a brick (3D, S = 1; with whole
+// bricks two thirds of the blocks ran one brick and the rest none at 196k nodes, 87 us
+// against 65).
 // Five 128-thread blocks per SM (96 registers, no spills): 10% faster than the
 // unconstrained 109-register build at four blocks; six (80 registers) take 5 times as
 // long.  456 -> 430 us at 2.25M nodes with the spline's terms saturated instead of
 // masked (123.6M warp instructions at 969k nodes, 135M before).
 // ---------------------------------------------------------------------------
-template<int DIM, bool FAST_H, bool FEAT>
+// Sum over the S lanes of a group (fixed tree; every lane gets it).
+template<int S> __device__ __forceinline__ float2 lanes_sum(float2 v) {
+#pragma unroll
+    for (int o = S / 2; o > 0; o >>= 1)
+        v = add2(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+    return v;
+}
+
+template<int DIM, bool FAST_H, bool FEAT, int S>
 __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const int * __restrict__ blist,
                                                     const int * __restrict__ bcount, NodeArrays N,
                                                     const float4 * __restrict__ pos, const float4 * __restrict__ vel,
@@ -141,13 +155,18 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
     constexpr int NX = 2;
     constexpr int XS = G::BX / NX;  // thread columns per brick row
     constexpr int TPB = G::BN / NX;
+    constexpr int PAIRS = 128 / S;      // node pairs of a queue item, one per group of S lanes
+    constexpr int ITEMS = TPB / PAIRS;  // queue items of a brick
+    const int part      = threadIdx.x % S;
     __shared__ int slot;
-    const int nb = *bcount;
-    for (int bi = queue_take(queue, &slot); bi < nb; bi = queue_take(queue, &slot)) {
-        const int b     = blist[bi];
+    const int nitems = *bcount * ITEMS;
+    for (int item = queue_take(queue, &slot); item < nitems; item = queue_take(queue, &slot)) {
+        const int b     = blist[item / ITEMS];
         const int3 bc   = brick_coords(L, b);
         const bool walls = bnear[b] != 0;  // boundary particles only near walls
-        for (int l4 = threadIdx.x; l4 < TPB; l4 += blockDim.x) {
+        const int first = item % ITEMS * PAIRS;
+        {
+            const int l4 = first + threadIdx.x / S;
             const int lx0 = (l4 % XS) * NX, ly = (l4 / XS) % G::BY, lz = l4 / (XS * G::BY);
             const int x0 = bc.x * G::BX + lx0, y = bc.y * G::BY + ly, z = bc.z * G::BZ + lz;
             const long long s0 = (long long) b * G::BN + lx0 + G::BX * (ly + G::BY * lz);
@@ -185,12 +204,18 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
                     const float4 * U = pass == 0 ? vel : bvel;
                     // cell rows (cy, cz) in order; the next row's range and the next
                     // candidate's position / velocity are loaded one step ahead
-                    int cy = cy0, cz = cz0;
+                    int cy = cy0 + part, cz = cz0;
+                    if (S > 1)
+                        while (cy > cy1) cy -= cy1 - cy0 + 1, cz++;
+                    if (S > 1 && cz > cz1) continue;           // fewer rows than lanes
                     const int row0 = L.nx * (cy + L.ny * cz);  // ncells < 2^31
                     int jb = cs[row0 + cxa], je = cs[row0 + cxb + 1];
                     for (;;) {
-                        int ny = cy + 1, nz = cz;
-                        if (ny > cy1) ny = cy0, nz++;
+                        int ny = cy + S, nz = cz;
+                        if (S == 1) {
+                            if (ny > cy1) ny = cy0, nz++;
+                        } else
+                            while (ny > cy1) ny -= cy1 - cy0 + 1, nz++;
                         const bool more = nz <= cz1;
                         int nb_ = 0, ne_ = 0;
                         if (more) {
@@ -232,6 +257,15 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
                         cy = ny, cz = nz, jb = nb_, je = ne_;
                     }
                 }
+            }
+            if (S > 1) {
+                __syncwarp();
+                a.wsum = lanes_sum<S>(a.wsum), a.rhoI = lanes_sum<S>(a.rhoI), a.VI = lanes_sum<S>(a.VI);
+                if (FEAT) a.cnt = lanes_sum<S>(a.cnt);
+                a.ux = lanes_sum<S>(a.ux), a.uy = lanes_sum<S>(a.uy), a.uz = lanes_sum<S>(a.uz);
+                a.bw = lanes_sum<S>(a.bw), a.dvg = lanes_sum<S>(a.dvg);
+                a.gx = lanes_sum<S>(a.gx), a.gy = lanes_sum<S>(a.gy), a.gz = lanes_sum<S>(a.gz);
+                if (part != 0) continue;  // to the next item
             }
 #pragma unroll
             for (int n = 0; n < NX; n++) {
@@ -588,7 +622,7 @@ __device__ float3 gradient_virtual_global(const Lattice & L, const Phys & P, con
 
 constexpr int kGradNT = 256;  // threads per block of the pressure gradient (one particle brick per block)
 
-template<int DIM>
+template<int DIM, int S>
 __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P, const unsigned char * __restrict__ bflag,
                                                            NodeArrays N, const int * __restrict__ plist,
                                                            const int * __restrict__ pcount,
@@ -600,7 +634,7 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
                                                            const float4 * __restrict__ bnrm,
                                                            const int * __restrict__ bcellStart,
                                                            const unsigned char * __restrict__ bcell,
-                                                           const CgState * __restrict__ cg, int * queue) {
+                                                           const CgState * __restrict__ cg, int parts, int * queue) {
     pdl_wait_and_release();
     using G = BrickGeom<DIM>;
     if (cg->done == 3) return;  // the solve broke down: the velocities stay as they are
@@ -612,10 +646,10 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
     constexpr int ROWS = G::BY * G::BZ;  // cell rows of a brick
     __shared__ int rinc[ROWS], rbeg[ROWS];
     __shared__ int slot;
-    const int nb = *pcount;
-    const int t  = threadIdx.x;
-    for (int bi = queue_take(queue, &slot); bi < nb; bi = queue_take(queue, &slot)) {
-        const int b   = plist[bi];
+    const int nitems = *pcount * parts;  // queue items: a brick's particles in `parts` pieces
+    const int t      = threadIdx.x;
+    for (int item = queue_take(queue, &slot); item < nitems; item = queue_take(queue, &slot)) {
+        const int b   = plist[item / parts];
         const int3 bc = brick_coords(L, b);
         const int x0 = bc.x * G::BX, x1 = min(x0 + G::BX, L.nx);
         load_tile4<DIM, kGradNT, PX>(L, bflag, bc, tile, [&](long long s) {
@@ -652,7 +686,8 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
             rbeg[t] -= w0;
         }
         __syncthreads();
-        const int total  = rinc[ROWS - 1];
+        const int piece = (rinc[ROWS - 1] + parts - 1) / parts, begin = item % parts * piece;
+        const int total = min(rinc[ROWS - 1], begin + piece);
         const bool walls = bnear[b] != 0;
         // tile origin (node of tile index 0) of the FP64 lattice as float-float
         // pairs: a particle's offset from it, (q - hi) - lo, is exact to a few ulp
@@ -662,62 +697,72 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
         const double tod_z = DIM == 3 ? L.oz_d + (bc.z * G::BZ - G::HALO) * L.dx_d : 0.0;
         const float tox = float(tod_x), toy = float(tod_y), toz = float(tod_z);
         const float tlx = float(tod_x - double(tox)), tly = float(tod_y - double(toy)), tlz = float(tod_z - double(toz));
-        for (int p = t; p < total; p += kGradNT) {
-            int lo = 0, hi = ROWS - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (rinc[mid] > p) hi = mid;
-                else lo = mid + 1;
-            }
-            const int j     = rbeg[lo] + p;
-            const float4 q  = pos[j];
-            const float4 vi = vel[j];
-            const float ux = ((q.x - tox) - tlx) * L.inv_dx, uy = ((q.y - toy) - tly) * L.inv_dx;
-            const float uz = DIM == 3 ? ((q.z - toz) - tlz) * L.inv_dx : 0.f;
-            float3 f = make_float3(0.f, 0.f, 0.f);
-            const bool inside = ux >= 3.f && ux < float(G::TX) - 4.f && uy >= 3.f && uy < float(G::TY) - 4.f &&
-                                (DIM == 2 || (uz >= 3.f && uz < float(G::TZ) - 4.f));
-            if (inside) {
-                // nodes within H of the particle lie in the 8^DIM window
-                // floor(u) - 3 .. floor(u) + 4 (offset -4 is excluded: r2 < 16)
-                const int cx = int(ux), cy = int(uy), cz = DIM == 3 ? int(uz) : 0;
-                const float fx = ux - float(cx - 3);
-                const float2 dxp[4] = {make_float2(fx - 2.f, fx - 3.f), make_float2(fx - 4.f, fx - 5.f),
-                                       make_float2(fx - 1.f, fx - 6.f), make_float2(fx, fx - 7.f)};
-                float2 sx = make_float2(0.f, 0.f);
-                float gy = 0.f, gz = 0.f;
-                const float fy    = uy - float(cy - 3);
-                const float * win = tile + PX * (cy - 3) + (cx - 3);
-                if constexpr (DIM == 3) {
-                    // planes 0..3 (at least 3, 2, 1, 0 away), then 7..4
-                    constexpr int PZ = PX * G::TY;
-                    const float fz   = uz - float(cz - 3);
-                    win += PZ * (cz - 3);
-                    float dz = fz, dstep = -1.f;
-                    int step = PZ;
+        for (int p0 = begin; p0 < total; p0 += kGradNT / S) {
+            const int p    = p0 + t / S;
+            const int half = t % S;
+            float3 f       = make_float3(0.f, 0.f, 0.f);
+            float4 vi      = make_float4(0.f, 0.f, 0.f, 0.f);
+            int j          = 0;
+            if (p < total) {
+                int lo = 0, hi = ROWS - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (rinc[mid] > p) hi = mid;
+                    else lo = mid + 1;
+                }
+                j = rbeg[lo] + p;
+                const float4 q = pos[j];
+                vi             = vel[j];
+                const float ux = ((q.x - tox) - tlx) * L.inv_dx, uy = ((q.y - toy) - tly) * L.inv_dx;
+                const float uz = DIM == 3 ? ((q.z - toz) - tlz) * L.inv_dx : 0.f;
+                const bool inside = ux >= 3.f && ux < float(G::TX) - 4.f && uy >= 3.f && uy < float(G::TY) - 4.f &&
+                                    (DIM == 2 || (uz >= 3.f && uz < float(G::TZ) - 4.f));
+                if (inside) {
+                    // nodes within H of the particle lie in the 8^DIM window
+                    // floor(u) - 3 .. floor(u) + 4 (offset -4 is excluded: r2 < 16)
+                    const int cx = int(ux), cy = int(uy), cz = DIM == 3 ? int(uz) : 0;
+                    const float fx = ux - float(cx - 3);
+                    const float2 dxp[4] = {make_float2(fx - 2.f, fx - 3.f), make_float2(fx - 4.f, fx - 5.f),
+                                           make_float2(fx - 1.f, fx - 6.f), make_float2(fx, fx - 7.f)};
+                    float2 sx = make_float2(0.f, 0.f);
+                    float gy = 0.f, gz = 0.f;
+                    const float fy    = uy - float(cy - 3);
+                    const float * win0 = tile + PX * (cy - 3) + (cx - 3);
+                    if constexpr (DIM == 3) {
+                        // planes 0..3 (at least 3, 2, 1, 0 away), then 7..4
+                        constexpr int PZ = PX * G::TY;
+                        const float fz   = uz - float(cz - 3);
+                        win0 += PZ * (cz - 3);
+                        // (with two lanes a particle, one of the halves each)
 #pragma unroll 1
-                    for (int h = 0; h < 2; h++) {
-                        gradient_plane<PX, 3>(win, dxp, fy, dz, sx, gy, gz);
-                        gradient_plane<PX, 2>(win + step, dxp, fy, dz + dstep, sx, gy, gz);
-                        gradient_plane<PX, 1>(win + 2 * step, dxp, fy, dz + 2.f * dstep, sx, gy, gz);
-                        gradient_plane<PX, 0>(win + 3 * step, dxp, fy, dz + 3.f * dstep, sx, gy, gz);
-                        win += 7 * PZ;
-                        step  = -PZ;
-                        dz    = fz - 7.f;
-                        dstep = 1.f;
-                    }
-                } else gradient_plane<PX, 0>(win, dxp, fy, 0.f, sx, gy, gz);
-                f = make_float3(P.c1H * (sx.x + sx.y), P.c1H * gy, P.c1H * gz);
-            } else {
-                f = gradient_virtual_global<DIM>(L, P, bflag, N, q);
+                        for (int h = half; h < 2; h += S) {
+                            const float dz = h ? fz - 7.f : fz, dstep = h ? 1.f : -1.f;
+                            const int step = h ? -PZ : PZ;
+                            const float * win = win0 + (h ? 7 * PZ : 0);
+                            gradient_plane<PX, 3>(win, dxp, fy, dz, sx, gy, gz);
+                            gradient_plane<PX, 2>(win + step, dxp, fy, dz + dstep, sx, gy, gz);
+                            gradient_plane<PX, 1>(win + 2 * step, dxp, fy, dz + 2.f * dstep, sx, gy, gz);
+                            gradient_plane<PX, 0>(win + 3 * step, dxp, fy, dz + 3.f * dstep, sx, gy, gz);
+                        }
+                    } else gradient_plane<PX, 0>(win0, dxp, fy, 0.f, sx, gy, gz);
+                    f = make_float3(P.c1H * (sx.x + sx.y), P.c1H * gy, P.c1H * gz);
+                } else if (half == 0) {
+                    f = gradient_virtual_global<DIM>(L, P, bflag, N, q);
+                }
+                // the wall sum only for particles whose cell is within reach of the boundary
+                if (walls && bcell[cell_linear(L, cell_of<DIM>(L, q.x, q.y, q.z))]) {
+                    const float3 w = wall_term<DIM, S>(L, P, bcellStart, bpos, bvel, bnrm, q, vi, half);
+                    f.x += w.x;
+                    f.y += w.y;
+                    f.z += w.z;
+                }
             }
-            // the wall sum only for particles whose cell is within reach of the boundary
-            if (walls && bcell[cell_linear(L, cell_of<DIM>(L, q.x, q.y, q.z))]) {
-                const float3 w = wall_term<DIM>(L, P, bcellStart, bpos, bvel, bnrm, q, vi);
-                f.x += w.x;
-                f.y += w.y;
-                f.z += w.z;
+            if (S == 2) {
+                f.x += __shfl_xor_sync(0xffffffffu, f.x, 1);
+                f.y += __shfl_xor_sync(0xffffffffu, f.y, 1);
+                f.z += __shfl_xor_sync(0xffffffffu, f.z, 1);
             }
+            if (p >= total || half != 0) continue;
             float4 o = vi;
             o.x += f.x;
             o.y += f.y;
@@ -736,13 +781,22 @@ void launch_pressure_gradient(const Lattice & L, const Phys & P, const BrickArra
                               const int * plist, const int * pcount, const unsigned char * bnear, const float4 * pos,
                               float4 * vel, const int * cellStart, const float4 * bpos, const float4 * bvel,
                               const float4 * bnrm, const int * bcellStart, const unsigned char * bcell,
-                              const CgState * cg, int grid, int * queue, cudaStream_t st) {
-    launch_pdl(k_pressure_gradient<DIM>, grid, kGradNT, 0, st, L, P, B.flag, N, plist, pcount, bnear, pos, vel, cellStart, bpos,
-                                                   bvel, bnrm, bcellStart, bcell, cg, queue);
+                              const CgState * cg, long long np, int grid, int * queue, cudaStream_t st) {
+    // Pieces of a brick and (3D) lanes per particle, one half of the planes each, while
+    // bricks are fewer than the resident blocks (608): with 1 x 1, 1 x 2, 2 x 1, 2 x 2 pieces
+    // x lanes 43 38 35 27 us at 15,625 particles, 73 58 54 56 at 167k, 83 78 84 80 at 262k,
+    // 118 114 118 121 at 524k, 364 383 419 450 at 2.1M.
+    const int parts = np <= (1 << 18) ? 2 : 1, S = DIM == 3 ? parts : 1;
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, int(std::min<long long>(grid, (long long) L.nbricks * parts)), kGradNT, 0, st, L, P, B.flag, N,
+                   plist, pcount, bnear, pos, vel, cellStart, bpos, bvel, bnrm, bcellStart, bcell, cg, parts, queue);
+    };
+    if (DIM == 3 && S == 2) go(k_pressure_gradient<DIM, DIM == 3 ? 2 : 1>);
+    else go(k_pressure_gradient<DIM, 1>);
 }
 template<int DIM> int pressure_gradient_blocks_per_sm() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pressure_gradient<DIM>, kGradNT, 0) != cudaSuccess) n = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pressure_gradient<DIM, 1>, kGradNT, 0) != cudaSuccess) n = 1;
     return n > 0 ? n : 1;
 }
 template<int DIM> int node_gather_blocks_per_sm() {
@@ -750,8 +804,8 @@ template<int DIM> int node_gather_blocks_per_sm() {
         int k = 0;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, 128, 0) == cudaSuccess ? k : 1;
     };
-    const int n = std::min(std::min(blocks(k_node_gather<DIM, true, true>), blocks(k_node_gather<DIM, true, false>)),
-                           std::min(blocks(k_node_gather<DIM, false, true>), blocks(k_node_gather<DIM, false, false>)));
+    const int n = std::min(std::min(blocks(k_node_gather<DIM, true, true, 1>), blocks(k_node_gather<DIM, true, false, 1>)),
+                           std::min(blocks(k_node_gather<DIM, false, true, 1>), blocks(k_node_gather<DIM, false, false, 1>)));
     return n > 0 ? n : 1;
 }
 void launch_brick_list(const unsigned char * bflag, int nbricks, int * list, int * count, cudaStream_t st) {
@@ -762,16 +816,28 @@ template<int DIM>
 void launch_node_gather(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N,
                         const float4 * pos, const float4 * vel, const int * cellStart, const float4 * bpos,
                         const float4 * bvel, const int * bcellStart, const unsigned char * bnear,
-                        const unsigned char * bcell, int grid, int * queue, cudaStream_t st) {
+                        const unsigned char * bcell, long long np, int grid, int * queue, cudaStream_t st) {
     // H >= 2h: particles within h only reach the inner branch of W_H; the
     // real-neighbour counts only where N.nreal is given
     const bool fast = double(P.H) >= 2.0 * double(P.h) * (1.0 - 1e-6), feat = N.nreal != nullptr;
-    auto go = [&](auto kernel) {
-        launch_pdl(kernel, grid, 128, 0, st, L, P, B.list, B.count, N, pos, vel, cellStart, bpos, bvel, bcellStart, bnear,
-                   bcell, queue);
+    auto go = [&](auto kernel, int s) {
+        const long long items = (long long) L.nbricks * (DIM == 3 ? 2 : 1) * s;
+        launch_pdl(kernel, int(std::min<long long>(grid, items)), 128, 0, st, L, P, B.list, B.count, N, pos, vel, cellStart,
+                   bpos, bvel, bcellStart, bnear, bcell, queue);
     };
-    if (fast) feat ? go(k_node_gather<DIM, true, true>) : go(k_node_gather<DIM, true, false>);
-    else feat ? go(k_node_gather<DIM, false, true>) : go(k_node_gather<DIM, false, false>);
+    auto lanes = [&](auto s) {
+        constexpr int S = decltype(s)::value;
+        if (fast) feat ? go(k_node_gather<DIM, true, true, S>, S) : go(k_node_gather<DIM, true, false, S>, S);
+        else feat ? go(k_node_gather<DIM, false, true, S>, S) : go(k_node_gather<DIM, false, false, S>, S);
+    };
+    // Lanes per node pair, by the particles (about as many as nodes): four while they fit
+    // the resident threads (97k at five blocks of 128 per SM), two up to three rounds of
+    // them.  Measured with 1, 2, 4 lanes: 41 24 22 us at 15,625 particles, 65 60 65 at 167k,
+    // 90 87 97 at 262k, 123 134 156 at 524k, 435 500 622 at 2.1M.
+    const int S = np <= 48000 ? 4 : np <= 290000 ? 2 : 1;
+    if (S == 4) lanes(std::integral_constant<int, 4>{});
+    else if (S == 2) lanes(std::integral_constant<int, 2>{});
+    else lanes(std::integral_constant<int, 1>{});
 }
 
 template<int DIM>
@@ -814,13 +880,13 @@ void launch_compact_import(const Lattice & L, const BrickArrays & B, const NodeA
 #define SWC_INST(D)                                                                                                    \
     template void launch_node_gather<D>(const Lattice &, const Phys &, const BrickArrays &, const NodeArrays &,        \
                                         const float4 *, const float4 *, const int *, const float4 *, const float4 *,   \
-                                        const int *, const unsigned char *, const unsigned char *, int, int *,         \
-                                        cudaStream_t);                                                                 \
+                                        const int *, const unsigned char *, const unsigned char *, long long, int,     \
+                                        int *, cudaStream_t);                                                                 \
     template void launch_pressure_gradient<D>(const Lattice &, const Phys &, const BrickArrays &, const NodeArrays &,  \
                                               const int *, const int *, const unsigned char *, const float4 *,         \
                                               float4 *, const int *, const float4 *, const float4 *, const float4 *,   \
-                                              const int *, const unsigned char *, const CgState *, int, int *,         \
-                                              cudaStream_t);                                                           \
+                                              const int *, const unsigned char *, const CgState *, long long, int,     \
+                                              int *, cudaStream_t);                                                    \
     template int pressure_gradient_blocks_per_sm<D>();                                                                 \
     template int node_gather_blocks_per_sm<D>();                                                                       \
     template void launch_segments<D>(const Lattice &, const BrickArrays &, const NodeArrays &, int *, int,             \

@@ -321,7 +321,7 @@ template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features =
     NodeArrays N = c->N;
     if (!features) N.nreal = nullptr;
     launch_node_gather<DIM>(c->L, c->P, c->B, N, c->pos, c->vel, c->cellStart, c->bpos, c->bvel, c->bcellStart,
-                            c->bnear, c->bcell, c->ggrid, c->queues, c->stream);
+                            c->bnear, c->bcell, c->n, c->ggrid, c->queues, c->stream);
     launch_segments<DIM>(c->L, c->B, c->N, c->scan_tiles, c->grid, c->stream);
     if (with_ahat) launch_ahat<DIM>(c->L, c->P, c->B, c->N, c->S, c->cgrid, c->stream);
 }
@@ -483,7 +483,7 @@ template<int DIM> int queue_projection(swc_ctx * c, Projection & pr) {
     mark(c, 6);
     // leaves the velocities unprojected when the solve broke down (cg->done = 3)
     launch_pressure_gradient<DIM>(c->L, c->P, c->B, c->N, c->plist, c->pcount, c->bnear, c->pos, c->vel,
-                                  c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->cg, c->pgrid,
+                                  c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->cg, c->n, c->pgrid,
                                   c->queues + 2, c->stream);
     mark(c, 7);
     // p in reference order (the next step's prefix warm start) and N_v for it;
@@ -736,8 +736,8 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
         const int go  = d3 ? node_gather_blocks_per_sm<3>() : node_gather_blocks_per_sm<2>();
         const int po  = d3 ? pressure_gradient_blocks_per_sm<3>() : pressure_gradient_blocks_per_sm<2>();
         c->cgrid      = std::max(1, std::min(L.nbricks, c->num_sms));
-        c->ggrid      = std::max(1, std::min(L.nbricks, c->num_sms * go));
-        c->pgrid      = std::max(1, std::min(L.nbricks, c->num_sms * po));
+        c->ggrid      = c->num_sms * go;
+        c->pgrid      = c->num_sms * po;
     }
     if (s->dim == 3 ? cg_solve_prepare<3>() : cg_solve_prepare<2>()) {
         cudaGetLastError();
@@ -1339,12 +1339,12 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
             switch (which) {
             case 2:
                 launch_node_gather<3>(c->L, c->P, c->B, c->N, c->pos, c->vel, c->cellStart, c->bpos, c->bvel,
-                                      c->bcellStart, c->bnear, c->bcell, c->ggrid, c->queues, c->stream);
+                                      c->bcellStart, c->bnear, c->bcell, c->n, c->ggrid, c->queues, c->stream);
                 break;
             case 3:
                 launch_pressure_gradient<3>(c->L, c->P, c->B, c->N, c->plist, c->pcount, c->bnear, c->pos, c->vel,
                                             c->cellStart, c->bpos, c->bvel, c->bnrm, c->bcellStart, c->bcell, c->cg,
-                                            c->pgrid, c->queues + 2, c->stream);
+                                            c->n, c->pgrid, c->queues + 2, c->stream);
                 break;
             case 4: launch_density<3>(c->pos, c->vel, c->rho, c->n, c->L, c->P, c->cellStart, c->pleft, c->stream); break;
             case 5: launch_forces<3>(c->pos, c->vel, c->vel2, c->n, c->L, c->P, c->cellStart, 0.f, c->pleft, c->stream); break;
@@ -1353,7 +1353,7 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
             switch (which) {
             case 2:
                 launch_node_gather<2>(c->L, c->P, c->B, c->N, c->pos, c->vel, c->cellStart, c->bpos, c->bvel,
-                                      c->bcellStart, c->bnear, c->bcell, c->ggrid, c->queues, c->stream);
+                                      c->bcellStart, c->bnear, c->bcell, c->n, c->ggrid, c->queues, c->stream);
                 break;
             case 4: launch_density<2>(c->pos, c->vel, c->rho, c->n, c->L, c->P, c->cellStart, c->pleft, c->stream); break;
             default: break;

@@ -488,12 +488,14 @@ template<int DIM> __device__ __forceinline__ bool near_pair(const Lattice & L, f
 // Friction-free wall term of the pressure-gradient update for particle
 // (q, vi): - sum_b V_b min(n_b.(v_i - v_b), 0) n_b W_h(x_i - x_b)
 // (VirtualParticle::applyPressureGradient, Cores/Structures/VirtualParticle.cpp:122-128).
-template<int DIM>
+// With S lanes a particle, lane `part`'s share of the rows.
+template<int DIM, int S>
 __device__ __forceinline__ float3 wall_term(const Lattice & L, const Phys & P, const int * __restrict__ bcellStart,
                                             const float4 * __restrict__ bpos, const float4 * __restrict__ bvel,
-                                            const float4 * __restrict__ bnrm, float4 q, float4 vi) {
+                                            const float4 * __restrict__ bnrm, float4 q, float4 vi, int part) {
     float3 f = make_float3(0.f, 0.f, 0.f);
-    for_each_in_radius<DIM>(L, bcellStart, q.x, q.y, q.z, P.h, P.h2, [&](int j) {
+    const float3 at = make_float3(q.x, q.y, q.z);
+    for_each_in_radius2<DIM, S>(L, bcellStart, at, at, P.h, P.h2, [&](int j) {
         const float4 p = bpos[j];
         const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         const float r2 = dx * dx + dy * dy + dz * dz;
@@ -506,7 +508,7 @@ __device__ __forceinline__ float3 wall_term(const Lattice & L, const Phys & P, c
             f.y -= c * nb.y;
             f.z -= c * nb.z;
         }
-    });
+    }, part);
     return f;
 }
 

@@ -123,7 +123,8 @@ template<int DIM>
 void launch_node_gather(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N,
                         const float4 * pos, const float4 * vel, const int * cellStart, const float4 * bpos,
                         const float4 * bvel, const int * bcellStart, const unsigned char * bnear,
-                        const unsigned char * bcell, int grid, int * queue, cudaStream_t st);
+                        const unsigned char * bcell, long long np, int grid, int * queue, cudaStream_t st);
+// (np: particles, for the split of the work)
 // Pressure-gradient update over the bricks that hold particles (plist / pcount),
 // node field staged per brick in shared memory; bnear flags bricks near walls.
 template<int DIM>
@@ -131,7 +132,7 @@ void launch_pressure_gradient(const Lattice & L, const Phys & P, const BrickArra
                               const int * plist, const int * pcount, const unsigned char * bnear, const float4 * pos,
                               float4 * vel, const int * cellStart, const float4 * bpos, const float4 * bvel,
                               const float4 * bnrm, const int * bcellStart, const unsigned char * bcell,
-                              const CgState * cg, int grid, int * queue, cudaStream_t st);
+                              const CgState * cg, long long np, int grid, int * queue, cudaStream_t st);
 // Resident blocks per SM of the persistent brick kernels (their grids are
 // SMs x this; gather and gradient take bricks from a zero-initialised queue of
 // two ints).
