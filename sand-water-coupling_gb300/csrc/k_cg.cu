@@ -243,15 +243,6 @@ void launch_cg_residual(const Lattice & L, const BrickArrays & B, const NodeArra
     launch_pdl(k_vmul<DIM>, ugrid, kUT, 0, st, B.list, B.count, N.V, x, N.u);
     launch_rows_residual<DIM>(L, B, N, S, x, r, d, sums, cg, partials, rblocks, st);
 }
-// r = b - A x: u = V x staged in N.u (free until the first CG direction pass),
-// the tiled residual pass, the start state.
-template<int DIM>
-void launch_cg_init(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    double * partials, double tol, int max_iterations, const int * nv, int rblocks, int ugrid,
-                    cudaStream_t st) {
-    launch_cg_residual<DIM>(L, B, N, S, N.x, N.r, N.d, cg->sums, cg, partials, rblocks, ugrid, st);
-    launch_pdl(k_cg_start, 1, 32, 0, st, cg, cg->sums, nullptr, nullptr, 0, tol, max_iterations, nv);
-}
 // Start state keeping the better of the prediction (residual in cg->sums[0..1],
 // already in N.x / N.r / N.d) and the base start xb (cg->sums[2..3], residual rb),
 // and the base copied in when it wins.
@@ -277,8 +268,6 @@ void launch_rhs_norm(const BrickArrays & B, const NodeArrays & N, CgState * cg, 
 #define SWC_INST(D)                                                                                                    \
     template void launch_apply_operator<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,   \
                                            const float *, float *, int, cudaStream_t);                                 \
-    template void launch_cg_init<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,         \
-                                    CgState *, double *, double, int, const int *, int, int, cudaStream_t);            \
     template void launch_cg_residual<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,     \
                                         const float *, float *, float *, double *, CgState *, double *, int, int,      \
                                         cudaStream_t);                                                                 \

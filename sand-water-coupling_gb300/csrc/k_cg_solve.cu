@@ -8,6 +8,9 @@
 //   step      x += alpha d, r -= alpha q, d = r + beta d, u = V d       (streaming)
 //   product   q = A d from the halo tile of u (swc_stencil.cuh), and the four dot
 //             products d.q, r.q, q.q, r.r
+// (before the first: u = V x, r = d = b - A x, r.r and b.b, and the stopping threshold,
+// unless the caller queued a start of its own.  As three launches, with the sums in FP64
+// in every block, the start took 19 us at 15,625 particles, against 7 here.)
 // alpha = r.r / d.q, and |r - alpha q|^2 = r.r - 2 alpha r.q + alpha^2 q.q gives beta
 // and the stopping test without a second trip: the sums hold 44 bits and more, the
 // quotient of two successive norms is seldom below a tenth, and where it is below
@@ -17,6 +20,8 @@
 // blocks meet once per iteration, for the sums, and each decides by itself whether to
 // go on, with no host check.  Dot products use exact FP32 products in float-float per
 // lane, triple floats below the block and FP64 above, in a fixed order.
+#include <type_traits>
+
 #include "swc_kernels.h"
 #include "swc_stencil.cuh"
 
@@ -165,10 +170,18 @@ struct CgScalars {
 template<int WARPS> struct MeetSmem {
     F3        part[WARPS][kSums];
     F3        sum[kSums];
+    double    start[2];
+    int       nv;  // block 0
     int       full[kSums];
     Outcome   out;
     CgScalars cg;  // block 0
 };
+// The power of two that brings |b|^2 to about 1.
+__device__ __forceinline__ float sum_scale(double bb) { return exp2f(float(-max(-120, min(120, ilogb(bb))))); }
+__device__ __forceinline__ CgScalars scalars_of(double rr, double threshold, int max_iter, float scale) {
+    const F3 r = f3_of(rr * double(scale)), t = f3_of(threshold * double(scale));
+    return CgScalars{F3{0.f, 0.f, 0.f}, r, r, t.h, t.m, 0, max_iter};
+}
 constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer blocks poll one line
 
 // The factors and the stopping test from the sums d.q, r.q, q.q, r.r (after kMeasure:
@@ -200,6 +213,38 @@ __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums],
     return o;
 }
 
+// Start state from |r|^2 and |b|^2 (Eigen's stopping rule: |r|^2 < max(tol, eps/|b|)^2
+// |b|^2, cap 2 N_v).  The outcome's alpha is the power of two that scales the sums.
+__device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, double rr, double bb, int nv,
+                                               const CgStart & from) {
+    const int cap = from.max_iterations >= 0 ? from.max_iterations : 2 * nv;
+    const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
+    int done = 0;
+    double threshold = 0;
+    if (nv == 0 || bb == 0.0) done = bb == 0.0 ? 4 : 1;  // 4: zero right-hand side -> x = 0
+    else {
+        // (the quotient only where it may be the larger one)
+        double tt = from.tolerance;
+        if (!(tt * tt * bb > 4 * eps * eps)) tt = fmax(tt, eps / sqrt(bb));
+        threshold = fmax(tt * tt * bb, dmin);
+        done      = rr < threshold ? 1 : (rr != rr ? 3 : 0);
+        if (done == 0 && cap <= 0) done = 2;
+    }
+    cg->start     = 0;
+    cg->bb        = bb;
+    cg->rr        = rr;
+    cg->rr0       = rr;
+    cg->rr_prev   = 0;
+    cg->pq        = 0;
+    cg->iter      = 0;
+    cg->max_iter  = cap;
+    cg->threshold = threshold;
+    cg->done      = done;
+    const float scale = sum_scale(bb);
+    c = scalars_of(rr, threshold, cap, scale);
+    return Outcome{scale, 0.f, unsigned(done)};
+}
+
 // Meeting of the blocks in use: v (value lane / 8 of the warp, as warp_sum4 gives it)
 // summed over their first `active` warps, and what block 0 decides on the sums, the
 // same on every thread.  Every block publishes its four partials under the meeting's
@@ -208,9 +253,11 @@ __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums],
 // with the sums published and FP64 quotients formed by every thread, 5 us.)  One set of
 // slots serves: a block publishes again only after it has the outcome, and block 0
 // only after every block has published again.
-template<int WARPS>
+// START: values 0 and 1 are |r|^2 and |b|^2, unscaled, in FP64 above the block (once a
+// solve, by one warp each); `decided` makes the outcome of the sums.
+template<bool START, int WARPS, class Decide>
 __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int stride, int blocks, int active,
-                                        unsigned & tag, MeetSmem<WARPS> & M, float alpha, bool measured) {
+                                        unsigned & tag, MeetSmem<WARPS> & M, Decide decided) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ulonglong2 * outcome = slots + (long long) stride * kSums;
     if ((lane & 7) == 0) M.part[warp][lane >> 3] = v;
@@ -221,7 +268,13 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
         for (int j = w; j < active; j += 8) part = f3_add(part, M.part[j][k]);
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) part = f3_add(part, f3_shfl(part, o));
-        if (w == 0) slot_put(slots + (long long) blockIdx.x * kSums + k, part, tag);
+        if (w == 0) {
+            ulonglong2 * p = slots + (long long) blockIdx.x * kSums + k;
+            if constexpr (START) {
+                if (k < 2)
+                    word_put(p, (unsigned long long) __double_as_longlong(f3_double(part)), (unsigned long long) tag << 32);
+            } else slot_put(p, part, tag);
+        }
         if (blockIdx.x != 0 && lane == 0) {
             const ulonglong2 * p = outcome + blockIdx.x % kCopies;
             Outcome o;
@@ -233,7 +286,27 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
     }
     if (blockIdx.x == 0) {
         // a warp per value, five slots a lane at once
-        if (warp < kSums) {
+        if constexpr (START) {
+            if (warp < 2) {
+                double s  = 0;
+                bool full = true;
+                for (int j = lane; j < blocks; j += 32) {
+                    ulonglong2 w{0, 0};
+                    bool there = false;
+                    for (int n = 0; n < kMeetPolls && !there; n++) {
+                        w     = word_get(slots + (long long) j * kSums + warp);
+                        there = unsigned(w.y >> 32) == tag;
+                    }
+                    full = full && there;
+                    s += __longlong_as_double((long long) w.x);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+                full = __all_sync(0xffffffffu, full);
+                if (lane == 0) M.start[warp] = s, M.full[warp] = full;
+            }
+        } else if (warp < kSums) {
             F3 s{0.f, 0.f, 0.f};
             bool full = true;
             for (int j0 = lane; j0 < blocks; j0 += 32 * 5) {
@@ -263,13 +336,19 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
         }
         __syncthreads();
         if (warp == 0) {
-            const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
-            CgScalars c         = M.cg;
-            Outcome o           = decide(c, sum, alpha, measured);
-            if (!(M.full[0] && M.full[1] && M.full[2] && M.full[3])) o.code = kFailed;
-            if (lane < kCopies) outcome_put(outcome + lane, o, tag);
-            __syncwarp();
-            if (lane == 0) M.cg = c, M.out = o;
+            if (!START || lane == 0) {
+                CgScalars c = M.cg;
+                Outcome o   = decided(c);
+                const bool full = M.full[0] && M.full[1] && (START || (M.full[2] && M.full[3]));
+                if (!full) o.code = kFailed;
+                if (!START && lane < kCopies) outcome_put(outcome + lane, o, tag);
+                __syncwarp(START ? 1u : 0xffffffffu);
+                if (lane == 0) M.cg = c, M.out = o;
+            }
+            if (START) {
+                __syncwarp();
+                if (lane < kCopies) outcome_put(outcome + lane, M.out, tag);
+            }
         }
     }
     __syncthreads();
@@ -292,8 +371,8 @@ __device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const in
 template<int DIM, int W>
 __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict__ blist, int nb, int P,
                                       const unsigned char * __restrict__ bflag, const NodeArrays & N, const Stencil & S,
-                                      CgState * cg, ulonglong2 * slots, unsigned * flags, CgPhases * phases,
-                                      MeetSmem<WarpBrick<DIM>::WARPS> & M) {
+                                      CgState * cg, const CgStart & from, ulonglong2 * slots, unsigned * flags,
+                                      CgPhases * phases, MeetSmem<WarpBrick<DIM>::WARPS> & M) {
     using B  = WarpBrick<DIM>;
     using G  = typename B::G;
     using Gr = Group<DIM, W>;
@@ -308,17 +387,16 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     fill_segments<DIM>(seg);
     for (int k = 0, bi = bfirst; k < B::TABS && bi < nb; k++, bi += bstep)
         fill_neighbours<DIM>(L, bflag, blist[bi], gl, tab + 27 * k);
-    // the sums' power of two
-    const float scale = exp2f(float(-max(-120, min(120, ilogb(cg->bb)))));
-    if (threadIdx.x == 0) {
-        const F3 rr = f3_of(cg->rr * double(scale)), t = f3_of(cg->threshold * double(scale));
-        M.cg        = CgScalars{F3{0.f, 0.f, 0.f}, rr, rr, t.h, t.m, 0, cg->max_iter};
+    float scale = 1.f;
+    if (!from.own) {
+        scale = sum_scale(cg->bb);
+        if (threadIdx.x == 0) M.cg = scalars_of(cg->rr, cg->threshold, cg->max_iter, scale);
     }
     __syncthreads();
     const int active = W * min(Gr::COUNT, (nb - int(blockIdx.x) + P - 1) / P);  // warps with bricks
 
     Outcome o{0.f, 0.f, kGoOn};
-    bool first   = true, ok = true;
+    bool first = true, ok = true;
     unsigned tag = cg->tick + 1;
     CgPhases spent{0, 0, 0};
     unsigned long long mark = phases ? global_ns() : 0;
@@ -329,7 +407,100 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
             mark = now;
         }
     };
-    for (;;) {
+    // u is there: the bricks' flags
+    auto publish = [&]() {
+        if (!idle) {
+            Gr::sync();
+            if (gl == 0) {
+                fence_gpu();
+                for (int bi = bfirst; bi < nb; bi += bstep) st_relaxed(flags + blist[bi], tag);
+            }
+        }
+    };
+    auto product = [&](auto start, FF (&part)[kSums]) {
+        constexpr bool START = decltype(start)::value;
+        for (int k = 0, bi = bfirst; bi < nb; bi += bstep, k++) {
+            const int b = blist[bi];
+            int * t     = tab + 27 * min(k, B::TABS);
+            if (k >= B::TABS) {
+                Gr::sync();
+                fill_neighbours<DIM>(L, bflag, b, gl, t);
+                __syncwarp();
+            }
+            if (gl < 32 && !wait_neighbours(flags, t, tag)) ok = false;
+            Gr::sync();  // also past the last brick's reads of the tile
+            tile_copy<DIM, W>(seg, t, N.u, tile);
+            const long long base = (long long) b * G::BN;
+            float q[Gr::NOUT];
+            // with few bricks the row's own operands are loaded under the tile's copy
+            constexpr bool FEW  = W == B::WMAX;
+            constexpr int AHEAD = FEW ? Gr::NOUT / 4 : 1;
+            float4 d_[AHEAD], a_[AHEAD], r_[AHEAD];
+            unsigned f_[AHEAD];
+            auto operands = [&](int i, int at) {  // (x and b for the start)
+                const long long s = base + Gr::row(i / Gr::NX) + i % Gr::NX;
+                d_[at] = ld4(START ? N.x : N.d, s), a_[at] = ld4(N.ahat, s), r_[at] = ld4(START ? N.D : N.r, s);
+                f_[at] = *reinterpret_cast<const unsigned *>(N.flag + s);
+            };
+            if constexpr (FEW) {
+#pragma unroll
+                for (int i = 0; i < Gr::NOUT; i += 4) operands(i, i / 4);
+            }
+            tile_wait<DIM, W>();
+            group_stencil<DIM, W>(tile, S, q);
+#pragma unroll
+            for (int i = 0; i < Gr::NOUT; i += 4) {
+                const long long s = base + Gr::row(i / Gr::NX) + i % Gr::NX;
+                const int at      = FEW ? i / 4 : 0;
+                if constexpr (!FEW) operands(i, 0);
+                const unsigned fl = f_[at];
+                const float4 d = d_[at], a = a_[at], r = r_[at];
+                float p[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    p[j] = (fl >> (8 * j)) & 0xffu ? fmaf(comp(a, j), comp(d, j), q[i + j]) : comp(d, j);
+                if constexpr (START) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        p[j] = comp(r, j) - p[j];
+                        ff_add_prod(part[0], p[j], p[j]);
+                        ff_add_prod(part[1], comp(r, j), comp(r, j));
+                    }
+                    st4(N.r, s, make_float4(p[0], p[1], p[2], p[3]));
+                    st4(N.d, s, make_float4(p[0], p[1], p[2], p[3]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        ff_add_prod(part[0], comp(d, j), p[j]);
+                        ff_add_prod(part[1], comp(r, j), p[j]);
+                        ff_add_prod(part[2], p[j], p[j]);
+                        ff_add_prod(part[3], comp(r, j), comp(r, j));
+                    }
+                    st4(N.q, s, make_float4(p[0], p[1], p[2], p[3]));
+                }
+            }
+        }
+    };
+    if (from.own) {
+        for (int bi = bfirst; bi < nb; bi += bstep) {
+            const long long base = (long long) blist[bi] * G::BN + 4 * gl;
+#pragma unroll 2
+            for (int k = 0; k < Q; k++) {
+                const long long s = base + 4 * Gr::NT * k;
+                st4(N.u, s, mul4(ld4(N.V, s), ld4(N.x, s)));
+            }
+        }
+        publish();
+        FF part[kSums] = {};
+        product(std::true_type{}, part);
+        o = meet<true>(warp_sum4(part, 1.f), slots, gridDim.x, P, active, tag, M, [&](CgScalars & c) {
+            return decide_start(cg, c, M.start[0], M.start[1], M.nv, from);
+        });
+        scale = o.alpha;
+        mark  = phases ? global_ns() : 0;
+    }
+    const bool started = o.code == kGoOn;
+    while (o.code == kGoOn) {
         for (int bi = bfirst; bi < nb; bi += bstep) {
             const long long base = (long long) blist[bi] * G::BN + 4 * gl;
 #pragma unroll 2
@@ -349,66 +520,16 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 st4(N.u, s, mul4(v, d));
             }
         }
-        if (!idle) {
-            Gr::sync();
-            if (gl == 0) {
-                fence_gpu();
-                for (int bi = bfirst; bi < nb; bi += bstep) st_relaxed(flags + blist[bi], tag);
-            }
-        }
+        publish();
         lap(spent.step);
 
         FF part[kSums] = {};
-        for (int k = 0, bi = bfirst; bi < nb; bi += bstep, k++) {
-            const int b = blist[bi];
-            int * t     = tab + 27 * min(k, B::TABS);
-            if (k >= B::TABS) {
-                Gr::sync();
-                fill_neighbours<DIM>(L, bflag, b, gl, t);
-                __syncwarp();
-            }
-            if (gl < 32 && !wait_neighbours(flags, t, tag)) ok = false;
-            Gr::sync();  // also past the last brick's reads of the tile
-            tile_copy<DIM, W>(seg, t, N.u, tile);
-            const long long base = (long long) b * G::BN;
-            float q[Gr::NOUT];
-            // with few bricks the row's own operands are loaded under the tile's copy
-            constexpr bool FEW  = W == B::WMAX;
-            constexpr int AHEAD = FEW ? Gr::NOUT / 4 : 1;
-            float4 d_[AHEAD], a_[AHEAD], r_[AHEAD];
-            unsigned f_[AHEAD];
-            auto operands = [&](int i, int at) {
-                const long long s = base + Gr::row(i / Gr::NX) + i % Gr::NX;
-                d_[at] = ld4(N.d, s), a_[at] = ld4(N.ahat, s), r_[at] = ld4(N.r, s);
-                f_[at] = *reinterpret_cast<const unsigned *>(N.flag + s);
-            };
-            if constexpr (FEW) {
-#pragma unroll
-                for (int i = 0; i < Gr::NOUT; i += 4) operands(i, i / 4);
-            }
-            tile_wait<DIM, W>();
-            group_stencil<DIM, W>(tile, S, q);
-#pragma unroll
-            for (int i = 0; i < Gr::NOUT; i += 4) {
-                const long long s = base + Gr::row(i / Gr::NX) + i % Gr::NX;
-                const int at      = FEW ? i / 4 : 0;
-                if constexpr (!FEW) operands(i, 0);
-                const unsigned fl = f_[at];
-                const float4 d = d_[at], a = a_[at], r = r_[at];
-                float p[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    p[j] = (fl >> (8 * j)) & 0xffu ? fmaf(comp(a, j), comp(d, j), q[i + j]) : comp(d, j);
-                    ff_add_prod(part[0], comp(d, j), p[j]);
-                    ff_add_prod(part[1], comp(r, j), p[j]);
-                    ff_add_prod(part[2], p[j], p[j]);
-                    ff_add_prod(part[3], comp(r, j), comp(r, j));
-                }
-                st4(N.q, s, make_float4(p[0], p[1], p[2], p[3]));
-            }
-        }
+        product(std::false_type{}, part);
         lap(spent.product);
-        o     = meet<B::WARPS>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, 0.f, false);
+        o = meet<false>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, [&](CgScalars & c) {
+            const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
+            return decide(c, sum, 0.f, false);
+        });
         first = false;
         if (o.code == kMeasure) {
 #pragma unroll
@@ -422,33 +543,40 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                     for (int j = 0; j < 4; j++) ff_add_prod(part[0], comp(r, j), comp(r, j));
                 }
             }
-            o = meet<B::WARPS>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, o.alpha, true);
+            const float alpha = o.alpha;
+            o = meet<false>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, [&](CgScalars & c) {
+                const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
+                return decide(c, sum, alpha, true);
+            });
         }
         lap(spent.meeting);
-        if (o.code != kGoOn) break;
     }
     if (!__syncthreads_and(ok)) o.code = kFailed;
-    // the last step of x; a breakdown leaves x = 0
-    if (o.code != kFailed)
+    // the last step of x (none after a start that is the solution already, or a cap of no
+    // iterations); a breakdown, a start that is not a number and b = 0 leave x = 0
+    const bool zero = o.code >= 3;
+    if (o.code != kFailed && (started || zero))
         for (int bi = bfirst; bi < nb; bi += bstep) {
             const long long base = (long long) blist[bi] * G::BN + 4 * gl;
 #pragma unroll
             for (int k = 0; k < Q; k++) {
                 const long long s = base + 4 * Gr::NT * k;
-                st4(N.x, s, o.code == 3 ? make_float4(0.f, 0.f, 0.f, 0.f) : fma4(o.alpha, ld4(N.d, s), ld4(N.x, s)));
+                st4(N.x, s, zero ? make_float4(0.f, 0.f, 0.f, 0.f) : fma4(o.alpha, ld4(N.d, s), ld4(N.x, s)));
             }
         }
     if (threadIdx.x == 0) {
         if (blockIdx.x == 0) {
-            cg->rr      = f3_double(M.cg.rr_next) / double(scale);
-            cg->rr_prev = f3_double(M.cg.rr) / double(scale);
-            cg->pq      = f3_double(M.cg.pq) / double(scale);
-            cg->iter    = M.cg.it;
-            cg->tick    = tag;
+            if (started) {
+                cg->rr      = f3_double(M.cg.rr_next) / double(scale);
+                cg->rr_prev = f3_double(M.cg.rr) / double(scale);
+                cg->pq      = f3_double(M.cg.pq) / double(scale);
+                cg->iter    = M.cg.it;
+                if (o.code != kFailed) cg->done = int(o.code);
+            }
+            cg->tick = tag;
             if (phases) *phases = spent;
         }
         if (o.code == kFailed) atomicExch(&cg->failed, 1);
-        else if (blockIdx.x == 0) cg->done = int(o.code);
     }
 }
 
@@ -464,13 +592,22 @@ template<int DIM> __device__ __forceinline__ bool few_bricks(int nb, int blocks)
 template<int DIM>
 __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     k_cg_solve(Lattice L, const int * __restrict__ blist, const int * __restrict__ bcount,
-               const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, CgState * cg, ulonglong2 * slots,
-               unsigned * flags, CgPhases * phases) {
+               const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, CgState * cg, CgStart from,
+               ulonglong2 * slots, unsigned * flags, CgPhases * phases) {
     using B = WarpBrick<DIM>;
     constexpr int Q = B::G::BN / 4;
     __shared__ MeetSmem<B::WARPS> M;
     const int nb   = *bcount;
-    const int done = cg->done;
+    const int done = from.own ? 0 : cg->done;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        M.nv        = *from.nv;
+        cg->nv      = M.nv;
+        cg->nbricks = nb;
+        if (from.own && nb == 0) {
+            CgScalars none;
+            decide_start(cg, none, 0.0, 0.0, 0, from);
+        }
+    }
     if (done) {
         // no solve: a zero right-hand side (4) or a start that is not a number (3) leaves x = 0
         if (done >= 3)
@@ -482,8 +619,8 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     const int P = min(int(gridDim.x), nb);
     if (int(blockIdx.x) >= P) return;
     if (few_bricks<DIM>(nb, gridDim.x))
-        solve<DIM, B::WMAX>(L, blist, nb, P, bflag, N, S, cg, slots, flags, phases, M);
-    else solve<DIM, B::WMIN>(L, blist, nb, P, bflag, N, S, cg, slots, flags, phases, M);
+        solve<DIM, B::WMAX>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, M);
+    else solve<DIM, B::WMIN>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, M);
 }
 
 // Row-stencil passes outside the iteration, the bricks strided over the warps of a
@@ -661,7 +798,8 @@ void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeAr
 }
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases, cudaStream_t st) {
+                    const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases,
+                    cudaStream_t st) {
     using W = WarpBrick<DIM>;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim          = blocks;
@@ -674,7 +812,7 @@ int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays &
     cfg.attrs    = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_cg_solve<DIM>, L, (const int *) B.list, (const int *) B.count,
-                              (const unsigned char *) B.flag, N, S, cg, slots, flags, phases) == cudaSuccess
+                              (const unsigned char *) B.flag, N, S, cg, from, slots, flags, phases) == cudaSuccess
                ? 0
                : -1;
 }
@@ -690,7 +828,8 @@ int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays &
                                          const StencilD &, unsigned int *, unsigned long long *, int, int,             \
                                          cudaStream_t);                                                                \
     template int launch_cg_solve<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,         \
-                                    CgState *, ulonglong2 *, unsigned *, int, CgPhases *, cudaStream_t);
+                                    CgState *, const CgStart &, ulonglong2 *, unsigned *, int, CgPhases *,             \
+                                    cudaStream_t);
 SWC_INST(2)
 SWC_INST(3)
 #undef SWC_INST

@@ -37,8 +37,6 @@ constexpr int kPhases = 8;
 struct HostCg {
     CgState st;
     double  res2[2];  // |b - A x|^2, |b|^2 of the true residual
-    int     nv;
-    int     nbricks;
     int     mlp_err;
 };
 
@@ -327,18 +325,13 @@ template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features =
 }
 
 // Queues the CG solve from the warm start in N.x (with `started`, from the start state
-// that the caller queued) and the copies of its outcome to the host.
+// that the caller queued).
 template<int DIM> int queue_cg(swc_ctx * c, bool started) {
-    if (!started)
-        launch_cg_init<DIM>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->opts.tolerance, c->opts.max_iterations,
-                            c->B.seg_off + c->B.nseg, c->cgrid, c->grid, c->stream);
-    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, c->slots, c->uflags, c->cgrid, nullptr, c->stream)) {
+    const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg};
+    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, nullptr, c->stream)) {
         c->err = std::string("CG solve: ") + cudaGetErrorString(cudaGetLastError());
         return SWC_CUDA_ERROR;
     }
-    CK(cudaMemcpyAsync(&c->hcg->st, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&c->hcg->nv, c->B.seg_off + c->B.nseg, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&c->hcg->nbricks, c->B.count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     if (c->opts.compute_true_residual) {
         launch_true_residual<DIM>(c->L, c->B, c->N, c->S, c->cg, c->partials, c->res2, c->rgrid, c->stream);
         CK(cudaMemcpyAsync(c->hcg->res2, c->res2, sizeof(c->hcg->res2), cudaMemcpyDeviceToHost, c->stream));
@@ -355,10 +348,11 @@ int cg_outcome(swc_ctx * c, swc_stats * st) {
     if (h.failed) {
         c->err = "CG solve: the blocks of the resident kernel did not meet in time";
         status = SWC_CUDA_ERROR;
+        cudaMemsetAsync(&c->cg->failed, 0, sizeof(int), c->stream);
     }
     if (st) {
-        st->n_virtual            = c->hcg->nv;
-        st->active_bricks        = c->hcg->nbricks;
+        st->n_virtual            = h.nv;
+        st->active_bricks        = h.nbricks;
         st->cg_iterations        = h.iter;
         st->rhs_norm             = std::sqrt(h.bb);
         st->rel_residual         = h.bb > 0 ? std::sqrt(h.rr / h.bb) : 0.0;
@@ -492,6 +486,8 @@ template<int DIM> int queue_projection(swc_ctx * c, Projection & pr) {
         if ((rc = export_prefix<DIM>(c))) return rc;
     } else c->pcomp_stale = true;
     mark(c, 8);
+    // (not between the solve and the gradient: three copies there cost 17 us a step)
+    CK(cudaMemcpyAsync(&c->hcg->st, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost, c->stream));
     return SWC_OK;
 }
 
@@ -1366,13 +1362,12 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
         CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
         for (int k = 0; k < 2; k++) {  // warm, then timed
-            auto go = [&](auto init, auto run) {
-                init(c->L, c->B, c->N, c->S, c->cg, c->partials, 0.0, reps, c->B.seg_off + c->B.nseg, c->cgrid, c->grid,
-                     c->stream);
-                run(c->L, c->B, c->N, c->S, c->cg, c->slots, c->uflags, c->cgrid, c->phases, c->stream);
+            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg};
+            auto go = [&](auto run) {
+                run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->phases, c->stream);
             };
-            if (c->dim == 3) go(launch_cg_init<3>, launch_cg_solve<3>);
-            else go(launch_cg_init<2>, launch_cg_solve<2>);
+            if (c->dim == 3) go(launch_cg_solve<3>);
+            else go(launch_cg_solve<2>);
             CK(cudaStreamSynchronize(c->stream));
         }
         CgPhases ph{};

@@ -529,7 +529,18 @@ struct CgState {
     double sums[4];    // residual sums of the CG start: |r|^2, |b|^2 (prediction / only start), |r|^2, |b|^2 (base)
     unsigned int ticket[4];
     unsigned int tick;  // meetings of the solves so far: the tags of the next solve's follow
-    int    failed;      // a block of the solve waited in vain
+    int    failed;      // a block of the solve waited in vain (cleared by the host)
+    int    nv;          // active nodes and bricks of the solve
+    int    nbricks;
+};
+
+// Where a solve starts: with `own`, from x, with the residual and the start state made in
+// the solve; else from the state that k_cg_start left.
+struct CgStart {
+    double      tolerance;
+    int         max_iterations;  // < 0: twice the active nodes
+    int         own;
+    const int * nv;              // device: active nodes
 };
 
 // Times of the solve's phases, summed over the iterations (ns, as the first warp of

@@ -167,15 +167,12 @@ void launch_compact_export(const Lattice & L, const BrickArrays & B, const NodeA
 template<int DIM> int cg_solve_prepare();
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases, cudaStream_t st);
+                    const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases,
+                    cudaStream_t st);
 template<int DIM>
 void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                           const float * x, float * r, float * d, double * sums, CgState * cg, double * partials,
                           int blocks, cudaStream_t st);
-template<int DIM>
-void launch_cg_init(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    double * partials, double tol, int max_iterations, const int * nv, int rblocks, int ugrid,
-                    cudaStream_t st);
 // Residual r = b - A x of one candidate CG start (r, and d when non-null;
 // |r|^2, |b|^2 into sums[0..1]).
 template<int DIM>

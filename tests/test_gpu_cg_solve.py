@@ -80,3 +80,22 @@ def test_residual_that_vanishes_in_one_step(swc_mod):
     assert 0 < st["rel_residual"] < 2e-6 + 2.0**-22
     assert abs(st["true_rel_residual"] - st["rel_residual"]) < 2.0**-22
     liq.close()
+
+
+@pytest.mark.parametrize("build,n", [(bricks_2d, 9), (bricks_2d, 121), (bricks_3d, 9), (bricks_3d, 60)])
+@pytest.mark.parametrize("tol,cap,status", [(2.0, -1, 0), (1e-6, 0, 1)])
+def test_solves_that_end_at_their_start(swc_mod, build, n, tol, cap, status):
+    """A start within the tolerance, and a cap of no iterations: x stays the start (0), whose
+    residual is b itself, so both norms are sums of the same terms."""
+    s = build(n).rounded_to_float32()
+    liq = swc_mod.DualParticleSphLiquid(s, warm_start="zero", tolerance=tol, max_iterations=cap)
+    liq.initialize()
+    st = liq.advance(s.dt)
+    assert st["status"] == status and st["cg_iterations"] == 0
+    assert st["rhs_norm"] == pytest.approx(np.linalg.norm(liq.virtual()["div"]), rel=1e-6)
+    assert st["rel_residual"] == 1.0 and st["initial_rel_residual"] == 1.0
+    assert not np.any(liq.virtual()["p"])
+    # and the next one runs as usual
+    st = liq.advance(s.dt)
+    assert st["n_virtual"] == liq.virtual()["node"].shape[0]
+    liq.close()
