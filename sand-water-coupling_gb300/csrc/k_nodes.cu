@@ -843,7 +843,6 @@ void launch_node_gather(const Lattice & L, const Phys & P, const BrickArrays & B
 template<int DIM>
 void launch_segments(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int * tiles, int grid,
                      cudaStream_t st) {
-    cudaMemsetAsync(B.seg, 0, sizeof(int) * B.nseg, st);
     launch_pdl(k_segment_count<DIM>, grid, kNT, 0, st, L, B.list, B.count, N.flag, B.seg);
     launch_scan(B.seg, B.nseg, B.seg_off, tiles, st);
 }

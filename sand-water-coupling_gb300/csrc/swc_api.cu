@@ -185,6 +185,7 @@ int alloc_sort(swc_ctx * c, SortScratch & S, long long n, bool aux) {
     if ((rc = dalloc(c, &S.rank, n))) return rc;
     if ((rc = dalloc(c, &S.perm, n))) return rc;
     if ((rc = dalloc(c, &S.count, c->L.ncells))) return rc;
+    CK(cudaMemsetAsync(S.count, 0, sizeof(int) * c->L.ncells, c->stream));
     if ((rc = dalloc(c, &S.tiles, scan_tile_count(c->L.ncells + 1) + 2))) return rc;
     if ((rc = dalloc(c, &S.pos2, n))) return rc;
     if ((rc = dalloc(c, &S.vel2, n))) return rc;
@@ -782,6 +783,7 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
     cudaMemsetAsync(c->B.flag, 0, L.nbricks, c->stream);
     cudaMemsetAsync(c->B.flag_prev, 0, L.nbricks, c->stream);
     cudaMemsetAsync(c->N.flag, 0, slots, c->stream);
+    cudaMemsetAsync(c->B.seg, 0, sizeof(int) * c->B.nseg, c->stream);
     cudaMemsetAsync(c->N.x, 0, slots * sizeof(float), c->stream);
     cudaMemsetAsync(c->nv_prev, 0, sizeof(int), c->stream);
     cudaMemsetAsync(c->bcellStart, 0, sizeof(int) * (L.ncells + 1), c->stream);

@@ -6,7 +6,7 @@
 
 namespace swc {
 
-// Scratch for the counting sort of one particle set.
+// Scratch for the counting sort of one particle set (count zeroed once at allocation).
 struct SortScratch {
     int *    key = nullptr, *rank = nullptr, *perm = nullptr, *count = nullptr, *tiles = nullptr;
     float4 * pos2 = nullptr, *vel2 = nullptr, *aux2 = nullptr;
@@ -52,7 +52,7 @@ struct BrickArrays {
     unsigned char * flag_m3   = nullptr;
     int *           list      = nullptr;  // active brick ids, ascending
     int *           count     = nullptr;  // device: number of active bricks
-    int *           seg       = nullptr;  // per (row, brick column) active-node counts
+    int *           seg       = nullptr;  // per (row, brick column) active-node counts (zero between the scans)
     int *           seg_off   = nullptr;  // exclusive scan of seg (+ total at the end)
     long long       nseg      = 0;
 };
@@ -67,7 +67,8 @@ void launch_export_scalar(const float * a, int stride, int comp, const int * id,
 void launch_max_speed2(const float4 * vel, long long n, int dim, unsigned long long * out, cudaStream_t st);
 void launch_export_ratio(const float * a, int stride, int comp, float num, const int * id, long long n, double * out,
                          cudaStream_t st);
-void launch_scan(const int * in, long long n, int * out, int * tile_buf, cudaStream_t st,
+// (in, zeroed once at allocation, is left zero)
+void launch_scan(int * in, long long n, int * out, int * tile_buf, cudaStream_t st,
                  const Lattice * Ld = nullptr);
 long long scan_tile_count(long long n);
 void launch_set_volume(float4 * pos, const float * rho, long long n, float mass, cudaStream_t st);

@@ -175,11 +175,61 @@ __device__ __forceinline__ unsigned f2ord(float f) {
 }
 __device__ __forceinline__ float ord2f(unsigned u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u); }
 
+// The step's cell lattice over the box (clipped to the home box), cells of 2r doubled
+// until the lattice fits `cap` cells, two cells of margin, by a warp (an axis a lane); then
+// the box accumulators are reset for the next step.
+struct SandBox {
+    float3    home_lo, home_hi;
+    float     cell0;
+    long long cap;
+};
+template<int DIM> __device__ void sand_lattice(unsigned * box, const SandBox & H, Lattice * Ld) {
+    const int a = threadIdx.x & 31;
+    float lo = 0.f, hi = 0.f;
+    if (a < DIM) {
+        const float hl = a == 0 ? H.home_lo.x : a == 1 ? H.home_lo.y : H.home_lo.z;
+        const float hh = a == 0 ? H.home_hi.x : a == 1 ? H.home_hi.y : H.home_hi.z;
+        const unsigned bl = __ldcg(box + a), bh = __ldcg(box + 3 + a);
+        if (bl != 0xffffffffu) {
+            lo = fmaxf(ord2f(bl), hl);
+            hi = fminf(ord2f(bh), hh);
+            if (lo > hi) lo = hi = fminf(fmaxf(lo, hl), hh);
+        }
+        box[a]     = 0xffffffffu;
+        box[3 + a] = 0u;
+    }
+    // the cell grows by at least 2x (or the factor the cell count asks for) until it fits
+    double cell = H.cell0, dims = 1, total = 1;
+    for (int it = 0; it < 64; it++) {
+        dims  = a < DIM ? floor((double(hi) - double(lo)) / cell) + 5 : 1;
+        total = __shfl_sync(0xffffffffu, dims, 0);
+#pragma unroll
+        for (int k = 1; k < DIM; k++) total *= __shfl_sync(0xffffffffu, dims, k);
+        if (total <= double(H.cap)) break;
+        cell *= fmax(2.0, 1.01 * pow(total / double(H.cap), 1.0 / DIM));
+    }
+    cell = fmin(cell, 1e37);
+    const float origin = float(lo - 2 * cell);
+    const int count    = int(dims);
+    Lattice L{};
+    L.ox     = __shfl_sync(0xffffffffu, origin, 0);
+    L.oy     = __shfl_sync(0xffffffffu, origin, 1);
+    L.oz     = DIM == 3 ? __shfl_sync(0xffffffffu, origin, 2) : 0.f;
+    L.dx     = float(cell);
+    L.inv_dx = float(1 / cell);
+    L.nx     = __shfl_sync(0xffffffffu, count, 0);
+    L.ny     = __shfl_sync(0xffffffffu, count, 1);
+    L.nz     = DIM == 3 ? __shfl_sync(0xffffffffu, count, 2) : 1;
+    L.bnx = L.bny = L.bnz = L.nbricks = 1;
+    L.ncells = (long long) L.nx * L.ny * L.nz;
+    if (a == 0) *Ld = L;
+}
+
 // Box of the positions after this step's move, x + v dt (FP32; the lattice pads
 // it and clamps whatever falls outside): box[0..2] minima, box[3..5] maxima.
 template<int DIM>
 __global__ void k_sand_bbox(const float4 * __restrict__ pos, const float4 * __restrict__ vel, long long n, float dt,
-                            unsigned * __restrict__ box) {
+                            unsigned * __restrict__ box, SandBox H, Lattice * __restrict__ Ld) {
     pdl_wait_and_release();
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
@@ -217,50 +267,20 @@ __global__ void k_sand_bbox(const float4 * __restrict__ pos, const float4 * __re
             atomicMax(box + 3 + a, f2ord(h));
         }
     }
-}
-
-// One thread: the step's cell lattice over the box (clipped to the home box),
-// cells of 2r doubled until the lattice fits `cap` cells, two cells of margin;
-// then the box accumulators are reset for the next step.
-__global__ void k_sand_lattice(unsigned * __restrict__ box, float3 home_lo, float3 home_hi, float cell0, long long cap,
-                               int dim, Lattice * __restrict__ Ld) {
-    pdl_wait_and_release();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const float hl[3] = {home_lo.x, home_lo.y, home_lo.z}, hh[3] = {home_hi.x, home_hi.y, home_hi.z};
-    float lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
-    for (int a = 0; a < dim; a++) {
-        if (box[a] != 0xffffffffu) {
-            lo[a] = fmaxf(ord2f(box[a]), hl[a]);
-            hi[a] = fminf(ord2f(box[3 + a]), hh[a]);
-            if (lo[a] > hi[a]) lo[a] = hi[a] = fminf(fmaxf(lo[a], hl[a]), hh[a]);
+    // the last block makes the lattice (box[6] counts the blocks; a launch of its own for
+    // one thread took 4.5 us)
+    __shared__ bool last;
+    if (threadIdx.x < 32) {
+        __threadfence();
+        __syncwarp();
+        if (threadIdx.x == 0) last = atomicAdd(box + 6, 1u) == gridDim.x - 1;
+        __syncwarp();
+        if (last) {
+            __threadfence();
+            if (threadIdx.x == 0) box[6] = 0u;
+            sand_lattice<DIM>(box, H, Ld);
         }
-        box[a]     = 0xffffffffu;
-        box[3 + a] = 0u;
     }
-    // the cell grows by at least 2x (or the factor the cell count asks for) until it fits
-    double cell = cell0, dims[3] = {1, 1, 1};
-    for (int it = 0; it < 64; it++) {
-        double total = 1;
-        for (int a = 0; a < dim; a++) {
-            dims[a] = floor((double(hi[a]) - double(lo[a])) / cell) + 5;
-            total *= dims[a];
-        }
-        if (total <= double(cap)) break;
-        cell *= fmax(2.0, 1.01 * pow(total / double(cap), 1.0 / dim));
-    }
-    cell = fmin(cell, 1e37);
-    Lattice L{};
-    L.ox     = float(lo[0] - 2 * cell);
-    L.oy     = float(lo[1] - 2 * cell);
-    L.oz     = dim == 3 ? float(lo[2] - 2 * cell) : 0.f;
-    L.dx     = float(cell);
-    L.inv_dx = float(1 / cell);
-    L.nx     = int(dims[0]);
-    L.ny     = int(dims[1]);
-    L.nz     = dim == 3 ? int(dims[2]) : 1;
-    L.bnx = L.bny = L.bnz = L.nbricks = 1;
-    L.ncells = (long long) L.nx * L.ny * L.nz;
-    *Ld      = L;
 }
 
 // The contact pass.  d = x_j - x_i, w = v_j - v_i as in DEMParticle::getForce
@@ -590,6 +610,7 @@ int ensure_sand_cells(swc_sand * s) {
     if ((rc = salloc(s, &s->cellStart, cap + 1)) || (rc = salloc(s, &s->S.count, cap)) ||
         (rc = salloc(s, &s->S.tiles, scan_tile_count(cap + 1) + 2)))
         return rc;
+    SK(cudaMemsetAsync(s->S.count, 0, sizeof(int) * cap, s->stream));
     return SWC_OK;
 }
 
@@ -597,11 +618,10 @@ int ensure_sand_cells(swc_sand * s) {
 // then the counting sort (with the float-float move when dt != 0).
 template<int DIM> void bin_sand(swc_sand * s, float dth, float dtl) {
     cudaStream_t st = s->stream;
-    if (s->n > 0)
-        launch_pdl(k_sand_bbox<DIM>, sand_grid(s->n, 256, 152 * 8), 256, 0, st, (const float4 *) s->pos,
-                   (const float4 *) s->vel, s->n, dth, s->dbox);
-    launch_pdl(k_sand_lattice, 1, 32, 0, st, s->dbox, make_float3(s->home_lo[0], s->home_lo[1], s->home_lo[2]),
-               make_float3(s->home_hi[0], s->home_hi[1], s->home_hi[2]), s->P.R, s->Lcap.ncells, s->dim, s->dL);
+    const SandBox home{make_float3(s->home_lo[0], s->home_lo[1], s->home_lo[2]),
+                       make_float3(s->home_hi[0], s->home_hi[1], s->home_hi[2]), s->P.R, s->Lcap.ncells};
+    launch_pdl(k_sand_bbox<DIM>, sand_grid(s->n, 256, 152 * 8), 256, 0, st, (const float4 *) s->pos,
+               (const float4 *) s->vel, s->n, dth, s->dbox, home, s->dL);
     launch_bin<DIM>(s->Lcap, s->n, s->pos, s->vel, s->plo, s->id, s->S, s->cellStart, dth, st, dtl, true, s->dL);
     s->sorted = true;
 }
@@ -637,6 +657,7 @@ template<int DIM> int do_initialize(swc_sand * s) {
         (rc = salloc(s, &B.id2, s->nb)) || (rc = salloc(s, &B.count, Lb.ncells)) ||
         (rc = salloc(s, &B.tiles, scan_tile_count(Lb.ncells + 1) + 2)))
         return rc;
+    SK(cudaMemsetAsync(B.count, 0, sizeof(int) * Lb.ncells, st));
     launch_bin<DIM>(Lb, s->nb, s->bpos, s->bnrm, s->blo, s->bid, B, s->bcellStart, 0.f, st);
     SK(cudaGetLastError());
     SK(cudaStreamSynchronize(st));
@@ -666,7 +687,7 @@ template<int DIM> int do_initialize(swc_sand * s) {
     // sand: cell arrays, box accumulators (min = all ones, max = 0), first binning
     if ((rc = ensure_sand_cells(s))) return rc;
     SK(cudaMemsetAsync(s->dbox, 0xff, 3 * sizeof(unsigned), st));
-    SK(cudaMemsetAsync(s->dbox + 3, 0, 3 * sizeof(unsigned), st));
+    SK(cudaMemsetAsync(s->dbox + 3, 0, 4 * sizeof(unsigned), st));
     bin_sand<DIM>(s, 0.f, 0.f);
     SK(cudaGetLastError());
     SK(cudaStreamSynchronize(st));
@@ -730,7 +751,7 @@ int swc_sand_create(const swc_sand_params * p, swc_sand ** out) {
     }
     s->own_stream = true;
     int rc;
-    if ((rc = salloc(s, &s->vbits, 1)) || (rc = salloc(s, &s->dL, 1)) || (rc = salloc(s, &s->dbox, 6))) {
+    if ((rc = salloc(s, &s->vbits, 1)) || (rc = salloc(s, &s->dL, 1)) || (rc = salloc(s, &s->dbox, 7))) {
         swc_sand_destroy(s);
         return rc;
     }
