@@ -13,43 +13,46 @@ namespace swc {
 
 
 // ---------------------------------------------------------------------------
-// Active-brick list (single CTA, ascending brick id).
+// Lists of the flagged bricks, ascending (a block each; 16 flags a thread at a time).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_brick_list(const unsigned char * __restrict__ bflag, int nbricks,
-                                                     int * __restrict__ list, int * __restrict__ count) {
+__global__ void __launch_bounds__(1024) k_brick_lists(BrickList a, BrickList b, int nbricks) {
     pdl_wait_and_release();
+    const BrickList l = blockIdx.x == 0 ? a : b;
     __shared__ int sm[32];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nbricks; base += 1024) {
-        const int i = base + threadIdx.x;
-        const int v = (i < nbricks && bflag[i]) ? 1 : 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < nbricks; base += 16 * 1024) {
+        const int i0 = base + 16 * threadIdx.x;
+        unsigned f[4] = {0, 0, 0, 0};  // 16 flags of 0 or 1
+        if (i0 + 16 <= nbricks) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(l.flag + i0);
+            f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+        } else
+            for (int k = 0; k < 16 && i0 + k < nbricks; k++) f[k / 4] |= unsigned(l.flag[i0 + k]) << (8 * (k % 4));
+        const int v = __popc(f[0]) + __popc(f[1]) + __popc(f[2]) + __popc(f[3]);
         int x       = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((threadIdx.x & 31) >= o) x += y;
+            if (lane >= o) x += y;
         }
-        if ((threadIdx.x & 31) == 31) sm[threadIdx.x >> 5] = x;
+        if (lane == 31) sm[warp] = x;
         __syncthreads();
-        if (threadIdx.x < 32) {
-            int w = sm[threadIdx.x];
+        // every warp scans the warps' sums for itself
+        int w = sm[lane];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, o);
-                if (threadIdx.x >= o) w += y;
-            }
-            sm[threadIdx.x] = w;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
         }
-        __syncthreads();
-        const int incl = x + ((threadIdx.x >> 5) ? sm[(threadIdx.x >> 5) - 1] : 0) + carry;
-        if (v) list[incl - 1] = i;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = incl;
+        int at = carry + x - v + (warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0);
+        carry += __shfl_sync(0xffffffffu, w, 31);
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            if (f[k / 4] >> (8 * (k % 4)) & 1u) l.list[at++] = i0 + k;
         __syncthreads();
     }
-    if (threadIdx.x == 0) *count = carry;
+    if (threadIdx.x == 0) *l.count = carry;
 }
 
 // Sums of two x-adjacent nodes, packed as FP32x2 (.x: node n, .y: node n + 1).
@@ -143,6 +146,7 @@ template<int S> __device__ __forceinline__ float2 lanes_sum(float2 v) {
 template<int DIM, bool FAST_H, bool FEAT, int S>
 __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const int * __restrict__ blist,
                                                     const int * __restrict__ bcount, NodeArrays N,
+                                                    int * __restrict__ seg,
                                                     const float4 * __restrict__ pos, const float4 * __restrict__ vel,
                                                     const int * __restrict__ cellStart,
                                                     const float4 * __restrict__ bpos,
@@ -265,10 +269,10 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
                 a.ux = lanes_sum<S>(a.ux), a.uy = lanes_sum<S>(a.uy), a.uz = lanes_sum<S>(a.uz);
                 a.bw = lanes_sum<S>(a.bw), a.dvg = lanes_sum<S>(a.dvg);
                 a.gx = lanes_sum<S>(a.gx), a.gy = lanes_sum<S>(a.gy), a.gz = lanes_sum<S>(a.gz);
-                if (part != 0) continue;  // to the next item
             }
 #pragma unroll
             for (int n = 0; n < NX; n++) {
+                if (S > 1 && part != 0) break;
                 const int x       = x0 + n;
                 const long long s = s0 + n;
                 if (!row_in || x >= L.nx) {
@@ -315,37 +319,23 @@ __global__ void __launch_bounds__(128, 5) k_node_gather(Lattice L, Phys P, const
                 if (FEAT) N.nreal[s] = (unsigned short) min(int(pick(a.cnt)), 65535);
                 if (N.vbar) N.vbar[s] = make_float4(vbx, vby, vbz, 0.f);
             }
+            // the row's active nodes, for the compaction: its flags, written by this warp, read
+            // back.  (From the slot alone: with anything more held through the walk the spills
+            // took the learned start's gather from 436 to 492 us at 2.25M nodes.)
+            __syncwarp();
+            if (threadIdx.x % (XS * S) == 0) {
+                const int row  = int(s0 % G::BN) / G::BX;
+                const int3 at  = brick_coords(L, int(s0 / G::BN));
+                const int sy   = at.y * G::BY + row % G::BY, sz = at.z * G::BZ + row / G::BY;
+                const uint2 * f = reinterpret_cast<const uint2 *>(N.flag + s0);
+                int count = 0;
+#pragma unroll
+                for (int k = 0; k < G::BX / 8; k++) count += __popc(f[k].x) + __popc(f[k].y);
+                if (sy < L.ny && (DIM == 2 || sz < L.nz)) seg[((long long) sz * L.ny + sy) * L.bnx + at.x] = count;
+            }
         }
     }
     queue_finish(queue);
-}
-
-// ---------------------------------------------------------------------------
-// Reference-order (x-fastest over the whole node grid, Grid.cpp:231-244)
-// compaction: per (row, brick column) segment counts, scanned.
-// ---------------------------------------------------------------------------
-template<int DIM>
-__global__ void __launch_bounds__(kNT) k_segment_count(Lattice L, const int * __restrict__ blist,
-                                                       const int * __restrict__ bcount,
-                                                       const unsigned char * __restrict__ flag, int * __restrict__ seg) {
-    pdl_wait_and_release();
-    using G      = BrickGeom<DIM>;
-    const int nb = *bcount;
-    constexpr int ROWS = G::BY * G::BZ;
-    for (int bi = blockIdx.x; bi < nb; bi += gridDim.x) {
-        const int b   = blist[bi];
-        const int3 bc = brick_coords(L, b);
-        for (int rrow = threadIdx.x; rrow < ROWS; rrow += kNT) {
-            const int ly = rrow % G::BY, lz = rrow / G::BY;
-            const int y = bc.y * G::BY + ly, z = bc.z * G::BZ + lz;
-            if (y >= L.ny || (DIM == 3 && z >= L.nz)) continue;
-            const unsigned char * f = flag + (long long) b * G::BN + G::BX * rrow;
-            int c = 0;
-#pragma unroll
-            for (int k = 0; k < G::BX; k++) c += f[k];
-            seg[((long long) z * L.ny + y) * L.bnx + bc.x] = c;
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -808,8 +798,8 @@ template<int DIM> int node_gather_blocks_per_sm() {
                            std::min(blocks(k_node_gather<DIM, false, true, 1>), blocks(k_node_gather<DIM, false, false, 1>)));
     return n > 0 ? n : 1;
 }
-void launch_brick_list(const unsigned char * bflag, int nbricks, int * list, int * count, cudaStream_t st) {
-    launch_pdl(k_brick_list, 1, 1024, 0, st, bflag, nbricks, list, count);
+void launch_brick_lists(const BrickList & a, const BrickList & b, int nbricks, cudaStream_t st) {
+    launch_pdl(k_brick_lists, 2, 1024, 0, st, a, b, nbricks);
 }
 
 template<int DIM>
@@ -822,8 +812,8 @@ void launch_node_gather(const Lattice & L, const Phys & P, const BrickArrays & B
     const bool fast = double(P.H) >= 2.0 * double(P.h) * (1.0 - 1e-6), feat = N.nreal != nullptr;
     auto go = [&](auto kernel, int s) {
         const long long items = (long long) L.nbricks * (DIM == 3 ? 2 : 1) * s;
-        launch_pdl(kernel, int(std::min<long long>(grid, items)), 128, 0, st, L, P, B.list, B.count, N, pos, vel, cellStart,
-                   bpos, bvel, bcellStart, bnear, bcell, queue);
+        launch_pdl(kernel, int(std::min<long long>(grid, items)), 128, 0, st, L, P, B.list, B.count, N, B.seg, pos, vel,
+                   cellStart, bpos, bvel, bcellStart, bnear, bcell, queue);
     };
     auto lanes = [&](auto s) {
         constexpr int S = decltype(s)::value;
@@ -839,14 +829,6 @@ void launch_node_gather(const Lattice & L, const Phys & P, const BrickArrays & B
     else if (S == 2) lanes(std::integral_constant<int, 2>{});
     else lanes(std::integral_constant<int, 1>{});
 }
-
-template<int DIM>
-void launch_segments(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int * tiles, int grid,
-                     cudaStream_t st) {
-    launch_pdl(k_segment_count<DIM>, grid, kNT, 0, st, L, B.list, B.count, N.flag, B.seg);
-    launch_scan(B.seg, B.nseg, B.seg_off, tiles, st);
-}
-
 
 template<int DIM>
 void launch_warm_start(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int mode, const float * pcomp,
@@ -888,8 +870,6 @@ void launch_compact_import(const Lattice & L, const BrickArrays & B, const NodeA
                                               int *, cudaStream_t);                                                    \
     template int pressure_gradient_blocks_per_sm<D>();                                                                 \
     template int node_gather_blocks_per_sm<D>();                                                                       \
-    template void launch_segments<D>(const Lattice &, const BrickArrays &, const NodeArrays &, int *, int,             \
-                                     cudaStream_t);                                                                    \
     template void launch_warm_start<D>(const Lattice &, const BrickArrays &, const NodeArrays &, int, const float *,   \
                                        const int *, const float *, int, cudaStream_t, int);                            \
     template void launch_compact_export<D>(const Lattice &, const BrickArrays &, const NodeArrays &, float *,          \

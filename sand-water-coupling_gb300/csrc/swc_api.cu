@@ -315,13 +315,12 @@ inline void mark(swc_ctx * c, int k) {
 // real-neighbour counts of the gather); without them the gather skips the count.
 template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features = true) {
     launch_mark_bricks<DIM>(c->cellStart, c->n, c->L, c->P, c->B.flag, c->pflag, c->stream);
-    launch_brick_list(c->B.flag, c->L.nbricks, c->B.list, c->B.count, c->stream);
-    launch_brick_list(c->pflag, c->L.nbricks, c->plist, c->pcount, c->stream);
+    launch_brick_lists({c->B.flag, c->B.list, c->B.count}, {c->pflag, c->plist, c->pcount}, c->L.nbricks, c->stream);
     NodeArrays N = c->N;
     if (!features) N.nreal = nullptr;
     launch_node_gather<DIM>(c->L, c->P, c->B, N, c->pos, c->vel, c->cellStart, c->bpos, c->bvel, c->bcellStart,
                             c->bnear, c->bcell, c->n, c->ggrid, c->queues, c->stream);
-    launch_segments<DIM>(c->L, c->B, c->N, c->scan_tiles, c->grid, c->stream);
+    launch_scan(c->B.seg, c->B.nseg, c->B.seg_off, c->scan_tiles, c->stream);
     if (with_ahat) launch_ahat<DIM>(c->L, c->P, c->B, c->N, c->S, c->cgrid, c->stream);
 }
 
@@ -536,18 +535,17 @@ int finish_projection(swc_ctx * c, swc_stats * st, const Projection & pr) {
 // ends the extrapolation history.
 void save_prev_flags(swc_ctx * c, bool move) {
     using namespace swc;
-    const size_t bn = c->dim == 3 ? BrickGeom<3>::BN : BrickGeom<2>::BN;
     c->extrap_shifted = false;
     if (move && history_on(c)) {
-        // rotate the history buffers (no kernel reads them inside the captured CG graphs)
         std::swap(c->N.flag_m3, c->N.flag_m2);
         std::swap(c->N.flag_m2, c->N.flag_prev);
         std::swap(c->B.flag_m3, c->B.flag_m2);
         std::swap(c->B.flag_m2, c->B.flag_prev);
         c->extrap_shifted = true;
     }
-    cudaMemcpyAsync(c->N.flag_prev, c->N.flag, size_t(c->L.nbricks) * bn, cudaMemcpyDeviceToDevice, c->stream);
-    cudaMemcpyAsync(c->B.flag_prev, c->B.flag, size_t(c->L.nbricks), cudaMemcpyDeviceToDevice, c->stream);
+    // the step's generation writes every brick's flag and, in the flagged bricks, every node's
+    std::swap(c->N.flag_prev, c->N.flag);
+    std::swap(c->B.flag_prev, c->B.flag);
 }
 
 template<int DIM> int do_advance(swc_ctx * c, double dt, swc_stats * st, bool move) {
@@ -1389,6 +1387,8 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         *mean_ms = ms / reps;
     }
     CK(cudaMemcpy(c->cg, &saved, sizeof(CgState), cudaMemcpyHostToDevice));
+    // (the gather alone, without the scan that clears its rows' counts)
+    if (which == 2) CK(cudaMemset(c->B.seg, 0, sizeof(int) * c->B.nseg));
     if (x_save) {
         cudaMemcpy(c->N.x, x_save, sizeof(float) * slots, cudaMemcpyDeviceToDevice);
         cudaMemcpy(c->N.r, x_save + slots, sizeof(float) * slots, cudaMemcpyDeviceToDevice);

@@ -52,7 +52,7 @@ struct BrickArrays {
     unsigned char * flag_m3   = nullptr;
     int *           list      = nullptr;  // active brick ids, ascending
     int *           count     = nullptr;  // device: number of active bricks
-    int *           seg       = nullptr;  // per (row, brick column) active-node counts (zero between the scans)
+    int *           seg       = nullptr;  // per (row, brick column) active-node counts: zero but between the gather and their scan
     int *           seg_off   = nullptr;  // exclusive scan of seg (+ total at the end)
     long long       nseg      = 0;
 };
@@ -119,7 +119,12 @@ void launch_debug_neighbors(int which, long long nq, const double * q, const Lat
                             cudaStream_t st);
 
 // ---- k_nodes.cu ----
-void launch_brick_list(const unsigned char * bflag, int nbricks, int * list, int * count, cudaStream_t st);
+struct BrickList {
+    const unsigned char * flag;   // 0 or 1 per brick, 16-byte aligned
+    int *                 list;   // ids of the flagged bricks, ascending
+    int *                 count;  // and their number
+};
+void launch_brick_lists(const BrickList & a, const BrickList & b, int nbricks, cudaStream_t st);
 template<int DIM>
 void launch_node_gather(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N,
                         const float4 * pos, const float4 * vel, const int * cellStart, const float4 * bpos,
@@ -139,9 +144,6 @@ void launch_pressure_gradient(const Lattice & L, const Phys & P, const BrickArra
 // two ints).
 template<int DIM> int node_gather_blocks_per_sm();
 template<int DIM> int pressure_gradient_blocks_per_sm();
-template<int DIM>
-void launch_segments(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int * tiles, int grid,
-                     cudaStream_t st);
 template<int DIM>
 void launch_ahat(const Lattice & L, const Phys & P, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                  int blocks, cudaStream_t st);
