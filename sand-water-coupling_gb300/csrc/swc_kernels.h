@@ -217,25 +217,31 @@ void launch_node_features(const NodeArrays & N, const int * slot_of, const int *
 // (mlp_train_ctas(n)) write their shares into share (mlp_train_share_floats(ctas)
 // floats), a second kernel adds them in order into grad[SWC_MLP_PARAMS] and the
 // mean squared error into *loss (NaN with *err set on a tensor-core timeout).
-// Returns nonzero when a launch failed.
+// Returns nonzero when a launch failed.  With batch.rows the batch is rows first ..
+// first + n - 1 of a pseudo-random permutation of the `rows` dataset rows in feat / target
+// (a Feistel network on 2 x half bits, 2^(2 half) >= rows), which nothing queued writes;
+// with adam.m the second kernel also takes the parameters' Adam step.
+struct MlpBatch {
+    long long rows = 0, first = 0;
+    int       half = 0;
+    uint4     key{0, 0, 0, 0};
+};
+struct MlpAdam {
+    float *m = nullptr, *v = nullptr, *params = nullptr;
+    float lr = 0, b1 = 0, b2 = 0, eps = 0, bc1 = 0, bc2 = 0;
+};
 constexpr int kMlpTrainShare = 128 * 80 + 64 + 2;  // floats of one CTA's share (D, dw3, db3, loss)
 int    mlp_train_ctas(long long n);
 size_t mlp_train_share_floats(int ctas);
 int    launch_mlp_train_grad(long long n, const float * params, const float * norm, const float * feat,
                              const float * target, float * share, int ctas, int * err, float * grad, float * loss,
-                             cudaStream_t st);
-void launch_adam(float * p, const float * g, float * m, float * v, int count, float lr, float b1, float b2, float eps,
-                 float bc1, float bc2, cudaStream_t st);
+                             cudaStream_t st, const MlpBatch & batch = {}, const MlpAdam & adam = {});
 template<int DIM>
 void launch_slot_of(const Lattice & L, const BrickArrays & B, const NodeArrays & N, int * slot_of, int grid,
                     cudaStream_t st);
 void launch_mlp_targets(long long rows_max, const int * nv, const int * slot_of, const float * x, const float * prev,
                         const float * xm1, const float * d2p, const float * ahat, const CgState * cg, float * target,
                         cudaStream_t st);
-// Rows b0 .. b0 + nb - 1 of a pseudo-random permutation of the n rows (a Feistel
-// network on 2 x half bits, 2^(2 half) >= n, keyed by key[4]) into dst / dst_t.
-void launch_gather_shuffled(const float * src, const float * src_t, long long n, long long b0, long long nb, int half,
-                            const unsigned * key, float * dst, float * dst_t, cudaStream_t st);
 // Per-block FP64 sums of ((pred - tgt) * inv_tstd)^2 over n rows into part[blocks].
 void launch_sq_err(const float * pred, const float * tgt, long long n, float inv_tstd, double * part, int blocks,
                    cudaStream_t st);

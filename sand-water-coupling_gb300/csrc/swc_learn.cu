@@ -49,8 +49,10 @@ int forward_batch(swc_trainer * t, const float * feat, long long n, float * out)
     return cudaGetLastError() == cudaSuccess ? SWC_OK : SWC_CUDA_ERROR;
 }
 // loss gradient of one batch (features / targets on the device) into t->grad, t->loss
-int gradient_batch(swc_trainer * t, const float * feat, const float * tgt, long long n) {
-    return launch_mlp_train_grad(n, t->params, t->norm, feat, tgt, t->share, t->ctas, t->err, t->grad, t->loss, t->st)
+int gradient_batch(swc_trainer * t, const float * feat, const float * tgt, long long n, const MlpBatch & batch = {},
+                   const MlpAdam & adam = {}) {
+    return launch_mlp_train_grad(n, t->params, t->norm, feat, tgt, t->share, t->ctas, t->err, t->grad, t->loss, t->st,
+                                 batch, adam)
                ? SWC_CUDA_ERROR
                : SWC_OK;
 }
@@ -160,11 +162,11 @@ int swc_trainer_fit(swc_trainer * t, int32_t epochs, float lr, uint64_t seed, fl
         const unsigned key[4] = {unsigned(k0), unsigned(k0 >> 32), unsigned(k1), unsigned(k1 >> 32)};
         for (long long b0 = 0; b0 < t->n; b0 += t->batch) {
             const long long nb = std::min<long long>(t->batch, t->n - b0);
-            launch_gather_shuffled(t->feat, t->tgt, t->n, b0, nb, half, key, t->bfeat, t->btgt, t->st);
-            if (int rc = gradient_batch(t, t->bfeat, t->btgt, nb)) return rc;
             t->adam_t++;
             const float bc1 = 1.f - std::pow(b1, float(t->adam_t)), bc2 = 1.f - std::pow(b2, float(t->adam_t));
-            launch_adam(t->params, t->grad, t->m, t->v, kP, lr, b1, b2, eps, bc1, bc2, t->st);
+            const MlpBatch batch{t->n, b0, half, make_uint4(key[0], key[1], key[2], key[3])};
+            const MlpAdam adam{t->m, t->v, t->params, lr, b1, b2, eps, bc1, bc2};
+            if (int rc = gradient_batch(t, t->feat, t->tgt, nb, batch, adam)) return rc;
         }
         if (epoch_loss) {
             // loss of the epoch's parameters over the whole dataset, on the device
