@@ -419,11 +419,12 @@ __device__ __forceinline__ void for_each_in_radius2(const Lattice & L, const int
 }
 
 // The same visit for one query point.
-template<int DIM, class F>
+template<int DIM, int S = 1, class F>
 __device__ __forceinline__ void for_each_in_radius(const Lattice & L, const int * __restrict__ cellStart,
-                                                   float qx, float qy, float qz, float R, float R2, F && f) {
+                                                   float qx, float qy, float qz, float R, float R2, F && f,
+                                                   int part = 0) {
     const float3 q = make_float3(qx, qy, qz);
-    for_each_in_radius2<DIM>(L, cellStart, q, q, R, R2, f);
+    for_each_in_radius2<DIM, S>(L, cellStart, q, q, R, R2, f, part);
 }
 
 // Row-parallel form of for_each_in_radius for one query point: the caller's

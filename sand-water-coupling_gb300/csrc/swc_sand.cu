@@ -283,9 +283,54 @@ __global__ void k_sand_bbox(const float4 * __restrict__ pos, const float4 * __re
     }
 }
 
+// Terms of one particle that S lanes find and evaluate together, added in ascending order
+// of the neighbour (the order of the cell rows), so that the sum is the one that a thread
+// by itself makes, to the bit.
+constexpr int kSandTerms = 32;  // terms of a particle; past that one lane adds them as it finds them
+struct SandTerms {
+    int   count;
+    int   odd;  // a term of two parts: added serially
+    int   j[kSandTerms];
+    float f[3][kSandTerms];
+};
+// visit(f, part) calls f(j) for the lane's share of the candidates that pass its test;
+// term(j, add) calls add(x, y, z) for each part of j's term, in order; all(f) calls f(j)
+// for every candidate in order.  Every lane of the warp calls it.
+template<int S, class Visit, class Term, class All, class Add>
+__device__ __forceinline__ void sum_terms(SandTerms & T, bool on, Visit && visit, Term && term, All && all, Add && add) {
+    const int part = threadIdx.x % S;
+    if (part == 0) T.count = T.odd = 0;
+    __syncwarp();
+    if (on)
+        visit([&](int j) {
+            const int k = atomicAdd(&T.count, 1);
+            if (k < kSandTerms) T.j[k] = j;
+        }, part);
+    __syncwarp();
+    const int total = on ? T.count : 0;
+    if (total <= kSandTerms)
+        for (int c = part; c < total; c += S) {
+            const int j = T.j[c];
+            int rank = 0, parts = 0;
+            for (int k = 0; k < total; k++) rank += T.j[k] < j ? 1 : 0;
+            float3 v = make_float3(0.f, 0.f, 0.f);
+            term(j, [&](float x, float y, float z) {
+                v = make_float3(x, y, z);
+                parts++;
+            });
+            if (parts > 1) T.odd = 1;
+            T.f[0][rank] = v.x, T.f[1][rank] = v.y, T.f[2][rank] = v.z;
+        }
+    __syncwarp();
+    if (total <= kSandTerms && T.odd == 0) {
+        for (int k = 0; k < total; k++) add(T.f[0][k], T.f[1][k], T.f[2][k]);
+    } else if (part == 0) all([&](int j) { term(j, add); });
+    __syncwarp();  // the terms are free again
+}
+
 // The contact pass.  d = x_j - x_i, w = v_j - v_i as in DEMParticle::getForce
 // (DEMParticle.cpp:62-67).
-template<int DIM>
+template<int DIM, int S>
 __global__ void __launch_bounds__(kSandNT, 5) k_sand_forces(const Lattice * __restrict__ Ld, Lattice Lb, SandPhys P,
                                                         const int * __restrict__ cellStart,
                                                         const float4 * __restrict__ pos, const float4 * __restrict__ plo,
@@ -296,10 +341,17 @@ __global__ void __launch_bounds__(kSandNT, 5) k_sand_forces(const Lattice * __re
                                                         const float4 * __restrict__ bnrm,
                                                         const unsigned char * __restrict__ bnear) {
     pdl_wait_and_release();
-    __shared__ int clist[kSandList * kSandNT];  // per-thread candidate lists, slot-major
+    __shared__ int clist[S == 1 ? kSandList * kSandNT : 1];  // per-thread candidate lists, slot-major
+    __shared__ SandTerms terms[S == 1 ? 1 : kSandNT / S];
+    SandTerms & T  = terms[S == 1 ? 0 : threadIdx.x / S];
+    const int lane = threadIdx.x & 31;
     const Lattice L = *Ld;
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        const float4 qi = pos[i], li = plo[i], vi = vel[i];
+    // (the warp's lanes in step where they share a particle)
+    for (long long i0 = (blockIdx.x * (long long) blockDim.x + (S == 1 ? threadIdx.x : threadIdx.x - lane)) / S; i0 < n;
+         i0 += (long long) gridDim.x * blockDim.x / S) {
+        const long long i = S == 1 ? i0 : i0 + lane / S;
+        const bool on     = S == 1 || i < n;
+        const float4 qi = pos[on ? i : 0], li = plo[on ? i : 0], vi = vel[on ? i : 0];
         // The FP32 window and pre-test ignore the low parts (|lo| <= 2^-24 |x|) and
         // round the difference once: widen the reach by 2^-21 (|x|_max + 2r).
         const float ax  = fmaxf(fabsf(qi.x), fmaxf(fabsf(qi.y), DIM == 3 ? fabsf(qi.z) : 0.f));
@@ -308,7 +360,7 @@ __global__ void __launch_bounds__(kSandNT, 5) k_sand_forces(const Lattice * __re
         float fx = 0.f, fy = 0.f, fz = 0.f;
         // the pair terms of the candidates that pass the FP32 pre-test; run from the
         // per-thread list below so the lanes of a warp take this path together
-        auto contact = [&](int j) {
+        auto contact = [&](int j, auto && add) {
             const float4 qj = pos[j];
             const float4 lj = plo[j];
             float hx, lx, hy, ly, hz = 0.f, lz = 0.f;
@@ -363,9 +415,7 @@ __global__ void __launch_bounds__(kSandNT, 5) k_sand_forces(const Lattice * __re
                     Sy *= k;
                     Sz *= k;
                 }
-                fx -= Nx + Sx;
-                fy -= Ny + Sy;
-                fz -= Nz + Sz;
+                add(Nx + Sx, Ny + Sy, Nz + Sz);
             }
             // DEMParticle::ComputeDemCapillaryForces (DEMParticle.cpp:98-124).  Every pair
             // that gets here has |d| < 2r, so H = |d| - 2r < 0 fails H > 1e-6: the
@@ -377,59 +427,102 @@ __global__ void __launch_bounds__(kSandNT, 5) k_sand_forces(const Lattice * __re
                 const float phi  = sqrtf(P.cap_b * H * (-1.f + sqrtf(1.f + P.cap_a / (H * H))));
                 const float s    = P.cap_neck / (1.f + H / (2.f * dd)) + P.cap_surf * phi;
                 const float inv  = 1.f / dist;
-                fx -= __fadd_rn(hx, lx) * inv * s;
-                fy -= __fadd_rn(hy, ly) * inv * s;
-                fz -= __fadd_rn(hz, lz) * inv * s;
+                add(__fadd_rn(hx, lx) * inv * s, __fadd_rn(hy, ly) * inv * s, __fadd_rn(hz, lz) * inv * s);
             }
         };
-        int cnt = 0;
-        for_each_in_radius<DIM>(L, cellStart, qi.x, qi.y, qi.z, Rq, Rq2, [&](int j) {
-            if (j == int(i)) return;  // d = 0, w = 0: the reference's self term is zero
+        auto take = [&](float x, float y, float z) {
+            fx -= x;
+            fy -= y;
+            fz -= z;
+        };
+        auto near = [&](int j) {
+            if (j == int(i)) return false;  // d = 0, w = 0: the reference's self term is zero
             const float4 qj = pos[j];
             const float ex = qj.x - qi.x, ey = qj.y - qi.y, ez = DIM == 3 ? qj.z - qi.z : 0.f;
-            if (ex * ex + ey * ey + ez * ez >= Rq2) return;
-            clist[cnt * kSandNT + threadIdx.x] = j;
-            if (++cnt == kSandList) {
-                for (int k = 0; k < cnt; k++) contact(clist[k * kSandNT + threadIdx.x]);
-                cnt = 0;
-            }
-        });
-        for (int k = 0; k < cnt; k++) contact(clist[k * kSandNT + threadIdx.x]);
+            return !(ex * ex + ey * ey + ez * ez >= Rq2);
+        };
+        if constexpr (S == 1) {
+            int cnt = 0;
+            for_each_in_radius<DIM>(L, cellStart, qi.x, qi.y, qi.z, Rq, Rq2, [&](int j) {
+                if (!near(j)) return;
+                clist[cnt * kSandNT + threadIdx.x] = j;
+                if (++cnt == kSandList) {
+                    for (int k = 0; k < cnt; k++) contact(clist[k * kSandNT + threadIdx.x], take);
+                    cnt = 0;
+                }
+            });
+            for (int k = 0; k < cnt; k++) contact(clist[k * kSandNT + threadIdx.x], take);
+        } else {
+            sum_terms<S>(
+                T, on,
+                [&](auto && found, int part) {
+                    for_each_in_radius<DIM, S>(L, cellStart, qi.x, qi.y, qi.z, Rq, Rq2,
+                                               [&](int j) { if (near(j)) found(j); }, part);
+                },
+                contact,
+                [&](auto && each) {
+                    for_each_in_radius<DIM>(L, cellStart, qi.x, qi.y, qi.z, Rq, Rq2,
+                                            [&](int j) { if (near(j)) each(j); });
+                },
+                take);
+        }
         // force = dt * sum_j F_ij, then the boundary terms without dt (DEMParticleSand.cpp:133-150)
         float Fx = fx * P.dt, Fy = fy * P.dt, Fz = fz * P.dt;
-        if (bnear[cell_linear(Lb, cell_of<DIM>(Lb, qi.x, qi.y, qi.z))]) {
-            for_each_in_radius<DIM>(Lb, bcellStart, qi.x, qi.y, qi.z, P.Rb * 1.0001f, P.Rb2 * 1.0002f, [&](int j) {
-                const float4 pb = bpos[j], lb = blo[j];
-                const float dx = (qi.x - pb.x) + (li.x - lb.x), dy = (qi.y - pb.y) + (li.y - lb.y);
-                const float dz = DIM == 3 ? (qi.z - pb.z) + (li.z - lb.z) : 0.f;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 >= P.Rb2) return;
-                const float w   = sand_wb(P, sqrtf(r2));
-                const float4 nb = bnrm[j];
-                // dv = v_i - v_b with v_b = 0 (the reference's _boundary_velocity is never set)
-                const float dvn = nb.x * vi.x + nb.y * vi.y + nb.z * vi.z;
-                const float m   = -pb.w * fminf(dvn, 0.f);
-                const float Nx = m * nb.x * w, Ny = m * nb.y * w, Nz = m * nb.z * w;
-                float ux = vi.x - dvn * nb.x, uy = vi.y - dvn * nb.y, uz = DIM == 3 ? vi.z - dvn * nb.z : 0.f;
-                if (ux * ux + uy * uy + uz * uz < 1e-4f * (vi.x * vi.x + vi.y * vi.y + vi.z * vi.z)) {
-                    // nearly normal motion: the tangential part in FP64, as in the contacts
-                    const double e = double(nb.x) * vi.x + double(nb.y) * vi.y + (DIM == 3 ? double(nb.z) * vi.z : 0.0);
-                    ux = float(double(vi.x) - e * nb.x);
-                    uy = float(double(vi.y) - e * nb.y);
-                    uz = DIM == 3 ? float(double(vi.z) - e * nb.z) : 0.f;
-                }
-                const float Tx = -P.Kt * ux, Ty = -P.Kt * uy, Tz = -P.Kt * uz;
-                const float nt = sqrtf(Tx * Tx + Ty * Ty + Tz * Tz);
-                float k        = 1.f;
-                if (nt > 0.000001f) {
-                    const float cap = sqrtf(Nx * Nx + Ny * Ny + Nz * Nz) * P.tanf;
-                    if (!(cap > nt)) k = cap / nt;
-                }
-                Fx += Nx + k * Tx;
-                Fy += Ny + k * Ty;
-                Fz += Nz + k * Tz;
-            });
+        auto wall_r2 = [&](int j) {
+            const float4 pb = bpos[j], lb = blo[j];
+            const float dx = (qi.x - pb.x) + (li.x - lb.x), dy = (qi.y - pb.y) + (li.y - lb.y);
+            const float dz = DIM == 3 ? (qi.z - pb.z) + (li.z - lb.z) : 0.f;
+            return dx * dx + dy * dy + dz * dz;
+        };
+        auto friction = [&](int j, auto && add) {
+            const float4 pb = bpos[j];
+            const float r2  = wall_r2(j);
+            if (r2 >= P.Rb2) return;
+            const float w   = sand_wb(P, sqrtf(r2));
+            const float4 nb = bnrm[j];
+            // dv = v_i - v_b with v_b = 0 (the reference's _boundary_velocity is never set)
+            const float dvn = nb.x * vi.x + nb.y * vi.y + nb.z * vi.z;
+            const float m   = -pb.w * fminf(dvn, 0.f);
+            const float Nx = m * nb.x * w, Ny = m * nb.y * w, Nz = m * nb.z * w;
+            float ux = vi.x - dvn * nb.x, uy = vi.y - dvn * nb.y, uz = DIM == 3 ? vi.z - dvn * nb.z : 0.f;
+            if (ux * ux + uy * uy + uz * uz < 1e-4f * (vi.x * vi.x + vi.y * vi.y + vi.z * vi.z)) {
+                // nearly normal motion: the tangential part in FP64, as in the contacts
+                const double e = double(nb.x) * vi.x + double(nb.y) * vi.y + (DIM == 3 ? double(nb.z) * vi.z : 0.0);
+                ux = float(double(vi.x) - e * nb.x);
+                uy = float(double(vi.y) - e * nb.y);
+                uz = DIM == 3 ? float(double(vi.z) - e * nb.z) : 0.f;
+            }
+            const float Tx = -P.Kt * ux, Ty = -P.Kt * uy, Tz = -P.Kt * uz;
+            const float nt = sqrtf(Tx * Tx + Ty * Ty + Tz * Tz);
+            float k        = 1.f;
+            if (nt > 0.000001f) {
+                const float cap = sqrtf(Nx * Nx + Ny * Ny + Nz * Nz) * P.tanf;
+                if (!(cap > nt)) k = cap / nt;
+            }
+            add(Nx + k * Tx, Ny + k * Ty, Nz + k * Tz);
+        };
+        auto push = [&](float x, float y, float z) {
+            Fx += x;
+            Fy += y;
+            Fz += z;
+        };
+        const bool wall = on && bnear[cell_linear(Lb, cell_of<DIM>(Lb, qi.x, qi.y, qi.z))];
+        const float Rb = P.Rb * 1.0001f, Rb2 = P.Rb2 * 1.0002f;
+        auto walls = [&](auto && each) {
+            for_each_in_radius<DIM>(Lb, bcellStart, qi.x, qi.y, qi.z, Rb, Rb2, each);
+        };
+        if constexpr (S == 1) {
+            if (wall) walls([&](int j) { friction(j, push); });
+        } else if (__any_sync(0xffffffffu, wall)) {
+            sum_terms<S>(
+                T, wall,
+                [&](auto && found, int part) {
+                    for_each_in_radius<DIM, S>(Lb, bcellStart, qi.x, qi.y, qi.z, Rb, Rb2,
+                                               [&](int j) { if (!(wall_r2(j) >= P.Rb2)) found(j); }, part);
+                },
+                friction, walls, push);
         }
+        if (S > 1 && (!on || lane % S != 0)) continue;
         float4 o = vi;
         o.x += Fx;
         o.y += Fy;
@@ -697,10 +790,18 @@ template<int DIM> int do_initialize(swc_sand * s) {
 
 template<int DIM> void launch_forces(swc_sand * s, float4 * out) {
     if (s->n == 0) return;
-    launch_pdl(k_sand_forces<DIM>, sand_grid(s->n, kSandNT, 152 * 64), kSandNT, 0, s->stream, (const Lattice *) s->dL,
-               s->Lb, s->P, (const int *) s->cellStart, (const float4 *) s->pos, (const float4 *) s->plo,
-               (const float4 *) s->vel, out, s->n, (const int *) s->bcellStart, (const float4 *) s->bpos,
-               (const float4 *) s->blo, (const float4 *) s->bnrm, (const unsigned char *) s->bnear);
+    const auto go = [&](auto kernel, int S) {
+        launch_pdl(kernel, sand_grid(s->n * S, kSandNT, 152 * 64), kSandNT, 0, s->stream, (const Lattice *) s->dL, s->Lb,
+                   s->P, (const int *) s->cellStart, (const float4 *) s->pos, (const float4 *) s->plo,
+                   (const float4 *) s->vel, out, s->n, (const int *) s->bcellStart, (const float4 *) s->bpos,
+                   (const float4 *) s->blo, (const float4 *) s->bnrm, (const unsigned char *) s->bnear);
+    };
+    // Eight lanes per particle while the chain of a particle's candidates bounds the pass, one
+    // once its instructions do.  With 1 and 8 lanes 15 and 7 us at 247 particles, 19 and 12 at
+    // 25,864, 21 and 19 at 58,370, 23 and 25 at 90,279 in 2D; 56 and 30 at 39,754, 68 and
+    // 58 at 92,597, 65 and 68 at 125,024, 79 and 99 at 194,509 in 3D.
+    if (s->n <= (DIM == 3 ? 7 << 14 : 1 << 16)) go(k_sand_forces<DIM, 8>, 8);
+    else go(k_sand_forces<DIM, 1>, 1);
 }
 
 template<int DIM> int do_advance(swc_sand * s, double dt) {

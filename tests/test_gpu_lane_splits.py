@@ -40,3 +40,28 @@ def test_splits_follow_the_oracle(swc_mod, oracle_mod, dim, n):
     np.testing.assert_allclose(gv["div"], ov["div"], rtol=0, atol=1e-4 * np.abs(ov["div"]).max())
     assert rel(liq.getParticles()[1], ref.particles()[1]) < TOL_V
     liq.close()
+
+
+# sand: 8 lanes per particle up to 114,688 particles (2D: 65,536), then one
+@pytest.mark.parametrize("dim,scale,low,high", [(3, 10, 1, 7 << 14), (3, 84, 1, 7 << 14), (3, 92, (7 << 14) + 1, 1 << 18),
+                                                (2, 16, 1, 1 << 16), (2, 500, (1 << 16) + 1, 1 << 18)])
+def test_sand_splits_follow_the_oracle(swc_mod, oracle_mod, dim, scale, low, high):
+    from test_gpu_sand import _check_step, _pair
+
+    s = scenes.sand_contact_block(dim, scale=scale, seed=scale, wall_depth=12 / (4 * scale))
+    assert low <= s.positions.shape[0] <= high, s.positions.shape
+    g, o = _pair(s, oracle_mod, swc_mod)
+    for _ in range(2):
+        _check_step(g, o, s.dt)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_sand_more_contacts_than_a_list(swc_mod, oracle_mod, dim):
+    """60 particles within a radius: 59 contacts each, past the 32 that the lanes share."""
+    from test_gpu_sand import _check_step, _pair
+
+    s = scenes.sand_contact_block(dim, scale=16, seed=2, wall_depth=12 / 64)
+    rng = np.random.default_rng(4)
+    s.positions[:60] = s.positions.mean(axis=0) + rng.uniform(-0.5, 0.5, (60, dim)) * s.radius
+    g, o = _pair(s, oracle_mod, swc_mod)
+    _check_step(g, o, s.dt)
