@@ -580,11 +580,13 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     }
 }
 
-// Few bricks: the larger groups take all bricks of a block at once (3D: at most four,
-// where their reads, 2,160 shared-memory wavefronts a brick against 1,250, still cost
-// less than the longer chain of the smaller groups).
+// Few bricks: the larger groups take all bricks of a block at once (3D: at most three,
+// where their reads, 2,160 shared-memory wavefronts a brick against 1,250, still cost no
+// more than the longer chain of the smaller groups: an iteration with the larger and the
+// smaller takes 7.9 and 8.8 us at 125 bricks, 10.2 and 11.3 at 216, 12.4 and 12.4 at 343,
+// 14.1 and 12.7 at 528).
 template<int DIM> __device__ __forceinline__ bool few_bricks(int nb, int blocks) {
-    return nb <= blocks * (DIM == 3 ? 4 : Group<DIM, WarpBrick<DIM>::WMAX>::COUNT);
+    return nb <= blocks * (DIM == 3 ? 3 : Group<DIM, WarpBrick<DIM>::WMAX>::COUNT);
 }
 
 }  // namespace

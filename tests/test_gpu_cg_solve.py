@@ -19,12 +19,12 @@ def bricks_3d(n):
     return scenes.projection_block_3d(n=n, seed=n)
 
 
-# active bricks on 152 SMs: one; a few; 3D up to 4 per block in groups of four warps and
+# active bricks on 152 SMs: one; a few; 3D up to 3 per block in groups of four warps and
 # past that in groups of two, with one more than a whole round; 2D up to 8 per block in
 # groups of two warps and past that single warps
 @pytest.mark.parametrize("build,n,low,high", [
     (bricks_2d, 9, 1, 4), (bricks_2d, 121, 60, 100), (bricks_2d, 601, 1217, 1700),
-    (bricks_3d, 9, 8, 8), (bricks_3d, 60, 609, 800), (bricks_3d, 96, 2129, 2500)])
+    (bricks_3d, 9, 8, 8), (bricks_3d, 45, 305, 456), (bricks_3d, 52, 457, 608), (bricks_3d, 60, 609, 800), (bricks_3d, 96, 2129, 2500)])
 def test_solve_at_brick_counts(swc_mod, build, n, low, high):
     s = build(n).rounded_to_float32()
     liq = swc_mod.DualParticleSphLiquid(s, warm_start="zero", tolerance=1e-5, compute_true_residual=True)
