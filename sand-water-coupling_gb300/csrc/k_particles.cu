@@ -475,16 +475,37 @@ __global__ void __launch_bounds__(256) k_near_x(Lattice L, const int * __restric
         out[c] = cellStart[row + min(x + R, L.nx - 1) + 1] > cellStart[row + max(x - R, 0)] ? 1 : 0;
     }
 }
-__global__ void __launch_bounds__(256) k_near_dilate(long long ncells, long long stride, int extent, int R,
+// A thread takes kDilate cells along the axis and their window as a bit mask, 14 loads
+// instead of 56 at R = 3 (a load per cell of every window and two 64-bit divisions a cell
+// took 33 us an axis at 8M cells).
+constexpr int kDilate = 8, kDilateReach = (64 - kDilate) / 2;
+__global__ void __launch_bounds__(256) k_near_dilate(unsigned outer, unsigned stride, int extent, int R,
                                                      const unsigned char * __restrict__ in,
                                                      unsigned char * __restrict__ out) {
     pdl_wait_and_release();
-    for (long long c = blockIdx.x * (long long) blockDim.x + threadIdx.x; c < ncells;
-         c += (long long) gridDim.x * blockDim.x) {
-        const int k = int((c / stride) % extent);
-        unsigned char v = 0;
-        for (int d = max(-R, -k); d <= min(R, extent - 1 - k); d++) v |= in[c + d * stride];
-        out[c] = v;
+    const unsigned chunks = (extent + kDilate - 1) / kDilate;
+    const long long total = (long long) outer * chunks * stride;  // cells < 2^31
+    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x) {
+        const unsigned i = unsigned(t) % stride, q = unsigned(t) / stride;
+        const int k0     = int(q % chunks) * kDilate;
+        const long long c0 = (long long) (q / chunks) * extent * stride + i;  // the line's first cell
+        if (R <= kDilateReach) {
+            unsigned long long m = 0;
+            for (int b = 0; b < kDilate + 2 * R; b++) {
+                const int k = k0 - R + b;
+                if (k >= 0 && k < extent && in[c0 + (long long) k * stride]) m |= 1ull << b;
+            }
+            const unsigned long long window = (2ull << 2 * R) - 1;
+#pragma unroll
+            for (int j = 0; j < kDilate; j++)
+                if (k0 + j < extent) out[c0 + (long long) (k0 + j) * stride] = m >> j & window ? 1 : 0;
+        } else {
+            for (int j = k0; j < min(k0 + kDilate, extent); j++) {
+                unsigned char v = 0;
+                for (int k = max(j - R, 0); k <= min(j + R, extent - 1); k++) v |= in[c0 + (long long) k * stride];
+                out[c0 + (long long) j * stride] = v;
+            }
+        }
     }
 }
 
@@ -616,131 +637,157 @@ __global__ void k_max_positive(const float * __restrict__ a, long long n, int * 
 
 // ---------------------------------------------------------------------------
 // Exclusive scan of int32 counts: sums of tiles, then each tile's scan from the sum of
-// the tiles before it, which its block adds up itself (past kScanSelf tiles a pass of its
-// own scans the tile sums).  out has n + 1 entries; out[n] = total.  The counts are left
-// zero, for the next count.  With Ld (a lattice in device memory) only its first
-// Ld->ncells <= n counts are scanned; the others stay zero.
+// the tiles before it.  Up to kScanSelf tiles a block adds those up itself (4 loads a
+// thread, 0.7 us); past that the last block of the first pass scans them (at 3,900 tiles
+// every block's own sum took the second pass from 17 to 30 us).  out has n + 1 entries;
+// out[n] = total.  The counts are left zero, for the next count.  With Ld (a lattice in
+// device memory) only its first Ld->ncells <= n counts are scanned; the others stay zero.
+// buf: 4 ints, zeroed once at allocation (buf[0] counts the first pass's blocks), then the
+// tiles.
 // ---------------------------------------------------------------------------
-constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
-// A block's own sum reads 16 tiles a thread at most there, under a microsecond, where the
-// pass that it saves takes 3; every block doing so reads tiles^2 / 2 words.
-constexpr int kScanSelf = 16 * kScanThreads;
+constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems, kScanHead = 4;
+constexpr int kScanSelf = 4 * kScanThreads;
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int * __restrict__ in, long long n,
-                                                              int * __restrict__ tile_sum, const Lattice * __restrict__ Ld) {
-    pdl_wait_and_release();
-    if (Ld) n = min(n, Ld->ncells);
-    __shared__ int sm[kScanThreads / 32];
-    const long long base = (long long) blockIdx.x * kScanTile;
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        const long long i = base + threadIdx.x + (long long) k * kScanThreads;
-        if (i < n) s += in[i];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < kScanThreads / 32; w++) t += sm[w];
-        tile_sum[blockIdx.x] = t;
-    }
-}
-
-__global__ void __launch_bounds__(1024) k_scan_top(int * __restrict__ tile_sum, int ntiles) {
-    pdl_wait_and_release();
-    __shared__ int sm[32];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < ntiles; base += 1024) {
-        const int i = base + threadIdx.x;
-        const int v = i < ntiles ? tile_sum[i] : 0;
-        int x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((threadIdx.x & 31) >= o) x += y;
-        }
-        if ((threadIdx.x & 31) == 31) sm[threadIdx.x >> 5] = x;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            int w = sm[threadIdx.x];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, o);
-                if (threadIdx.x >= o) w += y;
-            }
-            sm[threadIdx.x] = w;
-        }
-        __syncthreads();
-        const int warp_off = (threadIdx.x >> 5) ? sm[(threadIdx.x >> 5) - 1] : 0;
-        const int incl     = x + warp_off + carry;
-        if (i < ntiles) tile_sum[i] = incl - v;  // exclusive
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = incl;
-        __syncthreads();
-    }
-}
-
-// SELF: tiles holds the tiles' sums, else their exclusive scan.
-template<bool SELF>
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(int * __restrict__ in, long long n,
-                                                              const int * __restrict__ tiles, int * __restrict__ out,
-                                                              const Lattice * __restrict__ Ld) {
-    pdl_wait_and_release();
-    if (Ld) {
-        n = min(n, Ld->ncells);
-        if ((long long) blockIdx.x * kScanTile > n) return;  // past the lattice's cells (and past out[n])
-    }
-    __shared__ int sm[kScanThreads / 32], before[kScanThreads / 32];
-    if (SELF) {
-        int t = 0;
-        for (int i = threadIdx.x; i < int(blockIdx.x); i += kScanThreads) t += tiles[i];
-        t = __reduce_add_sync(0xffffffffu, t);
-        if ((threadIdx.x & 31) == 0) before[threadIdx.x >> 5] = t;
-    }
-    const long long base = (long long) blockIdx.x * kScanTile + (long long) threadIdx.x * kScanItems;
-    int v[kScanItems];
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        const long long i = base + k;
-        v[k]              = i < n ? in[i] : 0;
-        if (i < n) in[i] = 0;
-        s += v[k];
-    }
-    int x = s;
+// Exclusive scan over the block's threads of one value each; the block's sum into total.
+__device__ __forceinline__ int block_scan(int v, int * sm, int & total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if ((threadIdx.x & 31) >= o) x += y;
+        if (lane >= o) x += y;
     }
-    if ((threadIdx.x & 31) == 31) sm[threadIdx.x >> 5] = x;
+    __syncthreads();  // sm is free
+    if (lane == 31) sm[warp] = x;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        int w = threadIdx.x < kScanThreads / 32 ? sm[threadIdx.x] : 0;
+    int before = 0;
+    total      = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (threadIdx.x >= o) w += y;
+    for (int w = 0; w < kScanThreads / 32; w++) {
+        if (w == warp) before = total;
+        total += sm[w];
+    }
+    return before + x - v;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int * __restrict__ in, long long n, int * buf,
+                                                             const Lattice * __restrict__ Ld, int top) {
+    pdl_wait_and_release();
+    if (Ld) n = min(n, Ld->ncells);
+    __shared__ int sm[kScanThreads / 32];
+    __shared__ bool last;
+    int * tiles          = buf + kScanHead;
+    const long long base = (long long) blockIdx.x * kScanTile;
+    if (base < n) {
+        int s = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            const long long i = base + threadIdx.x + (long long) k * kScanThreads;
+            if (i < n) s += in[i];
         }
-        if (threadIdx.x < kScanThreads / 32) sm[threadIdx.x] = w;
+        s = __reduce_add_sync(0xffffffffu, s);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int t = 0;
+            for (int w = 0; w < kScanThreads / 32; w++) t += sm[w];
+            tiles[blockIdx.x] = t;
+        }
+    }
+    if (!top) return;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(buf, 1) == int(gridDim.x) - 1;
     }
     __syncthreads();
-    int run = x - s + ((threadIdx.x >> 5) ? sm[(threadIdx.x >> 5) - 1] : 0);
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x == 0) buf[0] = 0;
+    const int nt = int((n + kScanTile - 1) / kScanTile);
+    int carry = 0;
+    for (int t0 = 0; t0 < nt; t0 += kScanTile) {
+        int v[kScanItems], s = 0, total;
+        const int at = t0 + int(threadIdx.x) * kScanItems;
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            v[k] = at + k < nt ? __ldcg(tiles + at + k) : 0;
+            s += v[k];
+        }
+        int run = carry + block_scan(s, sm, total);
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            if (at + k < nt) tiles[at + k] = run;
+            run += v[k];
+        }
+        carry += total;
+    }
+}
+
+// SELF: the tiles hold their sums, else their exclusive scan.
+template<bool SELF>
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(int * __restrict__ in, long long n,
+                                                             const int * __restrict__ buf, int * __restrict__ out,
+                                                             const Lattice * __restrict__ Ld) {
+    pdl_wait_and_release();
+    if (Ld) n = min(n, Ld->ncells);
+    __shared__ int sm[kScanThreads / 32];
+    const int * tiles    = buf + kScanHead;
+    const long long base = (long long) blockIdx.x * kScanTile + (long long) threadIdx.x * kScanItems;
+    if ((long long) blockIdx.x * kScanTile >= n) {
+        // past the lattice's cells; an empty one has its total here
+        if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) out[0] = 0;
+        return;
+    }
+    int before = 0, total;
     if (SELF) {
+        int t = 0;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < int(blockIdx.x); i += kScanThreads) t += tiles[i];
+        t = __reduce_add_sync(0xffffffffu, t);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = t;
+        __syncthreads();
 #pragma unroll
-        for (int w = 0; w < kScanThreads / 32; w++) run += before[w];
-    } else run += tiles[blockIdx.x];
+        for (int w = 0; w < kScanThreads / 32; w++) before += sm[w];
+    } else before = tiles[blockIdx.x];
+    int v[kScanItems], s = 0;
+    const bool whole = base + kScanItems <= n;
+    if (whole) {
+        int4 * p = reinterpret_cast<int4 *>(in + base);
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        const long long i = base + k;
-        if (i < n) out[i] = run;
-        run += v[k];
-        if (i == n - 1) out[n] = run;
+        for (int k = 0; k < kScanItems / 4; k++) {
+            const int4 q = p[k];
+            p[k]         = make_int4(0, 0, 0, 0);
+            v[4 * k] = q.x, v[4 * k + 1] = q.y, v[4 * k + 2] = q.z, v[4 * k + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            v[k] = base + k < n ? in[base + k] : 0;
+            if (base + k < n) in[base + k] = 0;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) s += v[k];
+    int run = before + block_scan(s, sm, total);
+    if (whole) {
+        int4 * o = reinterpret_cast<int4 *>(out + base);
+#pragma unroll
+        for (int k = 0; k < kScanItems / 4; k++) {
+            int4 q;
+            q.x = run, q.y = q.x + v[4 * k], q.z = q.y + v[4 * k + 1], q.w = q.z + v[4 * k + 2];
+            run  = q.w + v[4 * k + 3];
+            o[k] = q;
+        }
+        if (base + kScanItems == n) out[n] = run;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            if (base + k < n) {
+                out[base + k] = run;
+                run += v[k];
+                if (base + k == n - 1) out[n] = run;
+            }
+        }
     }
 }
 
@@ -775,19 +822,18 @@ void launch_export_ratio(const float * a, int stride, int comp, float num, const
     if (n > 0) k_export_ratio<<<grid_for(n, 256), 256, 0, st>>>(a, stride, comp, num, id, n, out);
 }
 
-void launch_scan(int * in, long long n, int * out, int * tile_buf, cudaStream_t st, const Lattice * Ld) {
+void launch_scan(int * in, long long n, int * out, int * buf, cudaStream_t st, const Lattice * Ld) {
     const long long ntiles = (n + kScanTile - 1) / kScanTile;
     if (n <= 0) {
         cudaMemsetAsync(out, 0, sizeof(int), st);
         return;
     }
-    launch_pdl(k_scan_tiles, int(ntiles), kScanThreads, 0, st, (const int *) in, n, tile_buf, Ld);
-    if (ntiles > kScanSelf) {
-        launch_pdl(k_scan_top, 1, 1024, 0, st, tile_buf, int(ntiles));
-        launch_pdl(k_scan_apply<false>, int(ntiles), kScanThreads, 0, st, in, n, (const int *) tile_buf, out, Ld);
-    } else launch_pdl(k_scan_apply<true>, int(ntiles), kScanThreads, 0, st, in, n, (const int *) tile_buf, out, Ld);
+    const bool self = ntiles <= kScanSelf;
+    launch_pdl(k_scan_tiles, int(ntiles), kScanThreads, 0, st, (const int *) in, n, buf, Ld, self ? 0 : 1);
+    if (self) launch_pdl(k_scan_apply<true>, int(ntiles), kScanThreads, 0, st, in, n, (const int *) buf, out, Ld);
+    else launch_pdl(k_scan_apply<false>, int(ntiles), kScanThreads, 0, st, in, n, (const int *) buf, out, Ld);
 }
-long long scan_tile_count(long long n) { return (n + kScanTile - 1) / kScanTile + 1; }
+long long scan_buffer_ints(long long n) { return kScanHead + (n + kScanTile - 1) / kScanTile; }
 
 template<int DIM>
 void launch_bin(const Lattice & L, long long n, float4 *& pos, float4 *& vel, float4 *& aux, int *& id,
@@ -876,11 +922,13 @@ void launch_near_cells(const int * cellStart, long long n, const Lattice & L, co
     // 3D: x -> near, y: near -> tmp, z: tmp -> near; 2D: x -> tmp, y: tmp -> near
     unsigned char * xo = DIM == 3 ? near : tmp;
     launch_pdl(k_near_x<DIM>, g, 256, 0, st, L, cellStart, R, xo);
-    launch_pdl(k_near_dilate, g, 256, 0, st, L.ncells, (long long) L.nx, L.ny, R, (const unsigned char *) xo,
-               DIM == 3 ? tmp : near);
-    if (DIM == 3)
-        launch_pdl(k_near_dilate, g, 256, 0, st, L.ncells, (long long) L.nx * L.ny, L.nz, R, (const unsigned char *) tmp,
-                   near);
+    const auto dilate = [&](unsigned outer, unsigned stride, int extent, const unsigned char * in, unsigned char * out) {
+        const long long n = (long long) outer * ((extent + kDilate - 1) / kDilate) * stride;
+        launch_pdl(k_near_dilate, int(std::min<long long>((n + 255) / 256, 152LL * 16)), 256, 0, st, outer, stride, extent, R,
+                   in, out);
+    };
+    dilate(L.nz, L.nx, L.ny, xo, DIM == 3 ? tmp : near);
+    if (DIM == 3) dilate(1, L.nx * L.ny, L.nz, tmp, near);
 }
 void launch_rotate_boundary(float4 * bpos, float4 * bvel, float4 * bnrm, long long nb, float cx, float cz,
                             float omega, float dt, cudaStream_t st) {

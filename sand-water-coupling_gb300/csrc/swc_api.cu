@@ -186,7 +186,8 @@ int alloc_sort(swc_ctx * c, SortScratch & S, long long n, bool aux) {
     if ((rc = dalloc(c, &S.perm, n))) return rc;
     if ((rc = dalloc(c, &S.count, c->L.ncells))) return rc;
     CK(cudaMemsetAsync(S.count, 0, sizeof(int) * c->L.ncells, c->stream));
-    if ((rc = dalloc(c, &S.tiles, scan_tile_count(c->L.ncells + 1) + 2))) return rc;
+    if ((rc = dalloc(c, &S.tiles, scan_buffer_ints(c->L.ncells)))) return rc;
+    CK(cudaMemsetAsync(S.tiles, 0, 4 * sizeof(int), c->stream));
     if ((rc = dalloc(c, &S.pos2, n))) return rc;
     if ((rc = dalloc(c, &S.vel2, n))) return rc;
     if (aux && (rc = dalloc(c, &S.aux2, n))) return rc;
@@ -765,7 +766,7 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
         (rc = dalloc(c, &c->pcount, 1)) || (rc = dalloc(c, &c->bnear, L.nbricks)))
         return fail(rc);
     if ((rc = dalloc(c, &c->pcomp, size_t(L.ncells))) || (rc = dalloc(c, &c->nv_prev, 1)) ||
-        (rc = dalloc(c, &c->scan_tiles, scan_tile_count(std::max<long long>(c->B.nseg, L.ncells) + 1) + 2)) ||
+        (rc = dalloc(c, &c->scan_tiles, scan_buffer_ints(std::max<long long>(c->B.nseg, L.ncells)))) ||
         (rc = dalloc(c, &c->cg, 1)) || (rc = dalloc(c, &c->partials, npart)) || (rc = dalloc(c, &c->queues, 4)) ||
         (rc = dalloc(c, &c->slots, 4 * size_t(c->cgrid + 8))) || (rc = dalloc(c, &c->uflags, size_t(L.nbricks))) || (rc = dalloc(c, &c->phases, 1)) ||
         (rc = dalloc(c, &c->diag_bits, 1)) || (rc = dalloc(c, &c->max_bits, 1)) || (rc = dalloc(c, &c->res2, 2)) ||
@@ -782,6 +783,7 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
     cudaMemsetAsync(c->B.flag_prev, 0, L.nbricks, c->stream);
     cudaMemsetAsync(c->N.flag, 0, slots, c->stream);
     cudaMemsetAsync(c->B.seg, 0, sizeof(int) * c->B.nseg, c->stream);
+    cudaMemsetAsync(c->scan_tiles, 0, 4 * sizeof(int), c->stream);
     cudaMemsetAsync(c->N.x, 0, slots * sizeof(float), c->stream);
     cudaMemsetAsync(c->nv_prev, 0, sizeof(int), c->stream);
     cudaMemsetAsync(c->bcellStart, 0, sizeof(int) * (L.ncells + 1), c->stream);

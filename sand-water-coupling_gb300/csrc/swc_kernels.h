@@ -68,9 +68,9 @@ void launch_max_speed2(const float4 * vel, long long n, int dim, unsigned long l
 void launch_export_ratio(const float * a, int stride, int comp, float num, const int * id, long long n, double * out,
                          cudaStream_t st);
 // (in, zeroed once at allocation, is left zero)
-void launch_scan(int * in, long long n, int * out, int * tile_buf, cudaStream_t st,
+void launch_scan(int * in, long long n, int * out, int * buf, cudaStream_t st,
                  const Lattice * Ld = nullptr);
-long long scan_tile_count(long long n);
+long long scan_buffer_ints(long long n);  // of the buffer, whose first 4 ints are zeroed once
 void launch_set_volume(float4 * pos, const float * rho, long long n, float mass, cudaStream_t st);
 void launch_rotate_boundary(float4 * bpos, float4 * bvel, float4 * bnrm, long long nb, float cx, float cz,
                             float omega, float dt, cudaStream_t st);

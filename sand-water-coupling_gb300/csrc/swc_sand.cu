@@ -701,9 +701,10 @@ int ensure_sand_cells(swc_sand * s) {
     s->Lcap.ncells = cap;
     int rc;
     if ((rc = salloc(s, &s->cellStart, cap + 1)) || (rc = salloc(s, &s->S.count, cap)) ||
-        (rc = salloc(s, &s->S.tiles, scan_tile_count(cap + 1) + 2)))
+        (rc = salloc(s, &s->S.tiles, scan_buffer_ints(cap))))
         return rc;
     SK(cudaMemsetAsync(s->S.count, 0, sizeof(int) * cap, s->stream));
+    SK(cudaMemsetAsync(s->S.tiles, 0, 4 * sizeof(int), s->stream));
     return SWC_OK;
 }
 
@@ -748,9 +749,10 @@ template<int DIM> int do_initialize(swc_sand * s) {
     if ((rc = salloc(s, &B.key, s->nb)) || (rc = salloc(s, &B.rank, s->nb)) || (rc = salloc(s, &B.perm, s->nb)) ||
         (rc = salloc(s, &B.pos2, s->nb)) || (rc = salloc(s, &B.vel2, s->nb)) || (rc = salloc(s, &B.aux2, s->nb)) ||
         (rc = salloc(s, &B.id2, s->nb)) || (rc = salloc(s, &B.count, Lb.ncells)) ||
-        (rc = salloc(s, &B.tiles, scan_tile_count(Lb.ncells + 1) + 2)))
+        (rc = salloc(s, &B.tiles, scan_buffer_ints(Lb.ncells))))
         return rc;
     SK(cudaMemsetAsync(B.count, 0, sizeof(int) * Lb.ncells, st));
+    SK(cudaMemsetAsync(B.tiles, 0, 4 * sizeof(int), st));
     launch_bin<DIM>(Lb, s->nb, s->bpos, s->bnrm, s->blo, s->bid, B, s->bcellStart, 0.f, st);
     SK(cudaGetLastError());
     SK(cudaStreamSynchronize(st));

@@ -1,5 +1,5 @@
 """Binning: lattices past the size where a scan block adds up the tiles before its own
-(8.4M cells), and cells that hold many particles."""
+(2.1M cells), and cells that hold many particles."""
 import numpy as np
 import pytest
 
