@@ -367,12 +367,25 @@ __device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const in
     return __all_sync(0xffffffffu, there);
 }
 
+// The state to host memory (pinned), but for `failed`, which any block sets there.
+__device__ __forceinline__ void to_host(const CgState * cg, CgState * host) {
+    if (!host) return;
+    host->bb      = cg->bb;
+    host->rr      = cg->rr;
+    host->rr0     = cg->rr0;
+    host->iter    = cg->iter;
+    host->done    = cg->done;
+    host->start   = cg->start;
+    host->nv      = cg->nv;
+    host->nbricks = cg->nbricks;
+}
+
 // Groups of W warps own the bricks c + P (g + COUNT k): the solve's loop.
 template<int DIM, int W>
 __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict__ blist, int nb, int P,
                                       const unsigned char * __restrict__ bflag, const NodeArrays & N, const Stencil & S,
                                       CgState * cg, const CgStart & from, ulonglong2 * slots, unsigned * flags,
-                                      CgPhases * phases, MeetSmem<WarpBrick<DIM>::WARPS> & M) {
+                                      CgPhases * phases, CgState * host, MeetSmem<WarpBrick<DIM>::WARPS> & M) {
     using B  = WarpBrick<DIM>;
     using G  = typename B::G;
     using Gr = Group<DIM, W>;
@@ -575,8 +588,12 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
             }
             cg->tick = tag;
             if (phases) *phases = spent;
+            to_host(cg, host);
         }
-        if (o.code == kFailed) atomicExch(&cg->failed, 1);
+        if (o.code == kFailed) {
+            atomicExch(&cg->failed, 1);
+            if (host) host->failed = 1;
+        }
     }
 }
 
@@ -595,7 +612,7 @@ template<int DIM>
 __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     k_cg_solve(Lattice L, const int * __restrict__ blist, const int * __restrict__ bcount,
                const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, CgState * cg, CgStart from,
-               ulonglong2 * slots, unsigned * flags, CgPhases * phases) {
+               ulonglong2 * slots, unsigned * flags, CgPhases * phases, CgState * host) {
     using B = WarpBrick<DIM>;
     constexpr int Q = B::G::BN / 4;
     __shared__ MeetSmem<B::WARPS> M;
@@ -609,6 +626,7 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
             CgScalars none;
             decide_start(cg, none, 0.0, 0.0, 0, from);
         }
+        if (done || nb == 0) to_host(cg, host);
     }
     if (done) {
         // no solve: a zero right-hand side (4) or a start that is not a number (3) leaves x = 0
@@ -621,8 +639,8 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     const int P = min(int(gridDim.x), nb);
     if (int(blockIdx.x) >= P) return;
     if (few_bricks<DIM>(nb, gridDim.x))
-        solve<DIM, B::WMAX>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, M);
-    else solve<DIM, B::WMIN>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, M);
+        solve<DIM, B::WMAX>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, host, M);
+    else solve<DIM, B::WMIN>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, host, M);
 }
 
 // Row-stencil passes outside the iteration, the bricks strided over the warps of a
@@ -801,7 +819,7 @@ void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeAr
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
                     const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases,
-                    cudaStream_t st) {
+                    CgState * host, cudaStream_t st) {
     using W = WarpBrick<DIM>;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim          = blocks;
@@ -814,7 +832,7 @@ int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays &
     cfg.attrs    = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_cg_solve<DIM>, L, (const int *) B.list, (const int *) B.count,
-                              (const unsigned char *) B.flag, N, S, cg, from, slots, flags, phases) == cudaSuccess
+                              (const unsigned char *) B.flag, N, S, cg, from, slots, flags, phases, host) == cudaSuccess
                ? 0
                : -1;
 }
@@ -831,7 +849,7 @@ int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays &
                                          cudaStream_t);                                                                \
     template int launch_cg_solve<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,         \
                                     CgState *, const CgStart &, ulonglong2 *, unsigned *, int, CgPhases *,             \
-                                    cudaStream_t);
+                                    CgState *, cudaStream_t);
 SWC_INST(2)
 SWC_INST(3)
 #undef SWC_INST

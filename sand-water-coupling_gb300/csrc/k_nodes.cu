@@ -364,6 +364,7 @@ __global__ void __launch_bounds__(kNT) k_warm_start(Lattice L, const int * __res
                                                     BrickArrays B, NodeArrays N, int mode, int history,
                                                     const float * __restrict__ pcomp,
                                                     const int * __restrict__ nv_prev, const float * __restrict__ given) {
+    pdl_wait_and_release();
     using G      = BrickGeom<DIM>;
     const int nb = *bcount;
     const int np = nv_prev ? *nv_prev : 0;
@@ -440,8 +441,11 @@ __global__ void __launch_bounds__(kNT) k_compact_export(Lattice L, const int * _
                                                         long long * __restrict__ node_id, double * __restrict__ rho,
                                                         double * __restrict__ vol, double * __restrict__ vbar,
                                                         double * __restrict__ div, double * __restrict__ ahat,
-                                                        double * __restrict__ p, unsigned short * __restrict__ nreal_out) {
+                                                        double * __restrict__ p, unsigned short * __restrict__ nreal_out,
+                                                        const int * __restrict__ nv, int * __restrict__ nv_out) {
+    pdl_wait_and_release();
     using G      = BrickGeom<DIM>;
+    if (nv_out && blockIdx.x == 0 && threadIdx.x == 0) *nv_out = *nv;
     const int nb = *bcount;
     for (int bi = blockIdx.x; bi < nb; bi += gridDim.x) {
         const int b   = blist[bi];
@@ -840,16 +844,16 @@ void launch_warm_start(const Lattice & L, const BrickArrays & B, const NodeArray
                                                                                                     N, history);
         return;
     }
-    k_warm_start<DIM><<<grid, kNT, 0, st>>>(L, B.list, B.count, B.seg_off, B, N, mode, history, pcomp, nv_prev,
-                                            given);
+    launch_pdl(k_warm_start<DIM>, grid, kNT, 0, st, L, B.list, B.count, B.seg_off, B, N, mode, history, pcomp, nv_prev, given);
 }
 
 template<int DIM>
 void launch_compact_export(const Lattice & L, const BrickArrays & B, const NodeArrays & N, float * pcomp,
                            long long * node_id, double * rho, double * vol, double * vbar, double * div,
-                           double * ahat, double * p, unsigned short * nreal_out, int grid, cudaStream_t st) {
-    k_compact_export<DIM><<<grid, kNT, 0, st>>>(L, B.list, B.count, B.seg_off, N, pcomp, node_id, rho, vol, vbar, div,
-                                                ahat, p, nreal_out);
+                           double * ahat, double * p, unsigned short * nreal_out, int grid, cudaStream_t st,
+                           int * nv_out) {
+    launch_pdl(k_compact_export<DIM>, grid, kNT, 0, st, L, B.list, B.count, B.seg_off, N, pcomp, node_id, rho, vol, vbar,
+               div, ahat, p, nreal_out, B.seg_off + B.nseg, nv_out);
 }
 
 template<int DIM>
@@ -874,7 +878,7 @@ void launch_compact_import(const Lattice & L, const BrickArrays & B, const NodeA
                                        const int *, const float *, int, cudaStream_t, int);                            \
     template void launch_compact_export<D>(const Lattice &, const BrickArrays &, const NodeArrays &, float *,          \
                                            long long *, double *, double *, double *, double *, double *, double *,    \
-                                           unsigned short *, int, cudaStream_t);                                       \
+                                           unsigned short *, int, cudaStream_t, int *);                                       \
     template void launch_compact_import<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const double *,   \
                                            float *, int, cudaStream_t);
 SWC_INST(2)

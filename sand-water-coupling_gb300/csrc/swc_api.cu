@@ -329,7 +329,9 @@ template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features =
 // that the caller queued).
 template<int DIM> int queue_cg(swc_ctx * c, bool started) {
     const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg};
-    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, nullptr, c->stream)) {
+    c->hcg->st.failed = 0;
+    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, nullptr, &c->hcg->st,
+                             c->stream)) {
         c->err = std::string("CG solve: ") + cudaGetErrorString(cudaGetLastError());
         return SWC_CUDA_ERROR;
     }
@@ -370,8 +372,7 @@ int cg_outcome(swc_ctx * c, swc_stats * st) {
 // previous pressure vector, ParticlesBasedData.h:25-29).
 template<int DIM> int export_prefix(swc_ctx * c) {
     launch_compact_export<DIM>(c->L, c->B, c->N, c->pcomp, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                               nullptr, nullptr, c->grid, c->stream);
-    CK(cudaMemcpyAsync(c->nv_prev, c->B.seg_off + c->B.nseg, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
+                               nullptr, nullptr, c->grid, c->stream, c->nv_prev);
     c->pcomp_stale = false;
     return SWC_OK;
 }
@@ -487,8 +488,6 @@ template<int DIM> int queue_projection(swc_ctx * c, Projection & pr) {
         if ((rc = export_prefix<DIM>(c))) return rc;
     } else c->pcomp_stale = true;
     mark(c, 8);
-    // (not between the solve and the gradient: three copies there cost 17 us a step)
-    CK(cudaMemcpyAsync(&c->hcg->st, c->cg, sizeof(CgState), cudaMemcpyDeviceToHost, c->stream));
     return SWC_OK;
 }
 
@@ -1366,7 +1365,7 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         for (int k = 0; k < 2; k++) {  // warm, then timed
             const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg};
             auto go = [&](auto run) {
-                run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->phases, c->stream);
+                run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->phases, nullptr, c->stream);
             };
             if (c->dim == 3) go(launch_cg_solve<3>);
             else go(launch_cg_solve<2>);

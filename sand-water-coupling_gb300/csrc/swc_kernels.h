@@ -161,17 +161,19 @@ void launch_warm_start(const Lattice & L, const BrickArrays & B, const NodeArray
 template<int DIM>
 void launch_compact_export(const Lattice & L, const BrickArrays & B, const NodeArrays & N, float * pcomp,
                            long long * node_id, double * rho, double * vol, double * vbar, double * div,
-                           double * ahat, double * p, unsigned short * nreal_out, int grid, cudaStream_t st);
+                           double * ahat, double * p, unsigned short * nreal_out, int grid, cudaStream_t st,
+                           int * nv_out = nullptr);
 // CG.  The solve is one resident kernel (k_cg_solve.cu) on `blocks` blocks, one per
 // SM; `slots` (4 x (blocks + 8)) and `flags` (one per brick), zeroed once at allocation, are its
 // meeting slots and the bricks' flags.
-// A failed launch returns nonzero; a wait that times out sets cg->failed.
+// A failed launch returns nonzero; a wait that times out sets cg->failed.  The outcome goes
+// to `host` (pinned memory, or null) as well, there once the stream was waited for.
 // cg_solve_prepare sets the kernels' shared-memory attribute on the current device.
 template<int DIM> int cg_solve_prepare();
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
                     const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases,
-                    cudaStream_t st);
+                    CgState * host, cudaStream_t st);
 template<int DIM>
 void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                           const float * x, float * r, float * d, double * sums, CgState * cg, double * partials,
