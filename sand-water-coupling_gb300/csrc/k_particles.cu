@@ -197,9 +197,10 @@ template<int S> __device__ __forceinline__ float2 group_sum(float2 v) {
 // Cores/Structures/SmoothedParticles.cpp:25-31); writes vel.w = m / rho_i and rho_i.
 // One group of S lanes per pair of consecutive sorted particles, the cell rows of the
 // pair's window spread over the lanes (S = 1 where the pairs alone fill the SMs, see
-// pair_lanes).  A pair that is not in one cell row is appended to left (left[0] =
-// count, ids from left[2]) and visited particle by particle by k_density_left, so no
-// warp runs both paths.
+// pair_lanes).  With S = 1 a pair that is not in one cell row is appended to left (left[0]
+// = count, ids from left[2]) and visited particle by particle by k_density_left, so no
+// warp runs both paths; with lanes the group visits its two particles one after the other
+// (a launch more took 5 us where the pass itself takes 8).
 template<int DIM, int S>
 __global__ void __launch_bounds__(256) k_density(const float4 * __restrict__ pos, float4 * __restrict__ vel,
                                                  float * __restrict__ rho_out, long long n, Lattice L, Phys P,
@@ -216,9 +217,17 @@ __global__ void __launch_bounds__(256) k_density(const float4 * __restrict__ pos
         float2 s = f2(0.f);
         if (on) {
             const float4 qa = pos[ia], qb = pos[ib];
-            if (near_pair<DIM>(L, qa, qb)) s = density_sum2<DIM, S>(L, P, cellStart, pos, qa, qb, part);
+            const bool near = near_pair<DIM>(L, qa, qb);
+            if constexpr (S > 1) {
+#pragma unroll 1
+                for (int k = 0; k < (near ? 1 : 2); k++) {
+                    const float4 a = k ? qb : qa;
+                    const float2 r = density_sum2<DIM, S>(L, P, cellStart, pos, a, near ? qb : a, part);
+                    s              = k ? make_float2(s.x, r.x) : r;
+                }
+            } else if (near) s = density_sum2<DIM, S>(L, P, cellStart, pos, qa, qb, part);
             else {
-                if (part == 0) left[2 + atomicAdd(left, 1)] = int(t);
+                left[2 + atomicAdd(left, 1)] = int(t);
                 on = false;
             }
         }
@@ -340,10 +349,20 @@ __global__ void __launch_bounds__(256) k_forces(const float4 * __restrict__ pos,
             const float4 qa = pos[ia], qb = pos[ib];
             va = vel[ia], vb = vel[ib];
             if (P.viscosity != 0.f) {
-                if (near_pair<DIM>(L, qa, qb))
-                    viscous_sum2<DIM, S>(L, P, cellStart, pos, vel, qa, va, qb, vb, part, lx, ly, lz);
+                const bool near = near_pair<DIM>(L, qa, qb);
+                if constexpr (S > 1) {
+#pragma unroll 1
+                    for (int k = 0; k < (near ? 1 : 2); k++) {
+                        const float4 a = k ? qb : qa, u = k ? vb : va;
+                        float2 rx = f2(0.f), ry = f2(0.f), rz = f2(0.f);
+                        viscous_sum2<DIM, S>(L, P, cellStart, pos, vel, a, u, near ? qb : a, near ? vb : u, part, rx, ry, rz);
+                        lx = k ? make_float2(lx.x, rx.x) : rx;
+                        ly = k ? make_float2(ly.x, ry.x) : ry;
+                        lz = k ? make_float2(lz.x, rz.x) : rz;
+                    }
+                } else if (near) viscous_sum2<DIM, S>(L, P, cellStart, pos, vel, qa, va, qb, vb, part, lx, ly, lz);
                 else {
-                    if (part == 0) left[2 + atomicAdd(left, 1)] = int(t);
+                    left[2 + atomicAdd(left, 1)] = int(t);
                     on = false;
                 }
             }
@@ -875,7 +894,7 @@ void launch_density(const float4 * pos, float4 * vel, float * rho, long long n, 
                    left);
     };
     DIM == 3 && S == 8 ? go(k_density<DIM, 8>) : S == 4 ? go(k_density<DIM, 4>) : S == 2 ? go(k_density<DIM, 2>) : go(k_density<DIM, 1>);
-    launch_pdl(k_density_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass, left);
+    if (S == 1) launch_pdl(k_density_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass, left);
 }
 void launch_set_volume(float4 * pos, const float * rho, long long n, float mass, cudaStream_t st) {
     if (n > 0) k_set_volume<<<grid_for(n, 256), 256, 0, st>>>(pos, rho, n, mass);
@@ -890,7 +909,7 @@ void launch_forces(const float4 * pos, const float4 * vel, float4 * vel_out, lon
                    left);
     };
     DIM == 3 && S == 8 ? go(k_forces<DIM, 8>) : S == 4 ? go(k_forces<DIM, 4>) : S == 2 ? go(k_forces<DIM, 2>) : go(k_forces<DIM, 1>);
-    launch_pdl(k_forces_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt, left);
+    if (S == 1) launch_pdl(k_forces_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt, left);
 }
 template<int DIM>
 void launch_boundary_density(float4 * bpos, float4 * bvel, float * rho, long long nb, const Lattice & L,
