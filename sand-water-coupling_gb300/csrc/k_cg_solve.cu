@@ -3,7 +3,8 @@
 // of the CG start).
 //
 // CG (Eigen's Hestenes-Stiefel form on the full matrix, k_cg.cu) from the start
-// state to its end in one cooperative launch, one block per SM.  A group of W warps
+// state to its end in one cooperative launch, one block per SM (or, for lattices of few
+// bricks, one cluster).  A group of W warps
 // (fewer where bricks are many) owns its bricks in both phases of an iteration:
 //   step      x += alpha d, r -= alpha q, d = r + beta d, u = V d       (streaming)
 //   product   q = A d from the halo tile of u (swc_stencil.cuh), and the four dot
@@ -167,6 +168,7 @@ struct CgScalars {
     float threshold_h, threshold_l;
     int   it, max_iter;
 };
+constexpr int kCluster = 16;  // blocks of a cluster's solve, at most
 template<int WARPS> struct MeetSmem {
     F3        part[WARPS][kSums];
     F3        sum[kSums];
@@ -175,6 +177,12 @@ template<int WARPS> struct MeetSmem {
     int       full[kSums];
     Outcome   out;
     CgScalars cg;  // block 0
+};
+// A cluster's partials, by the meeting's parity: two meetings may have no other barrier
+// between them.
+template<int WARPS> struct ClusterSmem : MeetSmem<WARPS> {
+    F3     all[2][kCluster][kSums];
+    double all_start[kCluster][2];
 };
 // The power of two that brings |b|^2 to about 1.
 __device__ __forceinline__ float sum_scale(double bb) { return exp2f(float(-max(-120, min(120, ilogb(bb))))); }
@@ -214,7 +222,8 @@ __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums],
 }
 
 // Start state from |r|^2 and |b|^2 (Eigen's stopping rule: |r|^2 < max(tol, eps/|b|)^2
-// |b|^2, cap 2 N_v).  The outcome's alpha is the power of two that scales the sums.
+// |b|^2, cap 2 N_v), into *cg when given.  The outcome's alpha is the power of two that
+// scales the sums.
 __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, double rr, double bb, int nv,
                                                const CgStart & from) {
     const int cap = from.max_iterations >= 0 ? from.max_iterations : 2 * nv;
@@ -230,16 +239,18 @@ __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, dou
         done      = rr < threshold ? 1 : (rr != rr ? 3 : 0);
         if (done == 0 && cap <= 0) done = 2;
     }
-    cg->start     = 0;
-    cg->bb        = bb;
-    cg->rr        = rr;
-    cg->rr0       = rr;
-    cg->rr_prev   = 0;
-    cg->pq        = 0;
-    cg->iter      = 0;
-    cg->max_iter  = cap;
-    cg->threshold = threshold;
-    cg->done      = done;
+    if (cg) {
+        cg->start     = 0;
+        cg->bb        = bb;
+        cg->rr        = rr;
+        cg->rr0       = rr;
+        cg->rr_prev   = 0;
+        cg->pq        = 0;
+        cg->iter      = 0;
+        cg->max_iter  = cap;
+        cg->threshold = threshold;
+        cg->done      = done;
+    }
     const float scale = sum_scale(bb);
     c = scalars_of(rr, threshold, cap, scale);
     return Outcome{scale, 0.f, unsigned(done)};
@@ -356,6 +367,75 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
     return M.out;
 }
 
+// The cluster's barrier, with its blocks' writes before it visible after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// v to the same place in the shared memory of block `rank` of the cluster.
+__device__ __forceinline__ void cluster_put(float * p, int rank, float v) {
+    unsigned at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(unsigned(__cvta_generic_to_shared(p))), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_put(double * p, int rank, double v) {
+    unsigned at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(unsigned(__cvta_generic_to_shared(p))), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+// The meeting of a cluster: every block has all partials in its own shared memory and
+// decides for itself, in the same order on the same values.
+template<bool START, int WARPS, class Decide>
+__device__ __forceinline__ Outcome meet_cluster(const F3 & v, int active, unsigned & tag, ClusterSmem<WARPS> & M,
+                                                Decide decided) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, blocks = gridDim.x;
+    const int k = lane >> 3, w = lane & 7;
+    if (w == 0) M.part[warp][k] = v;
+    __syncthreads();
+    F3(&all)[kCluster][kSums] = M.all[tag & 1u];
+    if (warp == 0) {
+        F3 part{0.f, 0.f, 0.f};
+        for (int j = w; j < active; j += 8) part = f3_add(part, M.part[j][k]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) part = f3_add(part, f3_shfl(part, o));
+        for (int r = w; r < blocks; r += 8) {
+            if constexpr (START) {
+                if (k < 2) cluster_put(&M.all_start[blockIdx.x][k], r, f3_double(part));
+            } else {
+                F3 & to = all[blockIdx.x][k];
+                cluster_put(&to.h, r, part.h);
+                cluster_put(&to.m, r, part.m);
+                cluster_put(&to.l, r, part.l);
+            }
+        }
+    }
+    cluster_sync();
+    if (warp == 0) {
+        if constexpr (START) {
+            double s = 0;
+            for (int r = w; r < blocks; r += 8) s += M.all_start[r][k & 1];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (w == 0 && k < 2) M.start[k] = s;
+        } else {
+            F3 s{0.f, 0.f, 0.f};
+            for (int r = w; r < blocks; r += 8) s = f3_add(s, all[r][k]);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s = f3_add(s, f3_shfl(s, o));
+            if (w == 0) M.sum[k] = s;
+        }
+        __syncwarp();
+        if (!START || lane == 0) {
+            CgScalars c     = M.cg;
+            const Outcome o = decided(c);
+            __syncwarp(START ? 1u : 0xffffffffu);
+            if (lane == 0) M.cg = c, M.out = o;
+        }
+    }
+    __syncthreads();
+    tag++;
+    return M.out;
+}
+
 // A warp's wait for the flags of a brick's active neighbours (tab); false when they did
 // not come in time.
 __device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const int * tab, unsigned tag) {
@@ -380,12 +460,23 @@ __device__ __forceinline__ void to_host(const CgState * cg, CgState * host) {
     host->nbricks = cg->nbricks;
 }
 
-// Groups of W warps own the bricks c + P (g + COUNT k): the solve's loop.
-template<int DIM, int W>
+template<int DIM, bool CLUSTER>
+using MeetSmemOf = std::conditional_t<CLUSTER, ClusterSmem<WarpBrick<DIM>::WARPS>, MeetSmem<WarpBrick<DIM>::WARPS>>;
+// Dynamic shared memory of the tiles: a cluster uses the larger groups alone.
+template<int DIM, bool CLUSTER>
+constexpr size_t kSolveTiles = CLUSTER ? sizeof(float) * WarpBrick<DIM>::T::TILE * (WarpBrick<DIM>::WARPS / WarpBrick<DIM>::WMAX)
+                                       : WarpBrick<DIM>::kTileBytes;
+template<int DIM, bool CLUSTER>
+constexpr size_t kSolveSmem = WarpBrick<DIM>::kSmem - WarpBrick<DIM>::kTileBytes + kSolveTiles<DIM, CLUSTER>;
+
+// Groups of W warps own the bricks c + P (g + COUNT k): the solve's loop.  CLUSTER: the
+// grid is one cluster, whose barrier and shared memory take the place of the flags and the
+// slots.
+template<int DIM, int W, bool CLUSTER>
 __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict__ blist, int nb, int P,
                                       const unsigned char * __restrict__ bflag, const NodeArrays & N, const Stencil & S,
                                       CgState * cg, const CgStart & from, ulonglong2 * slots, unsigned * flags,
-                                      CgPhases * phases, CgState * host, MeetSmem<WarpBrick<DIM>::WARPS> & M) {
+                                      CgPhases * phases, CgState * host, MeetSmemOf<DIM, CLUSTER> & M) {
     using B  = WarpBrick<DIM>;
     using G  = typename B::G;
     using Gr = Group<DIM, W>;
@@ -393,8 +484,8 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     const int grp = Gr::index(), gl = Gr::lane();
     const bool idle  = grp >= Gr::COUNT;
     float * tile     = reinterpret_cast<float *>(smem) + B::T::TILE * grp;
-    int * tab        = reinterpret_cast<int *>(smem + B::kTileBytes) + 27 * (B::TABS + 1) * grp;
-    unsigned * seg   = reinterpret_cast<unsigned *>(smem + B::kTileBytes + B::kTabBytes);
+    int * tab        = reinterpret_cast<int *>(smem + kSolveTiles<DIM, CLUSTER>) + 27 * (B::TABS + 1) * grp;
+    unsigned * seg   = reinterpret_cast<unsigned *>(smem + kSolveTiles<DIM, CLUSTER> + B::kTabBytes);
     const int bfirst = idle ? nb : int(blockIdx.x) + P * grp, bstep = P * Gr::COUNT;
     constexpr int Q  = G::BN / 4 / Gr::NT;  // float4 per thread of a brick
     fill_segments<DIM>(seg);
@@ -422,7 +513,8 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     };
     // u is there: the bricks' flags
     auto publish = [&]() {
-        if (!idle) {
+        if constexpr (CLUSTER) cluster_sync();
+        else if (!idle) {
             Gr::sync();
             if (gl == 0) {
                 fence_gpu();
@@ -440,7 +532,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 fill_neighbours<DIM>(L, bflag, b, gl, t);
                 __syncwarp();
             }
-            if (gl < 32 && !wait_neighbours(flags, t, tag)) ok = false;
+            if (!CLUSTER && gl < 32 && !wait_neighbours(flags, t, tag)) ok = false;
             Gr::sync();  // also past the last brick's reads of the tile
             tile_copy<DIM, W>(seg, t, N.u, tile);
             const long long base = (long long) b * G::BN;
@@ -494,6 +586,11 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
             }
         }
     };
+    auto meeting = [&](auto start, const F3 & v, auto decided) {
+        constexpr bool START = decltype(start)::value;
+        if constexpr (CLUSTER) return meet_cluster<START, B::WARPS>(v, active, tag, M, decided);
+        else return meet<START, B::WARPS>(v, slots, gridDim.x, P, active, tag, M, decided);
+    };
     if (from.own) {
         for (int bi = bfirst; bi < nb; bi += bstep) {
             const long long base = (long long) blist[bi] * G::BN + 4 * gl;
@@ -506,8 +603,8 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
         publish();
         FF part[kSums] = {};
         product(std::true_type{}, part);
-        o = meet<true>(warp_sum4(part, 1.f), slots, gridDim.x, P, active, tag, M, [&](CgScalars & c) {
-            return decide_start(cg, c, M.start[0], M.start[1], M.nv, from);
+        o = meeting(std::true_type{}, warp_sum4(part, 1.f), [&](CgScalars & c) {
+            return decide_start(blockIdx.x == 0 ? cg : nullptr, c, M.start[0], M.start[1], M.nv, from);
         });
         scale = o.alpha;
         mark  = phases ? global_ns() : 0;
@@ -539,7 +636,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
         FF part[kSums] = {};
         product(std::false_type{}, part);
         lap(spent.product);
-        o = meet<false>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, [&](CgScalars & c) {
+        o = meeting(std::false_type{}, warp_sum4(part, scale), [&](CgScalars & c) {
             const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
             return decide(c, sum, 0.f, false);
         });
@@ -557,7 +654,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 }
             }
             const float alpha = o.alpha;
-            o = meet<false>(warp_sum4(part, scale), slots, gridDim.x, P, active, tag, M, [&](CgScalars & c) {
+            o = meeting(std::false_type{}, warp_sum4(part, scale), [&](CgScalars & c) {
                 const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
                 return decide(c, sum, alpha, true);
             });
@@ -608,16 +705,18 @@ template<int DIM> __device__ __forceinline__ bool few_bricks(int nb, int blocks)
 
 }  // namespace
 
-template<int DIM>
+template<int DIM, bool CLUSTER>
 __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
     k_cg_solve(Lattice L, const int * __restrict__ blist, const int * __restrict__ bcount,
                const unsigned char * __restrict__ bflag, NodeArrays N, Stencil S, CgState * cg, CgStart from,
                ulonglong2 * slots, unsigned * flags, CgPhases * phases, CgState * host) {
+    if constexpr (CLUSTER) pdl_wait_and_release();
     using B = WarpBrick<DIM>;
     constexpr int Q = B::G::BN / 4;
-    __shared__ MeetSmem<B::WARPS> M;
+    __shared__ MeetSmemOf<DIM, CLUSTER> M;
     const int nb   = *bcount;
     const int done = from.own ? 0 : cg->done;
+    if (CLUSTER && threadIdx.x == 0) M.nv = *from.nv;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         M.nv        = *from.nv;
         cg->nv      = M.nv;
@@ -636,11 +735,16 @@ __global__ void __launch_bounds__(WarpBrick<DIM>::NT, 1)
                 st4(N.x, (long long) blist[e / Q] * B::G::BN + 4 * (e % Q), make_float4(0.f, 0.f, 0.f, 0.f));
         return;
     }
-    const int P = min(int(gridDim.x), nb);
-    if (int(blockIdx.x) >= P) return;
-    if (few_bricks<DIM>(nb, gridDim.x))
-        solve<DIM, B::WMAX>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, host, M);
-    else solve<DIM, B::WMIN>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, host, M);
+    if constexpr (CLUSTER) {
+        if (nb == 0) return;
+        solve<DIM, B::WMAX, true>(L, blist, nb, int(gridDim.x), bflag, N, S, cg, from, slots, flags, phases, host, M);
+    } else {
+        const int P = min(int(gridDim.x), nb);
+        if (int(blockIdx.x) >= P) return;
+        if (few_bricks<DIM>(nb, gridDim.x))
+            solve<DIM, B::WMAX, false>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, host, M);
+        else solve<DIM, B::WMIN, false>(L, blist, nb, P, bflag, N, S, cg, from, slots, flags, phases, host, M);
+    }
 }
 
 // Row-stencil passes outside the iteration, the bricks strided over the warps of a
@@ -785,7 +889,7 @@ template<int DIM> int cg_solve_prepare() {
     auto set = [bytes](auto kernel) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
-    return set(k_cg_solve<DIM>) && set(k_rows_tiled<DIM, kRowsAhat>) && set(k_rows_tiled<DIM, kRowsResid>) &&
+    return set(k_cg_solve<DIM, false>) && set(k_rows_tiled<DIM, kRowsAhat>) && set(k_rows_tiled<DIM, kRowsResid>) &&
                    set(k_rows_tiled<DIM, kRowsDiag>)
                ? 0
                : -1;
@@ -816,23 +920,56 @@ void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeAr
     launch_pdl(k_rows_tiled<DIM, kRowsResid>, blocks, W::NT, W::kSmem, st, L, 0.f, B.list, B.count, B.flag, N, S, N.u, x,
                r, d, sums, partials, &cg->ticket[0], nullptr);
 }
+template<int DIM> int cg_cluster_blocks() {
+    auto kernel = k_cg_solve<DIM, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmem<DIM, true>)) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (int blocks = kCluster; blocks >= 8; blocks /= 2) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at[1];
+        cfg.gridDim          = blocks;
+        cfg.blockDim         = WarpBrick<DIM>::NT;
+        cfg.dynamicSmemBytes = kSolveSmem<DIM, true>;
+        at[0].id               = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = blocks;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs    = at;
+        cfg.numAttrs = 1;
+        int n        = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) return blocks;
+        cudaGetLastError();
+    }
+    return 0;
+}
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases,
-                    CgState * host, cudaStream_t st) {
+                    const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, int cluster,
+                    CgPhases * phases, CgState * host, cudaStream_t st) {
     using W = WarpBrick<DIM>;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = blocks;
+    cfg.gridDim          = cluster ? cluster : blocks;
     cfg.blockDim         = W::NT;
-    cfg.dynamicSmemBytes = W::kSmem;
+    cfg.dynamicSmemBytes = cluster ? kSolveSmem<DIM, true> : W::kSmem;
     cfg.stream           = st;
-    cudaLaunchAttribute at[1];
-    at[0].id              = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
+    cudaLaunchAttribute at[2];
+    if (cluster) {
+        at[0].id               = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at[1].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+    } else {
+        at[0].id              = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
     cfg.attrs    = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_cg_solve<DIM>, L, (const int *) B.list, (const int *) B.count,
-                              (const unsigned char *) B.flag, N, S, cg, from, slots, flags, phases, host) == cudaSuccess
+    cfg.numAttrs = cluster ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, cluster ? k_cg_solve<DIM, true> : k_cg_solve<DIM, false>, L, (const int *) B.list,
+                              (const int *) B.count, (const unsigned char *) B.flag, N, S, cg, from, slots, flags, phases,
+                              host) == cudaSuccess
                ? 0
                : -1;
 }
@@ -847,8 +984,9 @@ int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays &
     template void launch_diag_max_f64<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,    \
                                          const StencilD &, unsigned int *, unsigned long long *, int, int,             \
                                          cudaStream_t);                                                                \
+    template int cg_cluster_blocks<D>();                                                                              \
     template int launch_cg_solve<D>(const Lattice &, const BrickArrays &, const NodeArrays &, const Stencil &,         \
-                                    CgState *, const CgStart &, ulonglong2 *, unsigned *, int, CgPhases *,             \
+                                    CgState *, const CgStart &, ulonglong2 *, unsigned *, int, int, CgPhases *,        \
                                     CgState *, cudaStream_t);
 SWC_INST(2)
 SWC_INST(3)

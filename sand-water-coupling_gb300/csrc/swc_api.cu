@@ -55,6 +55,7 @@ struct swc_ctx {
     StencilD        SD{};
     int             grid  = 1;  // grid of the 256-thread brick / streaming kernels
     int             cgrid = 1;  // grid of the CG solve and the warp-per-brick row passes (one block per SM)
+    int             ccluster = 0;  // or one cluster of so many blocks for the solve
     int             rgrid = 1;  // grid of the block-per-brick row kernels (true residual, operator)
     int             ggrid = 1;  // resident grid of the virtual gather (brick queue)
     int             pgrid = 1;  // resident grid of the pressure gradient (brick queue)
@@ -330,8 +331,8 @@ template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features =
 template<int DIM> int queue_cg(swc_ctx * c, bool started) {
     const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg};
     c->hcg->st.failed = 0;
-    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, nullptr, &c->hcg->st,
-                             c->stream)) {
+    if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, nullptr,
+                             &c->hcg->st, c->stream)) {
         c->err = std::string("CG solve: ") + cudaGetErrorString(cudaGetLastError());
         return SWC_CUDA_ERROR;
     }
@@ -739,6 +740,13 @@ int swc_create(const swc_scene * s, const swc_solver_opts * o, swc_ctx ** out) {
         delete c;
         return SWC_CUDA_ERROR;
     }
+    // One cluster of 16 blocks for the solve of few bricks: its barrier and shared memory
+    // instead of words in L2.  An iteration in a cluster and over all SMs takes 4.0 and 5.5 us
+    // at 18 bricks (lattice 49), 4.6 and 5.9 at 25, 5.6 and 5.9 at 81, 6.0 and 6.4 at 100, 6.5
+    // and 6.6 at 121, 7.7 and 6.7 at 169 in 2D; 7.1 and 8.9 at 8, 8.3 and 8.5 at 27, 11.4 and
+    // 8.6 at 64 in 3D.
+    if (L.nbricks <= (s->dim == 3 ? 27 : 100))
+        c->ccluster = s->dim == 3 ? cg_cluster_blocks<3>() : cg_cluster_blocks<2>();
     const size_t npart = 3 * size_t(std::max({c->grid, c->cgrid, c->rgrid})) + 8;
     setup_phys(c);
     int rc = SWC_OK;
@@ -1365,7 +1373,8 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         for (int k = 0; k < 2; k++) {  // warm, then timed
             const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg};
             auto go = [&](auto run) {
-                run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->phases, nullptr, c->stream);
+                run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, c->phases, nullptr,
+                    c->stream);
             };
             if (c->dim == 3) go(launch_cg_solve<3>);
             else go(launch_cg_solve<2>);

@@ -168,12 +168,15 @@ void launch_compact_export(const Lattice & L, const BrickArrays & B, const NodeA
 // meeting slots and the bricks' flags.
 // A failed launch returns nonzero; a wait that times out sets cg->failed.  The outcome goes
 // to `host` (pinned memory, or null) as well, there once the stream was waited for.
+// With `cluster` the solve is that many blocks of one cluster instead (cg_cluster_blocks(),
+// 0 where the device has no room for one), for lattices of few bricks.
 // cg_solve_prepare sets the kernels' shared-memory attribute on the current device.
 template<int DIM> int cg_solve_prepare();
+template<int DIM> int cg_cluster_blocks();
 template<int DIM>
 int launch_cg_solve(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S, CgState * cg,
-                    const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, CgPhases * phases,
-                    CgState * host, cudaStream_t st);
+                    const CgStart & from, ulonglong2 * slots, unsigned * flags, int blocks, int cluster,
+                    CgPhases * phases, CgState * host, cudaStream_t st);
 template<int DIM>
 void launch_rows_residual(const Lattice & L, const BrickArrays & B, const NodeArrays & N, const Stencil & S,
                           const float * x, float * r, float * d, double * sums, CgState * cg, double * partials,

@@ -19,11 +19,12 @@ def bricks_3d(n):
     return scenes.projection_block_3d(n=n, seed=n)
 
 
-# active bricks on 152 SMs: one; a few; 3D up to 3 per block in groups of four warps and
+# active bricks on 152 SMs: one and a few (one cluster, lattices of up to 100 bricks or 27 in
+# 3D); more; 3D up to 3 per block in groups of four warps and
 # past that in groups of two, with one more than a whole round; 2D up to 8 per block in
 # groups of two warps and past that single warps
 @pytest.mark.parametrize("build,n,low,high", [
-    (bricks_2d, 9, 1, 4), (bricks_2d, 121, 60, 100), (bricks_2d, 601, 1217, 1700),
+    (bricks_2d, 9, 1, 4), (bricks_2d, 121, 60, 100), (bricks_2d, 170, 101, 144), (bricks_2d, 601, 1217, 1700),
     (bricks_3d, 9, 8, 8), (bricks_3d, 45, 305, 456), (bricks_3d, 52, 457, 608), (bricks_3d, 60, 609, 800), (bricks_3d, 96, 2129, 2500)])
 def test_solve_at_brick_counts(swc_mod, build, n, low, high):
     s = build(n).rounded_to_float32()
@@ -65,12 +66,13 @@ def test_small_systems_follow_the_oracle(swc_mod, oracle_mod, n, tol, cap):
         assert st["rel_residual"] == pytest.approx(o["rel_residual"], rel=1e-2)
 
 
-def test_residual_that_vanishes_in_one_step(swc_mod):
+@pytest.mark.parametrize("n", [9, 25])
+def test_residual_that_vanishes_in_one_step(swc_mod, n):
     """alpha0 a million times the largest diagonal: A is alpha0 times the identity but for
     rows of at most 1e-6 alpha0, so one step takes r down to 1e-6 of itself and its norm
     comes from r - alpha q itself, not from the cancelling sums.  Bound: the rows' 1e-6
     (within a factor 2 after the move) and two FP32 roundings of r."""
-    s = bricks_3d(9).rounded_to_float32()
+    s = bricks_3d(n).rounded_to_float32()
     liq = swc_mod.DualParticleSphLiquid(s, warm_start="zero", tolerance=1e-5, compute_true_residual=True)
     liq.initialize()
     sc = liq.scalars()
