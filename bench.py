@@ -70,10 +70,9 @@ def peaks():
 
 SM_MAX_MHZ = 2070.0
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the 128^3 block,
-# per active node of the captured launch: k_cg_spmv 32,769,792 B at 2,246,535 nodes,
-# k_node_gather 90,965,504 + 13,017,856 B and k_pressure_gradient 113,461,248 + 12,455,680 B
-# at 2,246,538 nodes (profiles/)
-DRAM_BYTES_PER_NODE = {"cg_spmv": 32769792 / 2246535, "virtual_gather": (90965504 + 13017856) / 2246538,
+# per active node of the captured launch: k_node_gather 90,965,504 + 13,017,856 B and
+# k_pressure_gradient 113,461,248 + 12,455,680 B at 2,246,538 nodes (profiles/)
+DRAM_BYTES_PER_NODE = {"virtual_gather": (90965504 + 13017856) / 2246538,
                        "pressure_gradient": (113461248 + 12455680) / 2246538}
 
 
@@ -315,7 +314,7 @@ def run_sand_leg(args, torch, stream, hbm, peak_kind, with_cpu):
     ms = e0.elapsed_time(e1)
     kern = {"contacts": g.timeKernel(0, 20), "binning": g.timeKernel(1, 20)}
     # algorithmic bytes: the contact pass reads pos, pos_lo, vel and writes vel (16 B each);
-    # the binning moves them (48 B in, 32 B out), writes key / rank, scatters, permutes
+    # the binning moves them (48 B in, 32 B out), writes key / rank, scatters, orders
     # pos, pos_lo, vel, id (52 B in and out)
     alg = {"contacts": 64 * n, "binning": (48 + 32 + 8) * n + (8 + 4) * n + (4 + 52 + 52) * n}
     dom = max(kern, key=kern.get)
@@ -363,7 +362,7 @@ def run_sand_leg(args, torch, stream, hbm, peak_kind, with_cpu):
                       "l2": "inputs larger than L2 (particle state 128 MB + sort scratch per step)"},
            "e2e": {"value": args.steps / (e2e_ms / 1e3), "unit": UNIT, "h2d_bytes_per_step": 2 * nbytes,
                    "d2h_bytes_per_step": 2 * nbytes},
-           "roofline": roof, "gpu_launches_per_step": 10}
+           "roofline": roof, "gpu_launches_per_step": 7}
     if with_cpu:
         out["cpu_baseline"] = sand_cpu_reference()
     return out
@@ -504,7 +503,8 @@ def run_gpu_arm(args):
     # dominant kernels timed live (CUDA events on the library stream)
     hbm, peak_kind = peaks()
     kern = {}
-    for which, name in ((6, "cg_direction"), (0, "cg_spmv"), (1, "cg_update"), (2, "virtual_gather"),
+    # (cg_*: the phases of an iteration of the resident solve, by its own clock)
+    for which, name in ((6, "cg_step"), (0, "cg_product"), (1, "cg_meeting"), (2, "virtual_gather"),
                         (3, "pressure_gradient"), (4, "density"), (5, "forces")):
         kern[name] = liq.timeKernel(which, 20)
     if args.warm_start.startswith("learned"):
@@ -512,18 +512,18 @@ def run_gpu_arm(args):
     n, nb = scene.n_particles, scene.n_boundary
     # algorithmic bytes per launch (each array touched once per pass)
     alg = {
-        "cg_direction": 20 * nv,  # reads d, r, V; writes d, u = V d
-        "cg_spmv": 16 * nv,  # reads u (halo tiles from L2), d, alpha_hat; writes q (FP32)
-        "cg_update": 24 * nv,  # reads x, r, d, q; writes x, r
+        "cg_step": 36 * nv,  # reads x, r, q, d, V; writes x, r, d, u = V d
+        "cg_product": 16 * nv,  # reads u (halo tiles from L2), d, alpha_hat; writes q (FP32)
+        "cg_meeting": 0,  # the blocks' sums: latency alone
         "virtual_gather": 32 * (n + nb) + 16 * nv,  # particle pos/vel once; V, D, rho, flag out
         "pressure_gradient": 32 * n + 8 * nv + 48 * nb,  # pos, vel r/w; V, p; boundary pos/vel/nrm
         "density": 16 * n + 4 * n + 4 * n,
         "forces": 32 * n + 16 * n,
         "mlp_forward": 32 * nv,  # per slot: flag, D, alpha_hat, n_real, p_base, p1, d2, rho read; p0 written
     }
-    cg_ms = kern["cg_direction"] + kern["cg_spmv"] + kern["cg_update"]
-    dominant = max(("cg_spmv", "virtual_gather", "pressure_gradient"),
-                   key=lambda k: kern[k] * (np.mean(iters) if k == "cg_spmv" else 1))
+    cg_ms = kern["cg_step"] + kern["cg_product"] + kern["cg_meeting"]
+    dominant = max(("cg_product", "virtual_gather", "pressure_gradient"),
+                   key=lambda k: kern[k] * (np.mean(iters) if k == "cg_product" else 1))
     ach = alg[dominant] / (kern[dominant] / 1e3) / 1e9
     # DRAM bytes (read + write) per active node of one launch, from the ncu captures of
     # the same workload summarised in profiles/
@@ -544,12 +544,12 @@ def run_gpu_arm(args):
         roofline["fp32"] = {"achieved": flops / (kern["pressure_gradient"] / 1e3) / 1e12, "peak": fp32_peak,
                             "unit": "TFLOP/s", "peak_source": "nominal",
                             "frac": flops / (kern["pressure_gradient"] / 1e3) / 1e12 / fp32_peak}
-    if dominant == "cg_spmv":
+    if dominant == "cg_product":
         # the stencil's arithmetic against the FP32 FMA roof (nominal: SMs x 128 lanes x 2 x max clock)
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         fp32_peak = sms * 128 * 2 * SM_MAX_MHZ * 1e6 / 1e12
         flops = 2 * 250 * nv  # 250 off-diagonal taps per active row (the reference's per-row work)
-        roofline["fp32"] = {"achieved": flops / (kern["cg_spmv"] / 1e3) / 1e12, "peak": fp32_peak,
+        roofline["fp32"] = {"achieved": flops / (kern["cg_product"] / 1e3) / 1e12, "peak": fp32_peak,
                             "unit": "TFLOP/s", "peak_source": "nominal"}
 
     # end-to-end through the public API with pinned host buffers, on a fresh
@@ -623,7 +623,7 @@ def run_gpu_arm(args):
     # step (each array once per pass; FP32 state): binning 92 N, rho_i 20 N,
     # viscosity + gravity 48 N, node activation 12 per lattice node, the fused
     # gather 36 (N + N_b) + 16 N_v, alpha_hat 8 N_v, CG 52 N_v per iteration
-    # (SpMV + dot 16, x/r update 24, direction 12), the pressure gradient
+    # (product + dots 16, step of x, r, d and u 36), the pressure gradient
     # 48 N + 8 N_v + 36 N_b.  The network's 28 N_v on the steps it runs is left out.
     def step_bytes(cg_its):
         return (92 + 20 + 48 + 48) * n + 12 * scene.n_nodes + 36 * (n + nb) + (16 + 8 + 8) * nv + 36 * nb + \
@@ -646,17 +646,15 @@ def run_gpu_arm(args):
     if args.sand:
         sand = run_sand_leg(args, torch, stream, hbm, peak_kind, with_cpu=rank == 0 and ws == 1 and not args.no_cpu)
 
-    # kernels launched per step (counted in the ncu launch list of this workload):
-    # binning 7 (count, three scan passes, scatter, segment sort, permute), density 2,
-    # viscosity 2, virtual generation 8 (brick marking, two brick lists, gather, segment
-    # count and its three scan passes), alpha_hat 1, warm start 1, CG start 3, 3 per CG
-    # iteration, gradient 1; a step that evaluates the network adds 4 more (not counted
-    # here, so this is a lower bound)
-    launches_per_step = 25 + 3 * float(np.mean(iters))
+    # kernels launched per step of the base start: binning 5 (count, two scan passes,
+    # scatter, order), density 2, viscosity 2, virtual generation 5 (brick marking, brick
+    # lists, gather, two scan passes), alpha_hat 1, warm start 1, the solve 1, gradient 1; a
+    # step that evaluates the network adds 7 more (not counted here, so this is a lower bound)
+    launches_per_step = 18
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
-                "scaling": "weak", "vs_baseline": None, "dtype": "f32 (FP64 CG reductions)",
+                "scaling": "weak", "vs_baseline": None, "dtype": "f32 (CG sums in triple FP32)",
                 "data": "synthetic (seeded)", "config": workload_config(args),
                 "wall_s_timed": wall, "cg_iterations_mean": float(np.mean(iters)), "n_virtual": nv,
                 "phases_ms": phases, "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,

@@ -259,9 +259,10 @@ __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, dou
 // Meeting of the blocks in use: v (value lane / 8 of the warp, as warp_sum4 gives it)
 // summed over their first `active` warps, and what block 0 decides on the sums, the
 // same on every thread.  Every block publishes its four partials under the meeting's
-// tag; block 0 reads them all and publishes the outcome, one word that the others poll.  (With every block polling every slot the polls themselves, 64 B x
-// blocks^2 a round, kept the slots from being written: 13 us a meeting of 152 blocks;
-// with the sums published and FP64 quotients formed by every thread, 5 us.)  One set of
+// tag; block 0 reads them all and publishes the outcome, one word that the others poll.
+// (With every block polling every slot the polls themselves, 64 B x blocks^2 a round, kept
+// the slots from being written: 13 us a meeting of 152 blocks; with the sums published and
+// FP64 quotients formed by every thread, 5 us.)  One set of
 // slots serves: a block publishes again only after it has the outcome, and block 0
 // only after every block has published again.
 // START: values 0 and 1 are |r|^2 and |b|^2, unscaled, in FP64 above the block (once a

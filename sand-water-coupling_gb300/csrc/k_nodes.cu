@@ -1,16 +1,13 @@
 // k_nodes.cu -- virtual-node (lattice) kernels of the dual-particle SPH
-// projection: active-brick list, the fused virtual gather (weight, rho_I, V_I,
-// vbar_I, D_I in one pass), reference-order compaction, the clamped diagonal
-// alpha_hat, warm starts and the matrix-free CG (stencil SpMV fused with the
-// search-direction update, and the x/r update), all with deterministic
-// FP64 reductions.
+// projection: brick lists, the fused virtual gather (weight, rho_I, V_I, vbar_I, D_I and
+// the row counts of the reference-order compaction in one pass), warm starts, exports and
+// the pressure gradient.
 #include <type_traits>
 
 #include "swc_kernels.h"
 #include "swc_tiles.cuh"
 
 namespace swc {
-
 
 // ---------------------------------------------------------------------------
 // Lists of the flagged bricks, ascending (a block each; 16 flags a thread at a time).

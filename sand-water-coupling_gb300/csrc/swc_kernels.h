@@ -90,7 +90,8 @@ template<int DIM>
 void launch_bin(const Lattice & L, long long n, float4 *& pos, float4 *& vel, float4 *& aux, int *& id, SortScratch & S,
                 int * cellStart, float advect_dt, cudaStream_t st, float advect_dt_lo = 0.f, bool aux_lo = false,
                 const Lattice * Ld = nullptr);
-// Density and forces run one thread per pair of consecutive sorted particles;
+// Density and forces run one thread (or several lanes, by n) per pair of consecutive sorted
+// particles; with one,
 // `left` (n/2 + 3 ints, zeroed once at allocation) collects the pairs that are
 // not in one cell row for a second, single-particle pass.
 template<int DIM>
