@@ -16,7 +16,9 @@
 // and the stopping test without a second trip: the sums hold 44 bits and more, the
 // quotient of two successive norms is seldom below a tenth, and where it is below
 // 1e-6 the norm is summed from r - alpha q itself.  r.r is summed from r in every
-// iteration, so nothing of a prediction is carried on.
+// iteration, so nothing of a prediction is carried on.  The sums with q take it times a
+// power of two near 1 / |A| (CgStart::qscale), so that all four are of the size of r.r and
+// their FP32 products hold over the same range of lengths and velocities as r.r itself.
 // Before a warp copies a tile it waits for the flags of the brick's neighbours; the
 // blocks meet once per iteration, for the sums, and each decides by itself whether to
 // go on, with no host check.  Dot products use exact FP32 products in float-float per
@@ -166,6 +168,7 @@ constexpr int kMeetPolls = 1 << 20;
 struct CgScalars {
     F3    pq, rr, rr_next;
     float threshold_h, threshold_l;
+    float qscale;  // of q in the sums
     int   it, max_iter;
 };
 constexpr int kCluster = 16;  // blocks of a cluster's solve, at most
@@ -186,14 +189,14 @@ template<int WARPS> struct ClusterSmem : MeetSmem<WARPS> {
 };
 // The power of two that brings |b|^2 to about 1.
 __device__ __forceinline__ float sum_scale(double bb) { return exp2f(float(-max(-120, min(120, ilogb(bb))))); }
-__device__ __forceinline__ CgScalars scalars_of(double rr, double threshold, int max_iter, float scale) {
+__device__ __forceinline__ CgScalars scalars_of(double rr, double threshold, int max_iter, float scale, float qscale) {
     const F3 r = f3_of(rr * double(scale)), t = f3_of(threshold * double(scale));
-    return CgScalars{F3{0.f, 0.f, 0.f}, r, r, t.h, t.m, 0, max_iter};
+    return CgScalars{F3{0.f, 0.f, 0.f}, r, r, t.h, t.m, qscale, 0, max_iter};
 }
 constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer blocks poll one line
 
-// The factors and the stopping test from the sums d.q, r.q, q.q, r.r (after kMeasure:
-// from |r - alpha q|^2).
+// The factors and the stopping test from the sums d.q, r.q, q.q, r.r, q times c.qscale
+// (after kMeasure: from |r - alpha q|^2).
 __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums], float alpha, bool measured) {
     Outcome o{alpha, 0.f, kGoOn};
     if (!measured) {
@@ -204,9 +207,10 @@ __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums],
             o.code = 3;
             return o;
         }
-        o.alpha   = f3_quotient(c.rr, c.pq);
-        const F3 t = f3_add(f3_scale(sum[2], o.alpha), f3_scale(sum[1], -2.f));
-        c.rr_next  = f3_add(c.rr, f3_scale(t, o.alpha));
+        const float a = f3_quotient(c.rr, c.pq);  // alpha / qscale
+        o.alpha       = a * c.qscale;
+        const F3 t    = f3_add(f3_scale(sum[2], a), f3_scale(sum[1], -2.f));
+        c.rr_next     = f3_add(c.rr, f3_scale(t, a));
         if (c.rr_next.h < 1e-6f * c.rr.h) {
             o.code = kMeasure;  // nearly all of r goes: its norm from r - alpha q itself
             return o;
@@ -252,7 +256,7 @@ __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, dou
         cg->done      = done;
     }
     const float scale = sum_scale(bb);
-    c = scalars_of(rr, threshold, cap, scale);
+    c = scalars_of(rr, threshold, cap, scale, from.qscale);
     return Outcome{scale, 0.f, unsigned(done)};
 }
 
@@ -495,7 +499,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     float scale = 1.f;
     if (!from.own) {
         scale = sum_scale(cg->bb);
-        if (threadIdx.x == 0) M.cg = scalars_of(cg->rr, cg->threshold, cg->max_iter, scale);
+        if (threadIdx.x == 0) M.cg = scalars_of(cg->rr, cg->threshold, cg->max_iter, scale, from.qscale);
     }
     __syncthreads();
     const int active = W * min(Gr::COUNT, (nb - int(blockIdx.x) + P - 1) / P);  // warps with bricks
@@ -577,9 +581,10 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 } else {
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        ff_add_prod(part[0], comp(d, j), p[j]);
-                        ff_add_prod(part[1], comp(r, j), p[j]);
-                        ff_add_prod(part[2], p[j], p[j]);
+                        const float qs = p[j] * from.qscale;
+                        ff_add_prod(part[0], comp(d, j), qs);
+                        ff_add_prod(part[1], comp(r, j), qs);
+                        ff_add_prod(part[2], qs, qs);
                         ff_add_prod(part[3], comp(r, j), comp(r, j));
                     }
                     st4(N.q, s, make_float4(p[0], p[1], p[2], p[3]));
@@ -680,7 +685,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
             if (started) {
                 cg->rr      = f3_double(M.cg.rr_next) / double(scale);
                 cg->rr_prev = f3_double(M.cg.rr) / double(scale);
-                cg->pq      = f3_double(M.cg.pq) / double(scale);
+                cg->pq      = f3_double(M.cg.pq) / (double(scale) * double(from.qscale));
                 cg->iter    = M.cg.it;
                 if (o.code != kFailed) cg->done = int(o.code);
             }

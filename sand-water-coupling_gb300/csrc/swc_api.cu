@@ -326,10 +326,24 @@ template<int DIM> void run_generate(swc_ctx * c, bool with_ahat, bool features =
     if (with_ahat) launch_ahat<DIM>(c->L, c->P, c->B, c->N, c->S, c->cgrid, c->stream);
 }
 
+// The power of two next to 1 / |A|, |A| from alpha0 and the diagonal -sum_k c(k) V of a node
+// amid nodes of V = spacing^dim (exact in the products that it scales).
+float operator_scale(const swc_ctx * c) {
+    double diag = 0;
+    const int zr = c->dim == 3 ? 3 : 0;
+    for (int z = -zr; z <= zr; z++)
+        for (int y = -3; y <= 3; y++)
+            for (int x = -3; x <= 3; x++)
+                if (const int r2 = x * x + y * y + z * z; r2 < 16) diag -= c->SD.c[r2];
+    diag = std::max(diag * std::pow(c->scene.grid_spacing, c->dim), c->alpha0);
+    return std::isfinite(diag) && diag > 0 ? float(std::ldexp(1.0, -std::clamp(std::ilogb(diag), -100, 100))) : 1.f;
+}
+
 // Queues the CG solve from the warm start in N.x (with `started`, from the start state
 // that the caller queued).
 template<int DIM> int queue_cg(swc_ctx * c, bool started) {
-    const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg};
+    const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg,
+                       operator_scale(c)};
     c->hcg->st.failed = 0;
     if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, nullptr,
                              &c->hcg->st, c->stream)) {
@@ -1371,7 +1385,7 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
         CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
         for (int k = 0; k < 2; k++) {  // warm, then timed
-            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg};
+            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg, operator_scale(c)};
             auto go = [&](auto run) {
                 run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, c->phases, nullptr,
                     c->stream);

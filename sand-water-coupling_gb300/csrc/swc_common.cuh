@@ -542,6 +542,7 @@ struct CgStart {
     int         max_iterations;  // < 0: twice the active nodes
     int         own;
     const int * nv;              // device: active nodes
+    float       qscale;          // power of two near 1 / |A|, for the sums with q = A d
 };
 
 // Times of the solve's phases, summed over the iterations (ns, as the first warp of
