@@ -45,8 +45,9 @@ constexpr int kSums = 4;  // values of a meeting
 // Triple floats (three error-free terms, about 70 bits) hold the sums above the lane and
 // the scalars of the iteration.  GB300 adds or converts two FP64 values per SM and
 // clock, with a latency of 65 clocks and far more for a quotient: with FP64 here a meeting
-// took 7,100 clocks in a block alone.  The sums are scaled by the power of two that
-// brings |b|^2 to about 1, so they stay in the range of the FP32 products.
+// took 7,100 clocks in a block alone.  The sums are scaled by a power of two that brings
+// |b|^2, and later r.r when it has left 2^-48 .. 2^48 (decide), to about 1, so they stay in
+// the range of the FP32 products however far the solve goes.
 struct F3 {
     float h, m, l;
 };
@@ -134,16 +135,18 @@ enum : unsigned { kGoOn = 0, kFailed = 5, kMeasure = 6 };  // 1, 2, 3: CgState::
 struct Outcome {
     float    alpha, beta;
     unsigned code;
+    int      shift = 0;  // the sums' scale grows by 2^shift
 };
 __device__ __forceinline__ void outcome_put(ulonglong2 * p, const Outcome & o, unsigned tag) {
     word_put(p, (unsigned long long) __float_as_uint(o.beta) << 32 | __float_as_uint(o.alpha),
-             (unsigned long long) tag << 32 | o.code);
+             (unsigned long long) tag << 32 | unsigned(o.shift) << 8 | o.code);
 }
 __device__ __forceinline__ bool outcome_get(const ulonglong2 * p, unsigned tag, Outcome & o) {
     const ulonglong2 w = word_get(p);
     o.alpha            = __uint_as_float(unsigned(w.x));
     o.beta             = __uint_as_float(unsigned(w.x >> 32));
-    o.code             = unsigned(w.y);
+    o.code             = unsigned(w.y) & 0xffu;
+    o.shift            = int(unsigned(w.y)) >> 8;
     return unsigned(w.y >> 32) == tag;
 }
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned * p) {
@@ -164,12 +167,19 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Polls of one slot before a block gives up (about a second).
 constexpr int kMeetPolls = 1 << 20;
 
-// Block 0's view of the solve (scaled; the threshold as two floats).
+// Block 0's view of the solve (scaled; the threshold also as two floats).
 struct CgScalars {
-    F3    pq, rr, rr_next;
-    float threshold_h, threshold_l;
-    float qscale;  // of q in the sums
-    int   it, max_iter;
+    F3     pq, rr, rr_next;
+    float  threshold_h, threshold_l;
+    double threshold;
+    float  qscale;  // of q in the sums
+    int    it, max_iter;
+    __device__ __forceinline__ void set_threshold(double t) {
+        const F3 f  = f3_of(t);
+        threshold   = t;
+        threshold_h = f.h;
+        threshold_l = f.m;
+    }
 };
 constexpr int kCluster = 16;  // blocks of a cluster's solve, at most
 template<int WARPS> struct MeetSmem {
@@ -190,9 +200,14 @@ template<int WARPS> struct ClusterSmem : MeetSmem<WARPS> {
 // The power of two that brings |b|^2 to about 1.
 __device__ __forceinline__ float sum_scale(double bb) { return exp2f(float(-max(-120, min(120, ilogb(bb))))); }
 __device__ __forceinline__ CgScalars scalars_of(double rr, double threshold, int max_iter, float scale, float qscale) {
-    const F3 r = f3_of(rr * double(scale)), t = f3_of(threshold * double(scale));
-    return CgScalars{F3{0.f, 0.f, 0.f}, r, r, t.h, t.m, qscale, 0, max_iter};
+    const F3 r = f3_of(rr * double(scale));
+    CgScalars c{F3{0.f, 0.f, 0.f}, r, r, 0.f, 0.f, 0.0, qscale, 0, max_iter};
+    c.set_threshold(threshold * double(scale));
+    return c;
 }
+// 2^e, |e| <= 120
+__device__ __forceinline__ float pow2(int e) { return __int_as_float((127 + e) << 23); }
+constexpr int kRescale = 48;  // bits that r.r may move before the sums' scale follows it
 constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer blocks poll one line
 
 // The factors and the stopping test from the sums d.q, r.q, q.q, r.r, q times c.qscale
@@ -219,8 +234,16 @@ __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums],
     c.it++;
     const F3 & n = c.rr_next;
     if (n.h != n.h) o.code = 3;
-    else if (n.h < c.threshold_h || (n.h == c.threshold_h && n.m < c.threshold_l)) o.code = 1;
+    // (r = 0 is below any threshold, also one that the scale takes to 0 in FP32)
+    else if (!(n.h > 0.f) || n.h < c.threshold_h || (n.h == c.threshold_h && n.m < c.threshold_l)) o.code = 1;
     else if (c.it >= c.max_iter) o.code = 2;
+    else {
+        const int e = int(__float_as_uint(n.h) >> 23) - 127;
+        if (abs(e) > kRescale) {
+            o.shift = max(-120, min(120, -e));
+            c.set_threshold(c.threshold * double(pow2(o.shift)));
+        }
+    }
     o.beta = f3_quotient(n, c.rr);
     return o;
 }
@@ -665,6 +688,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 return decide(c, sum, alpha, true);
             });
         }
+        if (o.code == kGoOn && o.shift) scale *= pow2(o.shift);
         lap(spent.meeting);
     }
     if (!__syncthreads_and(ok)) o.code = kFailed;

@@ -63,3 +63,20 @@ def test_scale_of_velocity(swc_mod, dim, n, velocity):
         liq.close()
     assert out[0][:2] == out[1][:2]
     assert np.array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("dim,n", SIZES)
+@pytest.mark.parametrize("velocity", [1.0, 1e5, 1e7, 1e12])
+def test_tolerance_zero(swc_mod, dim, n, velocity):
+    """Tolerance 0 runs down to the rule's own floor, |r| < 2.2e-16, from any |b|: up to 31
+    decades below it.  x is at its FP32 limit long before (true residual below 2e-6 |b|, as at
+    the other tolerances), so p is that of the unscaled velocities to the same measure."""
+    s = block(dim, n, velocity=velocity)
+    liq = swc_mod.DualParticleSphLiquid(s, warm_start="zero", tolerance=0.0, max_iterations=1500,
+                                        compute_true_residual=True)
+    liq.initialize()
+    st = liq.project()
+    assert st["status"] == 0, st
+    assert st["rel_residual"] * st["rhs_norm"] < 2.3e-16
+    assert 0 < st["true_rel_residual"] < 2e-6, st
+    liq.close()
