@@ -266,6 +266,14 @@ int swc_mlp_gradient_noalloc(const float * params, const float * norm, const flo
  * cudaMalloc; a negative value disarms it.  Process-wide, meant for tests. */
 int swc_debug_fail_alloc(int64_t after);
 
+/* Test hook for the failure path of the CG solve (no counterpart in the reference): the
+ * number of polls after which a block of its resident kernel gives up waiting for the
+ * others (0: it looks once; negative: the default, about a second).  A solve in which a
+ * wait ran out returns SWC_CUDA_ERROR: the step's particles have moved and felt the
+ * forces, their velocities are not projected, and the next solve starts from zero.
+ * Lattices whose solve is one thread-block cluster (no such waits) never fail this way. */
+int swc_debug_wait_limit(swc_ctx * ctx, int32_t polls);
+
 /* Pinned host memory helpers for callers that stream state every step. */
 void * swc_host_alloc(size_t bytes);
 void   swc_host_free(void * p);

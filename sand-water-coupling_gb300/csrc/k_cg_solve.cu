@@ -164,9 +164,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return v;
 }
 
-// Polls of one slot before a block gives up (about a second).
-constexpr int kMeetPolls = 1 << 20;
-
 // Block 0's view of the solve (scaled; the threshold also as two floats).
 struct CgScalars {
     F3     pq, rr, rr_next;
@@ -293,10 +290,11 @@ __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, dou
 // slots serves: a block publishes again only after it has the outcome, and block 0
 // only after every block has published again.
 // START: values 0 and 1 are |r|^2 and |b|^2, unscaled, in FP64 above the block (once a
-// solve, by one warp each); `decided` makes the outcome of the sums.
+// solve, by one warp each); `decided` makes the outcome of the sums.  A wait ends after
+// `polls` more looks at its word, with kFailed.
 template<bool START, int WARPS, class Decide>
 __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int stride, int blocks, int active,
-                                        unsigned & tag, MeetSmem<WARPS> & M, Decide decided) {
+                                        int polls, unsigned & tag, MeetSmem<WARPS> & M, Decide decided) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ulonglong2 * outcome = slots + (long long) stride * kSums;
     if ((lane & 7) == 0) M.part[warp][lane >> 3] = v;
@@ -318,7 +316,7 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
             const ulonglong2 * p = outcome + blockIdx.x % kCopies;
             Outcome o;
             bool there = outcome_get(p, tag, o);
-            for (int n = 0; n < kMeetPolls && !there; n++) there = outcome_get(p, tag, o);
+            for (int n = 0; n < polls && !there; n++) there = outcome_get(p, tag, o);
             if (!there) o.code = kFailed;
             M.out = o;
         }
@@ -332,7 +330,7 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
                 for (int j = lane; j < blocks; j += 32) {
                     ulonglong2 w{0, 0};
                     bool there = false;
-                    for (int n = 0; n < kMeetPolls && !there; n++) {
+                    for (int n = 0; n <= polls && !there; n++) {
                         w     = word_get(slots + (long long) j * kSums + warp);
                         there = unsigned(w.y >> 32) == tag;
                     }
@@ -351,7 +349,7 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
             for (int j0 = lane; j0 < blocks; j0 += 32 * 5) {
                 F3 e[5];
                 bool there = false;
-                for (int n = 0; n < kMeetPolls && !there; n++) {
+                for (int n = 0; n <= polls && !there; n++) {
                     there = true;
 #pragma unroll
                     for (int q = 0; q < 5; q++) {
@@ -466,11 +464,11 @@ __device__ __forceinline__ Outcome meet_cluster(const F3 & v, int active, unsign
 
 // A warp's wait for the flags of a brick's active neighbours (tab); false when they did
 // not come in time.
-__device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const int * tab, unsigned tag) {
+__device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const int * tab, int polls, unsigned tag) {
     const int lane = threadIdx.x & 31;
     const int b    = lane < 27 ? tab[lane] : -1;
     bool there     = b < 0 || ld_relaxed(flags + b) == tag;
-    for (int n = 0; n < kMeetPolls && !there; n++) there = ld_relaxed(flags + b) == tag;
+    for (int n = 0; n < polls && !there; n++) there = ld_relaxed(flags + b) == tag;
     fence_gpu();
     return __all_sync(0xffffffffu, there);
 }
@@ -560,7 +558,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 fill_neighbours<DIM>(L, bflag, b, gl, t);
                 __syncwarp();
             }
-            if (!CLUSTER && gl < 32 && !wait_neighbours(flags, t, tag)) ok = false;
+            if (!CLUSTER && gl < 32 && !wait_neighbours(flags, t, from.polls, tag)) ok = false;
             Gr::sync();  // also past the last brick's reads of the tile
             tile_copy<DIM, W>(seg, t, N.u, tile);
             const long long base = (long long) b * G::BN;
@@ -618,7 +616,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
     auto meeting = [&](auto start, const F3 & v, auto decided) {
         constexpr bool START = decltype(start)::value;
         if constexpr (CLUSTER) return meet_cluster<START, B::WARPS>(v, active, tag, M, decided);
-        else return meet<START, B::WARPS>(v, slots, gridDim.x, P, active, tag, M, decided);
+        else return meet<START, B::WARPS>(v, slots, gridDim.x, P, active, from.polls, tag, M, decided);
     };
     if (from.own) {
         for (int bi = bfirst; bi < nb; bi += bstep) {

@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(kGradNT) k_pressure_gradient(Lattice L, Phys P
                                                            const CgState * __restrict__ cg, int parts, int * queue) {
     pdl_wait_and_release();
     using G = BrickGeom<DIM>;
-    if (cg->done == 3) return;  // the solve broke down: the velocities stay as they are
+    if (cg->done == 3 || cg->failed) return;  // no solution: the velocities stay as they are
     // Row pitch 24 in 3D: a warp's particles span about four consecutive cell
     // rows of one z-plane, whose 8-node windows then fall in disjoint banks
     // (24 dy mod 32 = 0, 24, 16, 8).

@@ -33,6 +33,7 @@ bool debug_alloc_should_fail() {
 namespace {
 
 constexpr int kPhases = 8;
+constexpr int kWaitPolls = 1 << 20;  // of the CG solve's blocks for one another (about a second)
 
 struct HostCg {
     CgState st;
@@ -126,6 +127,7 @@ struct swc_ctx {
     ulonglong2 *    slots  = nullptr;  // meeting slots of the CG solve (4 x (cgrid + 8))
     unsigned *      uflags = nullptr;  // and its per-brick flags
     CgPhases *      phases = nullptr;  // its phase times (swc_time_kernel)
+    int             polls  = kWaitPolls;
 
     bool   initialized = false;
     double rho0 = 0, alpha0 = -1e6, kappa = 0;
@@ -343,7 +345,7 @@ float operator_scale(const swc_ctx * c) {
 // that the caller queued).
 template<int DIM> int queue_cg(swc_ctx * c, bool started) {
     const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg,
-                       operator_scale(c)};
+                       operator_scale(c), c->polls};
     c->hcg->st.failed = 0;
     if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, nullptr,
                              &c->hcg->st, c->stream)) {
@@ -366,7 +368,6 @@ int cg_outcome(swc_ctx * c, swc_stats * st) {
     if (h.failed) {
         c->err = "CG solve: the blocks of the resident kernel did not meet in time";
         status = SWC_CUDA_ERROR;
-        cudaMemsetAsync(&c->cg->failed, 0, sizeof(int), c->stream);
     }
     if (st) {
         st->n_virtual            = h.nv;
@@ -506,9 +507,25 @@ template<int DIM> int queue_projection(swc_ctx * c, Projection & pr) {
     return SWC_OK;
 }
 
+// After a solve that gave up: its x, half made, starts nothing (no prefix, no history), and
+// the words of the meetings start afresh, since a block that was late may have left some
+// under the next solve's tags.
+int forget_solve(swc_ctx * c) {
+    c->extrap_steps   = 0;
+    c->extrap_shifted = false;
+    c->pcomp_stale    = false;
+    c->features_valid = false;
+    CK(cudaMemsetAsync(&c->cg->failed, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->slots, 0, sizeof(ulonglong2) * 4 * size_t(c->cgrid + 8), c->stream));
+    CK(cudaMemsetAsync(c->uflags, 0, sizeof(unsigned) * size_t(c->L.nbricks), c->stream));
+    CK(cudaMemsetAsync(c->nv_prev, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * size_t(c->L.nbricks) * (c->dim == 3 ? 512 : 256), c->stream));
+    return SWC_CUDA_ERROR;
+}
+
 int finish_projection(swc_ctx * c, swc_stats * st, const Projection & pr) {
     const int status = cg_outcome(c, st);
-    if (status == SWC_CUDA_ERROR) return status;
+    if (status == SWC_CUDA_ERROR) return forget_solve(c);
     int used = pr.used;
     if (pr.picked) {
         used = c->hcg->st.start == 0 ? SWC_WARM_LEARNED : pr.base_used;
@@ -1385,7 +1402,7 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
         CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
         for (int k = 0; k < 2; k++) {  // warm, then timed
-            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg, operator_scale(c)};
+            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg, operator_scale(c), c->polls};
             auto go = [&](auto run) {
                 run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, c->phases, nullptr,
                     c->stream);
@@ -1423,6 +1440,12 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         cudaFree(vel_save);
     }
     CK(cudaGetLastError());
+    return SWC_OK;
+}
+
+int swc_debug_wait_limit(swc_ctx * c, int32_t polls) {
+    if (!valid_ctx(c)) return SWC_BAD_ARG;
+    c->polls = polls < 0 ? kWaitPolls : polls;
     return SWC_OK;
 }
 

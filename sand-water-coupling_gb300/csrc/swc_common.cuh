@@ -543,6 +543,7 @@ struct CgStart {
     int         own;
     const int * nv;              // device: active nodes
     float       qscale;          // power of two near 1 / |A|, for the sums with q = A d
+    int         polls;           // looks at a word before a block gives up waiting for it
 };
 
 // Times of the solve's phases, summed over the iterations (ns, as the first warp of

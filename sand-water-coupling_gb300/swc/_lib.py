@@ -142,6 +142,7 @@ SIGNATURES = {
     "swc_mlp_gradient_noalloc": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p,
                                            C.c_void_p, C.c_void_p]),
     "swc_debug_fail_alloc": (C.c_int, [C.c_int64]),
+    "swc_debug_wait_limit": (C.c_int, [_P, C.c_int32]),
     "swc_host_alloc": (C.c_void_p, [C.c_size_t]),
     "swc_host_free": (None, [C.c_void_p]),
     # DEM sand step (include/swc_sand.h)
