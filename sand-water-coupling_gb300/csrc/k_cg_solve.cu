@@ -13,9 +13,12 @@
 // unless the caller queued a start of its own.  As three launches, with the sums in FP64
 // in every block, the start took 19 us at 15,625 particles, against 7 here.)
 // alpha = r.r / d.q, and |r - alpha q|^2 = r.r - 2 alpha r.q + alpha^2 q.q gives beta
-// and the stopping test without a second trip: the sums hold 44 bits and more, the
-// quotient of two successive norms is seldom below a tenth, and where it is below
-// 1e-6 the norm is summed from r - alpha q itself.  r.r is summed from r in every
+// without a second trip: the sums hold 44 bits and more, so at a quotient of two
+// successive norms of a tenth, below which it seldom is, the prediction is good to 2^-44
+// and at kPredict to 2^-40, where the rounding of the stored r alone makes 2^-31 (at 1e-6,
+// where the line lay first, 2^-28).  Below kPredict, and where the prediction ends the
+// solve, the norm is summed from r - alpha q itself: the stopping test and the residual
+// that is reported are of the r that is stored.  r.r is summed from r in every
 // iteration, so nothing of a prediction is carried on.  The sums with q take it times a
 // power of two near 1 / |A| (CgStart::qscale), so that all four are of the size of r.r and
 // their FP32 products hold over the same range of lengths and velocities as r.r itself.
@@ -204,6 +207,7 @@ __device__ __forceinline__ CgScalars scalars_of(double rr, double threshold, int
 }
 // 2^e, |e| <= 120
 __device__ __forceinline__ float pow2(int e) { return __int_as_float((127 + e) << 23); }
+constexpr float kPredict = 1.f / 128.f;  // of r.r: a smaller norm is measured, not predicted
 constexpr int kRescale = 48;  // bits that r.r may move before the sums' scale follows it
 constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer blocks poll one line
 
@@ -223,8 +227,10 @@ __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums],
         o.alpha       = a * c.qscale;
         const F3 t    = f3_add(f3_scale(sum[2], a), f3_scale(sum[1], -2.f));
         c.rr_next     = f3_add(c.rr, f3_scale(t, a));
-        if (c.rr_next.h < 1e-6f * c.rr.h) {
-            o.code = kMeasure;  // nearly all of r goes: its norm from r - alpha q itself
+        // (the margin over the threshold is far above the prediction's error)
+        if (!(c.rr_next.h > kPredict * c.rr.h) || !(c.rr_next.h > c.threshold_h * (1.f + 0x1p-16f)) ||
+            c.it + 1 >= c.max_iter) {
+            o.code = kMeasure;
             return o;
         }
     } else c.rr_next = sum[0];
