@@ -182,9 +182,10 @@ int swc_get_phase_times(swc_ctx * ctx, double * ms, int n);
 /* Times `reps` back-to-back launches of one kernel on the live state with CUDA
  * events (2: virtual gather, 3: pressure gradient, 4: density, 5: forces,
  * 7: learned warm-start forward pass, after a projection that used it), or the
- * phases of `reps` iterations of the CG solve (0: product with the wait for
- * neighbouring bricks, 1: meeting for the dot products, 6: step of x, r and d);
- * writes the mean ms per launch or iteration. */
+ * phases of `reps` iterations of the CG solve from zero, made whatever their sums
+ * say (0: product with the wait for neighbouring bricks, 1: meeting for the dot
+ * products, 6: step of x, r and d); writes the mean ms per launch or iteration.
+ * The state is left as it was. */
 int swc_time_kernel(swc_ctx * ctx, int which, int reps, double * mean_ms);
 
 /* ---- Learned CG warm start (no counterpart in the reference) -------------

@@ -213,8 +213,14 @@ constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer bloc
 
 // The factors and the stopping test from the sums d.q, r.q, q.q, r.r, q times c.qscale
 // (after kMeasure: from |r - alpha q|^2).
-__device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums], float alpha, bool measured) {
+__device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums], float alpha, bool measured,
+                                          bool timed) {
     Outcome o{alpha, 0.f, kGoOn};
+    if (timed) {
+        o.alpha = f3_quotient(sum[3], sum[0]) * c.qscale;
+        o.code  = ++c.it >= c.max_iter ? 2u : unsigned(kGoOn);
+        return o;
+    }
     if (!measured) {
         c.pq      = sum[0];
         c.rr      = sum[3];
@@ -269,6 +275,7 @@ __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, dou
         done      = rr < threshold ? 1 : (rr != rr ? 3 : 0);
         if (done == 0 && cap <= 0) done = 2;
     }
+    if (from.timed) done = 0;
     if (cg) {
         cg->start     = 0;
         cg->bb        = bb;
@@ -663,15 +670,16 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 st4(N.u, s, mul4(v, d));
             }
         }
+        if constexpr (CLUSTER) lap(spent.step);
         publish();
-        lap(spent.step);
+        if constexpr (!CLUSTER) lap(spent.step);
 
         FF part[kSums] = {};
         product(std::false_type{}, part);
         lap(spent.product);
         o = meeting(std::false_type{}, warp_sum4(part, scale), [&](CgScalars & c) {
             const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
-            return decide(c, sum, 0.f, false);
+            return decide(c, sum, 0.f, false, from.timed);
         });
         first = false;
         if (o.code == kMeasure) {
@@ -689,7 +697,7 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
             const float alpha = o.alpha;
             o = meeting(std::false_type{}, warp_sum4(part, scale), [&](CgScalars & c) {
                 const F3 sum[kSums] = {M.sum[0], M.sum[1], M.sum[2], M.sum[3]};
-                return decide(c, sum, alpha, true);
+                return decide(c, sum, alpha, true, false);
             });
         }
         if (o.code == kGoOn && o.shift) scale *= pow2(o.shift);

@@ -345,7 +345,7 @@ float operator_scale(const swc_ctx * c) {
 // that the caller queued).
 template<int DIM> int queue_cg(swc_ctx * c, bool started) {
     const CgStart from{c->opts.tolerance, c->opts.max_iterations, started ? 0 : 1, c->B.seg_off + c->B.nseg,
-                       operator_scale(c), c->polls};
+                       operator_scale(c), c->polls, 0};
     c->hcg->st.failed = 0;
     if (launch_cg_solve<DIM>(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, nullptr,
                              &c->hcg->st, c->stream)) {
@@ -507,17 +507,21 @@ template<int DIM> int queue_projection(swc_ctx * c, Projection & pr) {
     return SWC_OK;
 }
 
-// After a solve that gave up: its x, half made, starts nothing (no prefix, no history), and
-// the words of the meetings start afresh, since a block that was late may have left some
-// under the next solve's tags.
+// After a solve that gave up, the words of the meetings start afresh, since a block that was
+// late may have left some under the next solve's tags.
+int reset_meetings(swc_ctx * c) {
+    CK(cudaMemsetAsync(&c->cg->failed, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->slots, 0, sizeof(ulonglong2) * 4 * size_t(c->cgrid + 8), c->stream));
+    CK(cudaMemsetAsync(c->uflags, 0, sizeof(unsigned) * size_t(c->L.nbricks), c->stream));
+    return SWC_OK;
+}
+// And its x, half made, starts nothing: no prefix, no history.
 int forget_solve(swc_ctx * c) {
     c->extrap_steps   = 0;
     c->extrap_shifted = false;
     c->pcomp_stale    = false;
     c->features_valid = false;
-    CK(cudaMemsetAsync(&c->cg->failed, 0, sizeof(int), c->stream));
-    CK(cudaMemsetAsync(c->slots, 0, sizeof(ulonglong2) * 4 * size_t(c->cgrid + 8), c->stream));
-    CK(cudaMemsetAsync(c->uflags, 0, sizeof(unsigned) * size_t(c->L.nbricks), c->stream));
+    if (int rc = reset_meetings(c)) return rc;
     CK(cudaMemsetAsync(c->nv_prev, 0, sizeof(int), c->stream));
     CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * size_t(c->L.nbricks) * (c->dim == 3 ? 512 : 256), c->stream));
     return SWC_CUDA_ERROR;
@@ -1361,6 +1365,10 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
     }
     float4 * vel_save = nullptr;
     if (which == 3) {
+        // (of a solution that is there, whatever became of the last solve)
+        CgState run = saved;
+        run.done    = 0;
+        CK(cudaMemcpyAsync(c->cg, &run, sizeof(CgState), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMalloc(&vel_save, sizeof(float4) * std::max<long long>(c->n, 1)));
         cudaMemcpy(vel_save, c->vel, sizeof(float4) * c->n, cudaMemcpyDeviceToDevice);
     }
@@ -1396,25 +1404,26 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
             }
         }
     };
+    int failed = 0;
     if (solve) {
         // `reps` iterations of the resident solve from the last right-hand side and a zero
         // start, the phases' own times
-        CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
-        CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
-        for (int k = 0; k < 2; k++) {  // warm, then timed
-            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg, operator_scale(c), c->polls};
-            auto go = [&](auto run) {
-                run(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster, c->phases, nullptr,
-                    c->stream);
-            };
-            if (c->dim == 3) go(launch_cg_solve<3>);
-            else go(launch_cg_solve<2>);
-            CK(cudaStreamSynchronize(c->stream));
-        }
         CgPhases ph{};
         CgState run{};
-        CK(cudaMemcpy(&ph, c->phases, sizeof(ph), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(&run, c->cg, sizeof(run), cudaMemcpyDeviceToHost));
+        for (int k = 0; k < 2 && !failed; k++) {  // warm, then timed
+            CK(cudaMemsetAsync(c->phases, 0, sizeof(CgPhases), c->stream));
+            CK(cudaMemsetAsync(c->N.x, 0, sizeof(float) * slots, c->stream));
+            const CgStart from{0.0, reps, 1, c->B.seg_off + c->B.nseg, operator_scale(c), c->polls, 1};
+            auto go = [&](auto launch_solve) {
+                return launch_solve(c->L, c->B, c->N, c->S, c->cg, from, c->slots, c->uflags, c->cgrid, c->ccluster,
+                                    c->phases, nullptr, c->stream);
+            };
+            failed = c->dim == 3 ? go(launch_cg_solve<3>) : go(launch_cg_solve<2>);
+            CK(cudaStreamSynchronize(c->stream));
+            CK(cudaMemcpy(&ph, c->phases, sizeof(ph), cudaMemcpyDeviceToHost));
+            CK(cudaMemcpy(&run, c->cg, sizeof(run), cudaMemcpyDeviceToHost));
+            failed = failed || run.failed;
+        }
         saved.tick = run.tick;  // the meetings' tags are not used twice
         *mean_ms = 1e-6 * double(which == 0 ? ph.product : which == 1 ? ph.meeting : ph.step) / std::max(run.iter, 1);
     } else {
@@ -1428,8 +1437,12 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         *mean_ms = ms / reps;
     }
     CK(cudaMemcpy(c->cg, &saved, sizeof(CgState), cudaMemcpyHostToDevice));
+    if (failed) {
+        if (int rc = reset_meetings(c)) return rc;
+        CK(cudaStreamSynchronize(c->stream));
+    }
     // (the gather alone, without the scan that clears its rows' counts)
-    if (which == 2) CK(cudaMemset(c->B.seg, 0, sizeof(int) * c->B.nseg));
+    if (which == 2) CK(cudaMemsetAsync(c->B.seg, 0, sizeof(int) * c->B.nseg, c->stream));
     if (x_save) {
         cudaMemcpy(c->N.x, x_save, sizeof(float) * slots, cudaMemcpyDeviceToDevice);
         cudaMemcpy(c->N.r, x_save + slots, sizeof(float) * slots, cudaMemcpyDeviceToDevice);
@@ -1440,6 +1453,10 @@ int swc_time_kernel(swc_ctx * c, int which, int reps, double * mean_ms) {
         cudaFree(vel_save);
     }
     CK(cudaGetLastError());
+    if (failed) {
+        c->err = "CG solve: not launched, or its blocks did not meet in time";
+        return SWC_CUDA_ERROR;
+    }
     return SWC_OK;
 }
 

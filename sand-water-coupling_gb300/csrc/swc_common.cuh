@@ -544,11 +544,12 @@ struct CgStart {
     const int * nv;              // device: active nodes
     float       qscale;          // power of two near 1 / |A|, for the sums with q = A d
     int         polls;           // looks at a word before a block gives up waiting for it
+    int         timed;           // max_iterations iterations whatever the sums say (x is not wanted)
 };
 
 // Times of the solve's phases, summed over the iterations (ns, as the first warp of
 // block 0 saw them; written when asked for): the step of x, r, d and u, the product with
-// the wait for the neighbours' u, the meeting for the sums.
+// the wait for the neighbours' u (in a cluster, its barrier), the meeting for the sums.
 struct CgPhases {
     unsigned long long step, product, meeting;
 };
