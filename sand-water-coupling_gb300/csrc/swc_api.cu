@@ -553,7 +553,7 @@ int finish_projection(swc_ctx * c, swc_stats * st, const Projection & pr) {
     const bool solved = status == SWC_OK || status == SWC_CG_NOT_CONVERGED;
     c->extrap_steps   = pr.hist_on && c->extrap_shifted && solved ? c->extrap_steps + 1 : 0;
     c->extrap_shifted = false;
-    if (pr.logging && solved) c->features_valid = true;
+    if (pr.logging) c->features_valid = solved;  // (the targets of a solve that broke down are of no solution)
     if (st) st->warm_start_used = used;
     if (status == SWC_NAN_DETECTED) {
         // drop the poisoned warm start
@@ -607,7 +607,10 @@ template<int DIM> int do_advance(swc_ctx * c, double dt, swc_stats * st, bool mo
         std::swap(c->vel, c->vel2);
     }
     Projection pr;
-    if (int rc = queue_projection<DIM>(c, pr)) return rc;
+    if (int rc = queue_projection<DIM>(c, pr)) {
+        c->features_valid = false;
+        return rc;
+    }
     CK(cudaEventRecord(c->evB, c->stream));
     CK(cudaEventSynchronize(c->evB));
     const int status = finish_projection(c, st, pr);
