@@ -893,7 +893,8 @@ void launch_density(const float4 * pos, float4 * vel, float * rho, long long n, 
         launch_pdl(kernel, grid_for((n + 1) / 2 * S, 256, 1 << 20), 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass,
                    left);
     };
-    DIM == 3 && S == 8 ? go(k_density<DIM, 8>) : S == 4 ? go(k_density<DIM, 4>) : S == 2 ? go(k_density<DIM, 2>) : go(k_density<DIM, 1>);
+    if (DIM == 3 && S == 8) go(k_density<DIM, DIM == 3 ? 8 : 4>);
+    else S == 4 ? go(k_density<DIM, 4>) : S == 2 ? go(k_density<DIM, 2>) : go(k_density<DIM, 1>);
     if (S == 1) launch_pdl(k_density_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, rho, n, L, P, cellStart, P.mass, left);
 }
 void launch_set_volume(float4 * pos, const float * rho, long long n, float mass, cudaStream_t st) {
@@ -908,7 +909,8 @@ void launch_forces(const float4 * pos, const float4 * vel, float4 * vel_out, lon
         launch_pdl(kernel, grid_for((n + 1) / 2 * S, 256, 1 << 20), 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt,
                    left);
     };
-    DIM == 3 && S == 8 ? go(k_forces<DIM, 8>) : S == 4 ? go(k_forces<DIM, 4>) : S == 2 ? go(k_forces<DIM, 2>) : go(k_forces<DIM, 1>);
+    if (DIM == 3 && S == 8) go(k_forces<DIM, DIM == 3 ? 8 : 4>);
+    else S == 4 ? go(k_forces<DIM, 4>) : S == 2 ? go(k_forces<DIM, 2>) : go(k_forces<DIM, 1>);
     if (S == 1) launch_pdl(k_forces_left<DIM>, kLeftBlocks, 256, 0, st, pos, vel, vel_out, n, L, P, cellStart, dt, left);
 }
 template<int DIM>

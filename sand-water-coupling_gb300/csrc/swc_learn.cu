@@ -25,7 +25,7 @@ struct swc_trainer {
     cudaStream_t st = nullptr;
     float *feat = nullptr, *tgt = nullptr;                       // dataset
     float *params = nullptr, *norm = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;
-    float *bfeat = nullptr, *btgt = nullptr, *pred = nullptr;    // batch
+    float * pred  = nullptr;                                     // predictions of a batch
     float * fpred = nullptr;                                     // predictions of the whole dataset (epoch loss)
     double * part = nullptr;                                     // block sums of the epoch loss
     float *share = nullptr, *loss = nullptr;                     // per-CTA gradient shares, batch loss
@@ -79,8 +79,7 @@ int swc_trainer_create(int64_t capacity, int32_t batch, swc_trainer ** out) {
     bool ok = cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && talloc(&t->feat, size_t(capacity) * kIn) && talloc(&t->tgt, size_t(capacity)) && talloc(&t->params, kP) &&
          talloc(&t->norm, kN) && talloc(&t->m, kP) && talloc(&t->v, kP) && talloc(&t->grad, kP) &&
-         talloc(&t->bfeat, B * kIn) && talloc(&t->btgt, B) && talloc(&t->pred, B) &&
-         talloc(&t->share, mlp_train_share_floats(t->ctas)) && talloc(&t->loss, 1) &&
+         talloc(&t->pred, B) && talloc(&t->share, mlp_train_share_floats(t->ctas)) && talloc(&t->loss, 1) &&
          talloc(&t->part, kLossBlocks) && talloc(&t->err, 1);
     if (!ok) {
         swc_trainer_destroy(t);
@@ -97,8 +96,8 @@ int swc_trainer_create(int64_t capacity, int32_t batch, swc_trainer ** out) {
 void swc_trainer_destroy(swc_trainer * t) {
     if (!t) return;
     if (t->st) cudaStreamSynchronize(t->st);
-    for (float ** p : {&t->feat, &t->tgt, &t->params, &t->norm, &t->m, &t->v, &t->grad, &t->bfeat, &t->btgt, &t->pred,
-                       &t->fpred, &t->share, &t->loss})
+    for (float ** p : {&t->feat, &t->tgt, &t->params, &t->norm, &t->m, &t->v, &t->grad, &t->pred, &t->fpred,
+                       &t->share, &t->loss})
         tfree(*p);
     tfree(t->part);
     tfree(t->err);
@@ -218,9 +217,9 @@ int swc_mlp_gradient(const float * params, const float * norm, const float * f, 
         swc_trainer_destroy(t);
         return rc;
     }
-    cudaMemcpy(t->bfeat, f, sizeof(float) * kIn * n, cudaMemcpyHostToDevice);
-    cudaMemcpy(t->btgt, y, sizeof(float) * n, cudaMemcpyHostToDevice);
-    rc = gradient_batch(t, t->bfeat, t->btgt, n);
+    cudaMemcpy(t->feat, f, sizeof(float) * kIn * n, cudaMemcpyHostToDevice);
+    cudaMemcpy(t->tgt, y, sizeof(float) * n, cudaMemcpyHostToDevice);
+    rc = gradient_batch(t, t->feat, t->tgt, n);
     if (!rc) rc = check_err(t);
     if (!rc) {
         cudaMemcpy(grad, t->grad, sizeof(float) * kP, cudaMemcpyDeviceToHost);
