@@ -141,8 +141,6 @@ __global__ void k_cg_start(CgState * cg, const double * __restrict__ sums_l, con
     cg->bb      = sbb;
     cg->rr      = srr;
     cg->rr0     = srr;
-    cg->rr_prev = 0;
-    cg->pq      = 0;
     cg->iter    = 0;
     const int n  = *nv;
     cg->max_iter = max_iterations >= 0 ? max_iterations : 2 * n;

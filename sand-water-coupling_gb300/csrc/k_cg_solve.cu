@@ -19,9 +19,9 @@
 // where the line lay first, 2^-28).  Below kPredict, and where the prediction ends the
 // solve, the norm is summed from r - alpha q itself: the stopping test and the residual
 // that is reported are of the r that is stored.  r.r is summed from r in every
-// iteration, so nothing of a prediction is carried on.  The sums with q take it times a
-// power of two near 1 / |A| (CgStart::qscale), so that all four are of the size of r.r and
-// their FP32 products hold over the same range of lengths and velocities as r.r itself.
+// iteration, so nothing of a prediction is carried on.  q.q is summed times a power of two
+// near 1 / |A| (CgStart::qscale), so that its FP32 products hold over the range of lengths and
+// velocities that those of d.q do.
 // Before a warp copies a tile it waits for the flags of the brick's neighbours; the
 // blocks meet once per iteration, for the sums, and each decides by itself whether to
 // go on, with no host check.  Dot products use exact FP32 products in float-float per
@@ -167,20 +167,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return v;
 }
 
-// Block 0's view of the solve (scaled; the threshold also as two floats).
+// Block 0's view of the solve (scaled).
 struct CgScalars {
-    F3     pq, rr, rr_next;
-    float  threshold_h, threshold_l;
-    double threshold;
-    float  qscale;  // of q in the sums
-    int    it, max_iter;
-    __device__ __forceinline__ void set_threshold(double t) {
-        const F3 f  = f3_of(t);
-        threshold   = t;
-        threshold_h = f.h;
-        threshold_l = f.m;
-    }
+    F3    rr, rr_next;
+    float threshold_h, threshold_l;  // times 2^threshold_e
+    int   threshold_e;
+    float qinv;  // 1 / qscale
+    int   it, max_iter;
 };
+// 2^e, 0 where it is below the normal floats
+__device__ __forceinline__ float pow2(int e) { return __int_as_float(max(0, min(254, 127 + e)) << 23); }
 constexpr int kCluster = 16;  // blocks of a cluster's solve, at most
 template<int WARPS> struct MeetSmem {
     F3        part[WARPS][kSums];
@@ -201,56 +197,52 @@ template<int WARPS> struct ClusterSmem : MeetSmem<WARPS> {
 __device__ __forceinline__ float sum_scale(double bb) { return exp2f(float(-max(-120, min(120, ilogb(bb))))); }
 __device__ __forceinline__ CgScalars scalars_of(double rr, double threshold, int max_iter, float scale, float qscale) {
     const F3 r = f3_of(rr * double(scale));
-    CgScalars c{F3{0.f, 0.f, 0.f}, r, r, 0.f, 0.f, 0.0, qscale, 0, max_iter};
-    c.set_threshold(threshold * double(scale));
-    return c;
+    const int e = threshold > 0 ? ilogb(threshold) : 0;
+    const F3 t  = f3_of(scalbn(threshold, -e));
+    return CgScalars{r, r, t.h, t.m, e + ilogbf(scale), 1.f / qscale, 0, max_iter};
 }
-// 2^e, |e| <= 120
-__device__ __forceinline__ float pow2(int e) { return __int_as_float((127 + e) << 23); }
 constexpr float kPredict = 1.f / 128.f;  // of r.r: a smaller norm is measured, not predicted
-constexpr int kRescale = 48;  // bits that r.r may move before the sums' scale follows it
-constexpr int kCopies = 8;  // copies of a meeting's outcome, so that fewer blocks poll one line
+constexpr int kRescale = 48;             // bits that r.r may move before the sums' scale follows it
+constexpr int kCopies = 8;               // copies of a meeting's outcome, so that fewer blocks poll one line
 
-// The factors and the stopping test from the sums d.q, r.q, q.q, r.r, q times c.qscale
-// (after kMeasure: from |r - alpha q|^2).
+// The factors and the stopping test from the sums d.q, r.q, q.q (times qscale), r.r (after
+// kMeasure: from |r - alpha q|^2).  Timed: the work of the first kind and no end but the cap.
 __device__ __forceinline__ Outcome decide(CgScalars & c, const F3 (&sum)[kSums], float alpha, bool measured,
                                           bool timed) {
     Outcome o{alpha, 0.f, kGoOn};
-    if (timed) {
-        o.alpha = f3_quotient(sum[3], sum[0]) * c.qscale;
-        o.code  = ++c.it >= c.max_iter ? 2u : unsigned(kGoOn);
-        return o;
-    }
+    const float t2 = pow2(c.threshold_e), th = c.threshold_h * t2, tl = c.threshold_l * t2;
     if (!measured) {
-        c.pq      = sum[0];
-        c.rr      = sum[3];
-        c.rr_next = c.rr;
-        if (!(c.pq.h != 0.f) || c.pq.h != c.pq.h) {
+        const F3 & pq = sum[0];
+        c.rr          = sum[3];
+        c.rr_next     = c.rr;
+        if (!timed && (!(pq.h != 0.f) || pq.h != pq.h)) {
             o.code = 3;
             return o;
         }
-        const float a = f3_quotient(c.rr, c.pq);  // alpha / qscale
-        o.alpha       = a * c.qscale;
-        const F3 t    = f3_add(f3_scale(sum[2], a), f3_scale(sum[1], -2.f));
-        c.rr_next     = f3_add(c.rr, f3_scale(t, a));
+        o.alpha    = f3_quotient(c.rr, pq);
+        const F3 t = f3_add(f3_scale(sum[2], o.alpha * c.qinv), f3_scale(sum[1], -2.f));
+        c.rr_next  = f3_add(c.rr, f3_scale(t, o.alpha));
         // (the margin over the threshold is far above the prediction's error)
-        if (!(c.rr_next.h > kPredict * c.rr.h) || !(c.rr_next.h > c.threshold_h * (1.f + 0x1p-16f)) ||
+        if (!(c.rr_next.h > kPredict * c.rr.h) || !(c.rr_next.h > th * (1.f + 0x1p-16f)) ||
             c.it + 1 >= c.max_iter) {
-            o.code = kMeasure;
-            return o;
+            if (!timed) {
+                o.code = kMeasure;
+                return o;
+            }
         }
     } else c.rr_next = sum[0];
     c.it++;
     const F3 & n = c.rr_next;
-    if (n.h != n.h) o.code = 3;
+    if (timed) o.code = c.it >= c.max_iter ? 2u : unsigned(kGoOn);
+    else if (n.h != n.h) o.code = 3;
     // (r = 0 is below any threshold, also one that the scale takes to 0 in FP32)
-    else if (!(n.h > 0.f) || n.h < c.threshold_h || (n.h == c.threshold_h && n.m < c.threshold_l)) o.code = 1;
+    else if (!(n.h > 0.f) || n.h < th || (n.h == th && n.m < tl)) o.code = 1;
     else if (c.it >= c.max_iter) o.code = 2;
     else {
         const int e = int(__float_as_uint(n.h) >> 23) - 127;
         if (abs(e) > kRescale) {
             o.shift = max(-120, min(120, -e));
-            c.set_threshold(c.threshold * double(pow2(o.shift)));
+            c.threshold_e += o.shift;
         }
     }
     o.beta = f3_quotient(n, c.rr);
@@ -281,8 +273,6 @@ __device__ __forceinline__ Outcome decide_start(CgState * cg, CgScalars & c, dou
         cg->bb        = bb;
         cg->rr        = rr;
         cg->rr0       = rr;
-        cg->rr_prev   = 0;
-        cg->pq        = 0;
         cg->iter      = 0;
         cg->max_iter  = cap;
         cg->threshold = threshold;
@@ -328,8 +318,10 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
         if (blockIdx.x != 0 && lane == 0) {
             const ulonglong2 * p = outcome + blockIdx.x % kCopies;
             Outcome o;
-            bool there = outcome_get(p, tag, o);
-            for (int n = 0; n < polls && !there; n++) there = outcome_get(p, tag, o);
+            bool there;
+            int n = polls;
+            do there = outcome_get(p, tag, o);
+            while (!there && n-- > 0);
             if (!there) o.code = kFailed;
             M.out = o;
         }
@@ -342,11 +334,12 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
                 bool full = true;
                 for (int j = lane; j < blocks; j += 32) {
                     ulonglong2 w{0, 0};
-                    bool there = false;
-                    for (int n = 0; n <= polls && !there; n++) {
+                    bool there;
+                    int n = polls;
+                    do {
                         w     = word_get(slots + (long long) j * kSums + warp);
                         there = unsigned(w.y >> 32) == tag;
-                    }
+                    } while (!there && n-- > 0);
                     full = full && there;
                     s += __longlong_as_double((long long) w.x);
                 }
@@ -361,8 +354,9 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
             bool full = true;
             for (int j0 = lane; j0 < blocks; j0 += 32 * 5) {
                 F3 e[5];
-                bool there = false;
-                for (int n = 0; n <= polls && !there; n++) {
+                bool there;
+                int n = polls;
+                do {
                     there = true;
 #pragma unroll
                     for (int q = 0; q < 5; q++) {
@@ -370,7 +364,7 @@ __device__ __forceinline__ Outcome meet(const F3 & v, ulonglong2 * slots, int st
                         e[q]        = F3{0.f, 0.f, 0.f};
                         if (j < blocks) there = slot_get(slots + (long long) j * kSums + warp, tag, e[q]) && there;
                     }
-                }
+                } while (!there && n-- > 0);
                 full = full && there;
                 if (blocks > 32) e[0] = f3_add(f3_add(f3_add(e[0], e[1]), f3_add(e[2], e[3])), e[4]);
                 s = f3_add(s, e[0]);
@@ -480,8 +474,12 @@ __device__ __forceinline__ Outcome meet_cluster(const F3 & v, int active, unsign
 __device__ __forceinline__ bool wait_neighbours(const unsigned * flags, const int * tab, int polls, unsigned tag) {
     const int lane = threadIdx.x & 31;
     const int b    = lane < 27 ? tab[lane] : -1;
-    bool there     = b < 0 || ld_relaxed(flags + b) == tag;
-    for (int n = 0; n < polls && !there; n++) there = ld_relaxed(flags + b) == tag;
+    bool there     = b < 0;
+    int n          = polls;
+    while (!there) {
+        there = ld_relaxed(flags + b) == tag;
+        if (n-- <= 0) break;
+    }
     fence_gpu();
     return __all_sync(0xffffffffu, there);
 }
@@ -615,10 +613,9 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
                 } else {
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        const float qs = p[j] * from.qscale;
-                        ff_add_prod(part[0], comp(d, j), qs);
-                        ff_add_prod(part[1], comp(r, j), qs);
-                        ff_add_prod(part[2], qs, qs);
+                        ff_add_prod(part[0], comp(d, j), p[j]);
+                        ff_add_prod(part[1], comp(r, j), p[j]);
+                        ff_add_prod(part[2], p[j], p[j] * from.qscale);
                         ff_add_prod(part[3], comp(r, j), comp(r, j));
                     }
                     st4(N.q, s, make_float4(p[0], p[1], p[2], p[3]));
@@ -720,8 +717,6 @@ __device__ __forceinline__ void solve(const Lattice & L, const int * __restrict_
         if (blockIdx.x == 0) {
             if (started) {
                 cg->rr      = f3_double(M.cg.rr_next) / double(scale);
-                cg->rr_prev = f3_double(M.cg.rr) / double(scale);
-                cg->pq      = f3_double(M.cg.pq) / (double(scale) * double(from.qscale));
                 cg->iter    = M.cg.it;
                 if (o.code != kFailed) cg->done = int(o.code);
             }

@@ -519,8 +519,6 @@ __device__ __forceinline__ float3 wall_term(const Lattice & L, const Phys & P, c
 struct CgState {
     double bb;         // |b|^2
     double rr;         // |r_i|^2
-    double rr_prev;    // |r_{i-1}|^2
-    double pq;         // d_i . A d_i
     double threshold;  // max(tol^2 |b|^2, DBL_MIN)
     double rr0;        // initial |r_0|^2
     int    iter;       // completed iterations (SpMV count in the loop)
@@ -542,7 +540,7 @@ struct CgStart {
     int         max_iterations;  // < 0: twice the active nodes
     int         own;
     const int * nv;              // device: active nodes
-    float       qscale;          // power of two near 1 / |A|, for the sums with q = A d
+    float       qscale;          // power of two near 1 / |A|, for the sum q.q of q = A d
     int         polls;           // looks at a word before a block gives up waiting for it
     int         timed;           // max_iterations iterations whatever the sums say (x is not wanted)
 };
