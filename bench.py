@@ -70,10 +70,10 @@ def peaks():
 
 SM_MAX_MHZ = 2070.0
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the 128^3 block,
-# per active node of the captured launch: k_node_gather 90,965,504 + 13,017,856 B and
-# k_pressure_gradient 113,461,248 + 12,455,680 B at 2,246,538 nodes (profiles/)
-DRAM_BYTES_PER_NODE = {"virtual_gather": (90965504 + 13017856) / 2246538,
-                       "pressure_gradient": (113461248 + 12455680) / 2246538}
+# per active node of the captured launch: k_node_gather 91,485,184 + 13,213,184 B and
+# k_pressure_gradient 113,536,768 + 12,678,912 B at 2,246,535 nodes (profiles/)
+DRAM_BYTES_PER_NODE = {"virtual_gather": (91485184 + 13213184) / 2246535,
+                       "pressure_gradient": (113536768 + 12678912) / 2246535}
 
 
 class ClockSampler:
@@ -424,8 +424,8 @@ def run_training_leg(args, torch, epochs=5):
         out.update({"train_rows": F.shape[0], "epochs": epochs, "batch": 16384, "seconds": t2 - t1,
                     "setup_seconds": t1 - t0, "rows_per_s": epochs * F.shape[0] / (t2 - t1),
                     "epoch_loss": [float(x) for x in ep_loss],
-                    "note": "per batch: device shuffle gather, fused tcgen05 gradient pass (BF16 operands, FP32 "
-                            "accumulation), Adam; the epoch loss over the whole dataset on the device"})
+                    "note": "per batch: fused tcgen05 gradient pass over the rows of a device permutation (BF16 "
+                            "operands, FP32 accumulation), reduction with Adam; the epoch loss over the whole dataset on the device"})
     return out
 
 
@@ -513,7 +513,7 @@ def run_gpu_arm(args):
     # algorithmic bytes per launch (each array touched once per pass)
     alg = {
         "cg_step": 36 * nv,  # reads x, r, q, d, V; writes x, r, d, u = V d
-        "cg_product": 16 * nv,  # reads u (halo tiles from L2), d, alpha_hat; writes q (FP32)
+        "cg_product": 21 * nv,  # reads u (halo tiles from L2), d, alpha_hat, r, flag; writes q (FP32)
         "cg_meeting": 0,  # the blocks' sums: latency alone
         "virtual_gather": 32 * (n + nb) + 16 * nv,  # particle pos/vel once; V, D, rho, flag out
         "pressure_gradient": 32 * n + 8 * nv + 48 * nb,  # pos, vel r/w; V, p; boundary pos/vel/nrm

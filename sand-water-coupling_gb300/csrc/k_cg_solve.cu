@@ -25,7 +25,8 @@
 // Before a warp copies a tile it waits for the flags of the brick's neighbours; the
 // blocks meet once per iteration, for the sums, and each decides by itself whether to
 // go on, with no host check.  Dot products use exact FP32 products in float-float per
-// lane, triple floats below the block and FP64 above, in a fixed order.
+// lane and triple floats above (the start's |r|^2 and |b|^2: FP64 above the block), in a
+// fixed order.
 #include <type_traits>
 
 #include "swc_kernels.h"

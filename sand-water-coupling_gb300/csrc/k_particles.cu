@@ -87,8 +87,8 @@ __global__ void k_max_speed2(const float4 * __restrict__ vel, long long n, int d
 }
 
 // ---------------------------------------------------------------------------
-// Counting sort into cells.  Order within a cell is made deterministic by an
-// insertion sort on the original id, so the final order is (cell, id).
+// Counting sort into cells.  Order within a cell is made deterministic by ranking
+// its particles by the original id, so the final order is (cell, id).
 // ---------------------------------------------------------------------------
 // With vel non-null the particles are first moved, x += v dt
 // (SmthParticleHydrodLiquid::moveParticles, Cores/Physics/SmthParticleHydrodLiquid.cpp:72-76,

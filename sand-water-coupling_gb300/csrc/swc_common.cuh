@@ -238,7 +238,7 @@ __device__ __forceinline__ double kW_d(double r, double inv_h, double c0) {
 // --------------------------------------------------------------------------
 // Float-float accumulation (error-free transforms, Knuth TwoSum / FMA TwoProd).
 // Products are exact; sums keep ~44 significant bits.  Used below the warp
-// level; warp partials are converted to FP64 and summed in FP64.
+// level; above it the passes sum in FP64, the CG solve in triple floats.
 // --------------------------------------------------------------------------
 struct FF {
     float hi, lo;

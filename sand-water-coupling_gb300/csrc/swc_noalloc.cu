@@ -13,8 +13,8 @@
 //
 // The arrays exist once per device that loads this library and live until the
 // process exits (about 0.7 MB).  Every call reuses them and they keep the last
-// call's contents; the shares are overwritten in full by each call and only the
-// error flag needs to start at zero, which each call clears.  Calls that overlap
+// call's contents; what a call reads of the shares it has written before, and only
+// the error flag needs to start at zero, which each call clears.  Calls that overlap
 // on the GPU (different streams, or the same arrays used by two host threads at
 // once) race on the scratch.  The device addresses of the arrays are looked up
 // once per device; they do not survive a cudaDeviceReset of that device.
